@@ -458,6 +458,18 @@ unsigned tile_grid(pi_batch* b, int persist) {
     if (!persist) return (unsigned)std::max(1, b->ntiles);
     return (unsigned)std::max(1, std::min(b->ntiles, persist * b->nsm));
 }
+
+// Work units per tile of k32_move and k32_physiology in blocks of bs threads (unit_tile): whole
+// tiles once they are 8 blocks per SM, otherwise tiles are cut in two until they are, down to one
+// slot per thread.
+int tile_sub(const pi_batch* b, int bs) {
+    int sub = 1;
+    while (sub < F32_TILE / bs && (long long)b->ntiles * sub < 8LL * b->nsm) sub *= 2;
+    return sub;
+}
+unsigned unit_grid(pi_batch* b, int persist, int sub) {
+    return sub > 1 ? (unsigned)std::max(1, b->ntiles * sub) : tile_grid(b, persist);
+}
 unsigned warp_grid(long long nitems, int wpb) { return std::max(1u, nblk(nitems, wpb)); }
 
 // Enqueues one step on the batch stream (eager launches, or the body of a graph capture).
@@ -514,8 +526,9 @@ pi_status enqueue_step(pi_batch* b, double dT, int cur) {
         a.T = b->T; a.P = b->P; a.sp = b->sp; a.bgc = b->bgc; a.F = b->F; a.rdzC = b->rdzC; a.st = b->st;
         a.dT = fdT; a.Gtot = G; a.pop = b->pop; a.pop_sp = b->pop_sp; a.chl_acc = b->chl_acc; a.acc = b->acc;
         a.dcnt = b->dcnt; a.err = b->errw;
+        a.sub = tile_sub(b, b->tune.bs_move);
         BScope sc(b, "k32_move");
-        const unsigned g = tile_grid(b, b->tune.persist_move);
+        const unsigned g = unit_grid(b, b->tune.persist_move, a.sub);
         if (b->tune.occ_move == 4) k32_move<4><<<g, b->tune.bs_move, 0, s>>>(a);
         else if (b->tune.occ_move == 3) k32_move<3><<<g, b->tune.bs_move, 0, s>>>(a);
         else k32_move<2><<<g, b->tune.bs_move, 0, s>>>(a);
@@ -539,8 +552,9 @@ pi_status enqueue_step(pi_batch* b, double dT, int cur) {
         a.par = b->par; a.pop = b->pop; a.pop_sp = b->pop_sp; a.env = b->env; a.acc = b->acc; a.dcnt = b->dcnt;
         a.err = b->errw; a.dec64 = b->dec64; a.guard = b->guard;
         a.dproc = b->diag_proc; a.pmask = b->proc_mask;
+        a.sub = tile_sub(b, b->tune.bs_phys);
         BScope sc(b, "k32_physiology");
-        const unsigned g = tile_grid(b, b->tune.persist_phys);
+        const unsigned g = unit_grid(b, b->tune.persist_phys, a.sub);
         if (b->tune.occ_phys == 4) k32_physiology<4><<<g, b->tune.bs_phys, 0, s>>>(a);
         else if (b->tune.occ_phys == 3) k32_physiology<3><<<g, b->tune.bs_phys, 0, s>>>(a);
         else k32_physiology<2><<<g, b->tune.bs_phys, 0, s>>>(a);

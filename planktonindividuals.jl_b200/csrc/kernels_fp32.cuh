@@ -330,7 +330,19 @@ struct MoveArgs {
     unsigned long long* acc;       // ACC_N × Gtot
     uint32_t* dcnt;                // nsp × 4 × Gtot: num, graz, mort, dvid
     uint32_t* err;
+    int sub;                       // work units per tile (see unit_tile)
 };
+
+// A work unit of the particle kernels is 1/sub of a tile: F32_TILE / sub consecutive slots. With
+// sub = 1 a thread walks F32_TILE / blockDim.x slots and loads the next while it works on the
+// current one, which is best when the tiles fill the chip. A model of few tiles leaves most SMs
+// idle that way (1024 individuals are one tile, that is one block walking 8 slots deep: 34 µs of
+// k32_physiology); there sub = F32_TILE / blockDim.x gives every slot its own thread.
+__device__ __forceinline__ int unit_tile(int u, int sub, int& first) {
+    const int t = sub == 1 ? u : u / sub;
+    first = (u - t * sub) * (F32_TILE / sub);
+    return t;
+}
 
 // bit of logical slot L of species s of member m in a logical-slot bitmap
 __device__ __forceinline__ void slot_bit(const MemberDev& m, int s, int L, long long& w, uint32_t& bit) {
@@ -489,17 +501,18 @@ template <int MINB>
 __global__ void __launch_bounds__(256, MINB) k32_move(MoveArgs a) {
     if (stopped(a.err)) return;
     __shared__ PGeom sg;
-    const int bs = blockDim.x, ppt = F32_TILE / bs;
+    const int bs = blockDim.x, ppt = F32_TILE / (bs * a.sub);
     const uint32_t iter = (uint32_t)(a.st->iteration + 1);
-    for (int t = blockIdx.x; t < a.T.ntiles; t += gridDim.x) {
-        const int2 tl = a.T.tiles[t];
+    for (int u = blockIdx.x; u < a.T.ntiles * a.sub; u += gridDim.x) {
+        int first;
+        const int2 tl = a.T.tiles[unit_tile(u, a.sub, first)];
         int mi, s;
         seg_of(a.T, tl.x, mi, s);
         const MemberDev& m = a.T.md[mi];
         if (threadIdx.x == 0) sg = pgeom(m, a.F[mi]);
         __syncthreads();
         const long long base = m.slot_off + (long long)s * m.C;
-        long long slot = (long long)tl.y + threadIdx.x;
+        long long slot = (long long)tl.y + first + threadIdx.x;
         MState nx = move_state(a.P, base + slot, slot < m.C);
         for (int p = 0; p < ppt; ++p, slot += bs) {
             const MState cur = nx;
@@ -864,6 +877,7 @@ struct PhysArgs {
     unsigned long long* guard;  // [0] decisions recomputed in Float64, [1] of those, decisions changed
     unsigned long long* dproc;  // optional process diagnostics, fixed point: (species * PI_NPROC + q) * Gtot
     uint32_t pmask;             // enabled processes (PI_PROC_* bits)
+    int sub;                    // work units per tile (see unit_tile)
 };
 
 // Fixed-point units of the process diagnostics: rates (mmol s⁻¹) in the mass unit per minute,
@@ -1086,16 +1100,17 @@ __device__ __forceinline__ void scatter_phys(const PhysArgs& a, int s, const Phy
 template <int MINB>
 __global__ void __launch_bounds__(256, MINB) k32_physiology(PhysArgs a) {
     if (stopped(a.err)) return;
-    const int bs = blockDim.x, ppt = F32_TILE / bs;
+    const int bs = blockDim.x, ppt = F32_TILE / (bs * a.sub);
     const uint32_t iter = (uint32_t)(a.st->iteration + 1);
     const double tnow = (double)(a.st->iteration + 1) * (double)a.dT;
-    for (int t = blockIdx.x; t < a.T.ntiles; t += gridDim.x) {
-        const int2 tl = a.T.tiles[t];
+    for (int u = blockIdx.x; u < a.T.ntiles * a.sub; u += gridDim.x) {
+        int first;
+        const int2 tl = a.T.tiles[unit_tile(u, a.sub, first)];
         int mi, s;
         seg_of(a.T, tl.x, mi, s);
         const MemberDev& m = a.T.md[mi];
         const long long base = m.slot_off + (long long)s * m.C;
-        long long slot = (long long)tl.y + threadIdx.x;
+        long long slot = (long long)tl.y + first + threadIdx.x;
         PHead hd = phys_head(a.P, base + slot, phys_pre(a.P, base + slot, slot < m.C), m, a.env);
         PPre pre = phys_pre(a.P, base + slot + bs, 1 < ppt && slot + bs < m.C);
         for (int p = 0; p < ppt; ++p, slot += bs) {
