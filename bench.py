@@ -188,14 +188,13 @@ def step_roofline(n_ind, n_cells, ms_per_step):
 
 def gpu_launches(prof, P, K, workload):
     """Own kernels launched in K timed steps, from the kernels one profiled step launched: one per
-    profiled scope, except the halo fill (three passes in the 0D boxes, whose N < H) and the
-    storage-order sort (count, three scan passes, scatter; once per SORT_INTERVAL steps), plus
-    k32_copy_if_err and k32_end_step in every step."""
-    per_step = 2
+    profiled scope, except the storage-order sort (count, three scan passes, scatter; once per
+    SORT_INTERVAL steps)."""
+    per_step = 0
     for name, (n, _) in prof.items():
         if name == "k32_sort":
             continue
-        per_step += (3 if (name == "k32_halo" and workload == "config5") else 1) * n // P
+        per_step += n // P
     return K * per_step + 5 * (-(-K // SORT_INTERVAL))
 
 

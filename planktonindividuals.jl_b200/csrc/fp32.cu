@@ -100,7 +100,8 @@ struct pi_batch {
     std::string err;
     std::vector<void*> allocs;
     long long Gtot = 0, Stot = 0, ncol = 0, maxG = 0, maxcol = 0, maxhalo = 0;
-    bool halo_direct = true;        // every member has N >= H on every axis: one-pass halo fill
+    bool halo_direct = true;        // no member has a periodic axis with N < H: one-pass halo fill
+    bool n_ge_h = true;             // every member has N >= H on every axis
     int nlev = 0;
     // device
     MemberDev* md = nullptr;
@@ -281,7 +282,7 @@ void free_tables(pi_batch* b) {
 // general path), every axis of every member has at least as many cells as halo points (one-pass
 // halo fill), and the tracers' halos are filled (not the first step after an upload).
 bool use_fused(const pi_batch* b) {
-    if (!b->tune.fused || !b->halo_direct || b->tracers_dirty) return false;
+    if (!b->tune.fused || !b->n_ge_h || b->tracers_dirty) return false;
     for (int m = 0; m < b->nm; ++m) {
         if (b->mdh[m].any_bc) return false;
         const pi_bgc_params& p = b->mh[m].bgc;
@@ -585,19 +586,21 @@ pi_status enqueue_step(pi_batch* b, double dT, int cur) {
         }
         }
     }
+    const StepEnd end{ b->nm, b->F, b->st, dT, trn, tr, (long long)PI_NTRACERS * G };
     if (fused) {
         // k32_tracer wrote the halo cells with the interior
+        k32_end_step<<<148 * 4, 256, 0, s>>>(end, b->errw);
     } else if (b->halo_direct) { BScope sc(b, "k32_halo");
       // about 16 blocks per SM over all members, enough for every member's halo cells
       const unsigned gx = std::max(1u, std::min<unsigned>(nblk(b->maxhalo, 256), std::max(1, b->nsm * 16 / b->nm)));
-      k32_halo_direct<<<dim3(gx, b->nm), 256, 0, s>>>(b->md, G, trn, PI_NTRACERS, b->errw);
+      k32_halo_direct<<<dim3(gx, b->nm), 256, 0, s>>>(b->md, G, trn, end, b->errw);
+    } else if (b->maxG <= HALO_SMALL) { BScope sc(b, "k32_halo");
+      k32_halo_small<<<dim3(b->nm, PI_NTRACERS), 256, 0, s>>>(b->md, G, trn, end, b->errw);
     } else { BScope sc(b, "k32_halo");
-      k32_halo<0><<<std::min<unsigned>(nblk(b->nlines[0], 128), 148 * 8), 128, 0, s>>>(b->md, b->line_off[0], b->nm, G, trn, PI_NTRACERS, b->errw);
-      k32_halo<1><<<std::min<unsigned>(nblk(b->nlines[1], 128), 148 * 8), 128, 0, s>>>(b->md, b->line_off[1], b->nm, G, trn, PI_NTRACERS, b->errw);
-      k32_halo<2><<<std::min<unsigned>(nblk(b->nlines[2], 128), 148 * 8), 128, 0, s>>>(b->md, b->line_off[2], b->nm, G, trn, PI_NTRACERS, b->errw); }
-    k32_copy_if_err<<<148 * 4, 256, 0, s>>>(trn, tr, (long long)PI_NTRACERS * G, b->errw);
+      k32_halo<0><<<dim3(std::min<unsigned>(nblk(b->nlines[0], 128), 148 * 8), PI_NTRACERS), 128, 0, s>>>(b->md, b->line_off[0], b->nm, G, trn, end, b->errw);
+      k32_halo<1><<<dim3(std::min<unsigned>(nblk(b->nlines[1], 128), 148 * 8), PI_NTRACERS), 128, 0, s>>>(b->md, b->line_off[1], b->nm, G, trn, end, b->errw);
+      k32_halo<2><<<dim3(std::min<unsigned>(nblk(b->nlines[2], 128), 148 * 8), PI_NTRACERS), 128, 0, s>>>(b->md, b->line_off[2], b->nm, G, trn, end, b->errw); }
     if (b->tr_mask) k32_diag_tracers<<<148 * 4, 256, 0, s>>>(b->diag_tr, trn, b->tr_mask, G, b->errw);
-    k32_end_step<<<nblk(b->nm, 128), 128, 0, s>>>(b->nm, b->F, b->st, dT, b->errw);
     BK(cudaGetLastError(), "step launch");
     return PI_OK;
 }
@@ -809,7 +812,8 @@ pi_status pi_batch_create(const pi_member* members, int32_t nmembers, int32_t ns
         col += (long long)g.Nx * g.Ny;
         lev += g.Gz;
         b->maxG = std::max(b->maxG, g.G);
-        if (g.Nx < g.Hx || g.Ny < g.Hy || g.Nz < g.Hz) b->halo_direct = false;
+        if (g.Nx < g.Hx || g.Ny < g.Hy || g.Nz < g.Hz) b->n_ge_h = false;
+        if ((g.topo[0] == PI_PERIODIC && g.Nx < g.Hx) || (g.topo[1] == PI_PERIODIC && g.Ny < g.Hy)) b->halo_direct = false;
         b->maxhalo = std::max(b->maxhalo, g.G - (long long)g.Nx * g.Ny * g.Nz);
         b->maxcol = std::max(b->maxcol, (long long)g.Nx * g.Ny);
     }
