@@ -2,10 +2,13 @@
 // include/pib200.h). A PlanktonModel created with PI_FP32 is a batch of one member.
 //
 // One step is this sequence of launches, each covering every member:
-//   k32_bind             forcing of the step from device-resident series; vel½ buffer choice
-//   k32_velhalf          vel½ for members whose vel₀ and vel₁ differ
+//   k32_begin            forcing of the step from device-resident series, vel½ for members whose
+//                        vel₀ and vel₁ differ, per-cell counts cleared
 //   k32_move             RK4 + diffusion + find_inds!, pop/Chl sums, previous decisions; dividers
-//                        and newly freed slots marked in bitmaps over logical slots
+//                        and newly freed slots marked in bitmaps over logical slots and counted per
+//                        segment
+//   k32_par_divide       small segments: calc_par! down each column beside the division of each
+//                        segment by one block; otherwise
 //   k32_par              calc_par! down each column
 //   k32_count_tiles      dividers and free slots of every tile of logical slots
 //   scan(tile counts)    division and free-slot offsets of every tile
@@ -20,8 +23,8 @@
 //   k32_xy               DST3FL x and y sweeps of every tracer on level tiles in shared memory
 //   k32_ztail            z sweep walking columns, then diffusion, sinking, forcing, BCs, particle
 //                        terms and apply_tendency!
-//   k32_halo<x,y,z>      fill_halo_tracer!
-//   k32_end_step         vel₀ ← vel₁, iteration and t
+//   k32_halo_direct (k32_halo_small, k32_halo<x,y,z>)  fill_halo_tracer!, then vel₀ ← vel₁,
+//                        iteration and t
 // Every sort_interval steps (and before the first step after an upload) the slots of every segment
 // are put back in cell order by a counting sort into the second buffer of the individual arrays
 // (k32_sort_count, a scan of the bin populations, k32_sort_scatter).
@@ -78,7 +81,7 @@ struct Tuning {
     int persist_move = 2, persist_phys = 0;   // 0: one tile per block; k: k blocks per SM, looping
     int ty = 16;                              // rows of an x-y tracer tile (4, 8, 16 or 28)
     int lz = 32;                              // levels walked by a z thread (8, 16, 32 or 64)
-    int wpb_par = 2;
+    int wpb_par = 0;                          // warps per 32 columns of k32_par (0: by the levels)
     int occ_move = 2, occ_phys = 4;           // register fit of k32_move / k32_physiology (blocks of 256 per SM)
     int concurrent = 0;                       // k32_xy on a second branch beside the particle kernels
     int fused = 0;                            // k32_tracer when the batch allows it (the autotuner
@@ -144,12 +147,14 @@ struct pi_batch {
     long long since_sort = 0;
     bool need_sort = true;
     long long nwords = 0;           // words of each logical-slot bitmap
+    long long maxwps = 0;           // the most words of a segment
     int ntiles = 0;
     int2* tiles = nullptr;
     int* seg_tile0 = nullptr;
     unsigned long long *tile_cnt = nullptr, *tile_off = nullptr;
     int *divlist = nullptr, *freelist = nullptr;
     uint32_t* ndiv = nullptr;
+    int maxNz = 1;
     long long* line_off[3] = {nullptr, nullptr, nullptr};
     long long nlines[3] = {0, 0, 0};
     double last_dT = 0.0;
@@ -471,7 +476,6 @@ int tile_sub(const pi_batch* b, int bs) {
 unsigned unit_grid(pi_batch* b, int persist, int sub) {
     return sub > 1 ? (unsigned)std::max(1, b->ntiles * sub) : tile_grid(b, persist);
 }
-unsigned warp_grid(long long nitems, int wpb) { return std::max(1u, nblk(nitems, wpb)); }
 
 // Enqueues one step on the batch stream (eager launches, or the body of a graph capture).
 pi_status enqueue_step(pi_batch* b, double dT, int cur) {
@@ -481,16 +485,11 @@ pi_status enqueue_step(pi_batch* b, double dT, int cur) {
     float* tr = b->trbuf[cur];
     float* trn = b->trbuf[cur ^ 1];
     const bool fused = use_fused(b);
-    BK(cudaMemsetAsync(b->pop, 0, G * sizeof(int), s), "zero pop");
-    if (b->pop_sp) BK(cudaMemsetAsync(b->pop_sp, 0, (size_t)b->nsp * G * sizeof(int), s), "zero pop");
-    { BScope sc(b, "k32_bind");
-      const unsigned gx = std::max(1u, std::min<unsigned>(nblk(b->maxcol, 256), 64));
-      k32_bind<<<dim3(gx, b->nm), 256, 0, s>>>(b->nm, b->md, b->S, b->F, b->st, dT, b->PARF, b->errw); }
-    // grids of the field passes: about 8 blocks per SM over all members
-    const unsigned fgx = std::max(1u, std::min<unsigned>(nblk(b->maxG, 256), std::max(1, b->nsm * 8 / b->nm)));
-    { BScope sc(b, "k32_velhalf");
-      const unsigned gx = fgx;
-      k32_velhalf<<<dim3(gx, b->nm), 256, 0, s>>>(b->md, b->F, b->errw); }
+    { BScope sc(b, "k32_begin");
+      // about 8 blocks per SM over all members
+      const unsigned gx = std::max(1u, std::min<unsigned>(nblk(b->maxG, 256), std::max(1, b->nsm * 8 / b->nm)));
+      k32_begin<<<dim3(gx, b->nm), 256, 0, s>>>(BeginArgs{ b->md, b->S, b->F, b->st, dT, b->PARF, b->pop, b->pop_sp, b->P.segdiv,
+                                                      b->P.segfree, b->nsp, G, b->errw }); }
     TrArgs ta;
     ta.T = b->T; ta.lm = b->lm; ta.dzF = b->dzF; ta.dzC = b->dzC; ta.rdzC = b->rdzC; ta.bgc = b->bgc;
     ta.bcs = b->bcs; ta.st = b->st; ta.F = b->F; ta.Gtot = G; ta.tr = tr; ta.tb = b->tb; ta.tr_next = trn;
@@ -534,10 +533,18 @@ pi_status enqueue_step(pi_batch* b, double dT, int cur) {
         else if (b->tune.occ_move == 3) k32_move<3><<<g, b->tune.bs_move, 0, s>>>(a);
         else k32_move<2><<<g, b->tune.bs_move, 0, s>>>(a);
     }
+    // light: as many warps per 32 columns as the levels give work to
+    const int lw = b->tune.wpb_par ? b->tune.wpb_par : b->maxNz <= PAR_CH ? 1 : b->maxNz <= 2 * PAR_CH ? 2 : b->maxNz <= 4 * PAR_CH ? 4 : 8;
+    const ParArgs pa{ b->T, b->dzF, b->bgc, b->chl_acc, b->PARF, b->par, b->diag_par, tr, G, b->F, b->pop, b->env, b->st, lw, b->maxNz };
+    const unsigned parblocks = nblk((long long)b->T.nicol * lw, PAR_WARPS);
+    // a block per segment reads every segment's counts: at most 1,024 of them
+    if (b->maxwps <= DIV_WORDS && b->nseg <= 1024) {
+      BScope sc(b, "k32_par_divide");
+      k32_par_divide<<<b->nseg + parblocks, 32 * DIV_WARPS, 0, s>>>(
+          pa, DivArgs{ b->T, b->P, b->divlist, b->freelist, b->nseg, b->st, b->errw });
+    } else {
     { BScope sc(b, "k32_par");
-      k32_par<<<warp_grid(b->T.nicol, b->tune.wpb_par), 32 * b->tune.wpb_par, 0, s>>>(b->T, b->dzF, b->bgc, b->chl_acc, b->PARF,
-                                                                                   b->par, b->diag_par, tr, G, b->F, b->pop,
-                                                                                   b->env, b->errw); }
+      k32_par<<<parblocks, 32 * PAR_WARPS, 0, s>>>(pa); }
     { BScope sc(b, "k32_count_tiles");
       k32_count_tiles<<<nblk((long long)b->ntiles * 32, 256), 256, 0, s>>>(b->T, b->P, b->tile_cnt, b->errw); }
     { BScope sc(b, "k32_scan_tiles");
@@ -547,6 +554,7 @@ pi_status enqueue_step(pi_batch* b, double dT, int cur) {
           b->T, b->P, b->tile_cnt, b->tile_off, b->divlist, b->freelist, b->ndiv, b->st, b->errw); }
     { BScope sc(b, "k32_daughters");
       k32_daughters<<<dim3(4, b->nseg), 128, 0, s>>>(b->T, b->P, b->divlist, b->freelist, b->ndiv, b->errw); }
+    }
     {
         PhysArgs a;
         a.T = b->T; a.P = b->P; a.sp = b->sp; a.F = b->F; a.st = b->st; a.dT = fdT; a.Gtot = G; a.tr = tr;
@@ -682,6 +690,7 @@ pi_status check_errors(pi_batch* b) {
         // the step stopped after the decisions: drop the unconsumed loss sums and divider marks
         BK(cudaMemsetAsync(b->acc, 0, (size_t)ACC_N * b->Gtot * sizeof(unsigned long long), b->stream), "clear sums");
         BK(cudaMemsetAsync(b->P.dvbits, 0, (size_t)b->nwords * sizeof(uint32_t), b->stream), "clear divider marks");
+        BK(cudaMemsetAsync(b->P.segdiv, 0, (size_t)b->nseg * sizeof(uint32_t), b->stream), "clear divider counts");
         BK(cudaStreamSynchronize(b->stream), "synchronize");
         // TimeStep! advanced model.iteration and model.t before it threw (time_step.jl:14-15)
         hs.iteration = hs.err_iter;
@@ -808,10 +817,12 @@ pi_status pi_batch_create(const pi_member* members, int32_t nmembers, int32_t ns
         cell += (g.G + 63) / 64 * 64;       // members start on 256-byte boundaries
         slot += (long long)nspecies * h.C;
         words += (long long)nspecies * d.wps;
+        b->maxwps = std::max(b->maxwps, d.wps);
         bins += (long long)nspecies * ((long long)g.Nx * g.Ny * g.Nz + (h.C + F32_TILE - 1) / F32_TILE);
         col += (long long)g.Nx * g.Ny;
         lev += g.Gz;
         b->maxG = std::max(b->maxG, g.G);
+        b->maxNz = std::max(b->maxNz, g.Nz);
         if (g.Nx < g.Hx || g.Ny < g.Hy || g.Nz < g.Hz) b->n_ge_h = false;
         if ((g.topo[0] == PI_PERIODIC && g.Nx < g.Hx) || (g.topo[1] == PI_PERIODIC && g.Ny < g.Hy)) b->halo_direct = false;
         b->maxhalo = std::max(b->maxhalo, g.G - (long long)g.Nx * g.Ny * g.Nz);
@@ -843,7 +854,9 @@ pi_status pi_batch_create(const pi_member* members, int32_t nmembers, int32_t ns
         BA(Pq.lslot, S);
     }
     BA(b->Pbuf[0].phys, S); BA(b->Pbuf[0].freebits, words); BA(b->Pbuf[0].dvbits, words);
+    BA(b->Pbuf[0].segdiv, b->nseg); BA(b->Pbuf[0].segfree, b->nseg);
     b->Pbuf[1].phys = b->Pbuf[0].phys; b->Pbuf[1].freebits = b->Pbuf[0].freebits; b->Pbuf[1].dvbits = b->Pbuf[0].dvbits;
+    b->Pbuf[1].segdiv = b->Pbuf[0].segdiv; b->Pbuf[1].segfree = b->Pbuf[0].segfree;
     b->pcur = 0;
     b->P = b->Pbuf[0];
     IndDev32& P = b->P;
@@ -937,6 +950,10 @@ pi_status pi_batch_create(const pi_member* members, int32_t nmembers, int32_t ns
                 for (long long L = 0; L < d.C; ++L) fb[d.woff + sp * d.wps + (L >> 5)] |= 1u << (L & 31);
         }
         H2D(P.freebits, fb.data(), words * sizeof(uint32_t));
+        std::vector<uint32_t> sf(b->nseg);
+        for (int q = 0; q < b->nseg; ++q) sf[q] = (uint32_t)b->mdh[q / nspecies].C;
+        H2D(P.segfree, sf.data(), sf.size() * sizeof(uint32_t));
+        Z(P.segdiv, b->nseg * sizeof(uint32_t));
         ok = ok && cudaStreamSynchronize(s0) == cudaSuccess;
     }
     for (int m = 0; m < nmembers && ok; ++m)
@@ -1045,10 +1062,13 @@ pi_status pi_batch_set_individuals(pi_batch* b, int32_t member, int32_t sp, cons
     k32_identity_order<<<std::min<unsigned>(nblk(C, 256), 1024), 256, 0, s>>>(P, g0, C);
     BK(cudaGetLastError(), "upload individuals");
     std::vector<uint32_t> fb(d.wps, 0u);
-    for (long long i = 0; i < C; ++i) if (!in->ac[i]) fb[i >> 5] |= 1u << (i & 31);
+    uint32_t nfree = 0;
+    for (long long i = 0; i < C; ++i) if (!in->ac[i]) { fb[i >> 5] |= 1u << (i & 31); ++nfree; }
     const long long w0 = d.woff + (long long)sp * d.wps;
     BK(cudaMemcpyAsync(P.freebits + w0, fb.data(), d.wps * sizeof(uint32_t), cudaMemcpyHostToDevice, s), "upload individuals");
     BK(cudaMemsetAsync(P.dvbits + w0, 0, d.wps * sizeof(uint32_t), s), "upload individuals");
+    BK(cudaMemsetAsync(P.segdiv + (member * b->nsp + sp), 0, sizeof(uint32_t), s), "upload individuals");
+    BK(cudaMemcpyAsync(P.segfree + (member * b->nsp + sp), &nfree, sizeof nfree, cudaMemcpyHostToDevice, s), "upload individuals");
     BK(cudaStreamSynchronize(s), "synchronize");
     b->need_sort = true;
     return PI_OK;
@@ -1834,7 +1854,7 @@ pi_status pi_batch_autotune(pi_batch* b, double dT, int32_t k, char* report, siz
         { "k32_assign", &t.bs_assign, {128, 256, 512, 1024}, "assign block", 1 },
         { "k32_xy", &t.ty, {4, 8, 16, 28}, "x-y tracer tile rows", 0 },
         { "k32_ztail", &t.lz, {8, 16, 32, 64}, "z levels per thread", 0 },
-        { "k32_par", &t.wpb_par, {1, 2, 4, 8}, "par warps/block", 32 },
+        { "k32_par|k32_par_divide", &t.wpb_par, {1, 2, 4, 8}, "par warps per 32 columns", 0 },
     };
     // the largest block each kernel can be launched with (registers per thread)
     auto max_threads = [](const char* kernel) -> int {

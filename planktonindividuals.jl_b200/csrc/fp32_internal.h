@@ -104,7 +104,7 @@ struct StepState {
     int64_t call_step;      // steps taken in the current update! call (time_offset indexing)
     int64_t err_iter;       // iteration at which a capacity error occurred
     int32_t err_member;     // member of that error
-    int32_t pad;
+    int32_t live;           // the step in progress began without an error (k32_begin)
 };
 
 // Individuals of all members and species.
@@ -127,6 +127,9 @@ struct IndDev32 {
     int32_t* phys;          // physical position (within the segment) of each logical slot
     uint32_t* freebits;     // bit set: the logical slot is inactive (MemberDev::woff layout)
     uint32_t* dvbits;       // bit set: the logical slot divides in this step
+    // per segment (shared by both physical buffers)
+    uint32_t* segdiv;       // dividers of this step
+    uint32_t* segfree;      // free slots
 };
 
 struct SpeciesDev32 {

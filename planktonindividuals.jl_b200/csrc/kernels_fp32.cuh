@@ -250,10 +250,6 @@ __device__ __forceinline__ T run_sum(T v, const WarpRuns& R) {
 // step prologue: forcing of the step, vel½
 // ------------------------------------------------------------------------------------------
 
-// update!'s forcing selection (Simulation/update.jl:14-26) for members with device-resident
-// series, from model.t before the step (or the step index of the call with time_offset), and the
-// choice of the vel½ buffer. Grid: (x blocks, members); block x = 0 binds the fields, every block
-// copies its share of the surface PAR snapshot.
 __device__ __forceinline__ long long snap_index(double tm, double tc, int use_call, double dT_s, long long n,
                                                 uint32_t* err, bool flag) {
     long long t = (long long)floor((use_call ? tc : tm) / dT_s);
@@ -261,52 +257,79 @@ __device__ __forceinline__ long long snap_index(double tm, double tc, int use_ca
     return t;
 }
 
-__global__ void k32_bind(int nm, const MemberDev* __restrict__ md, const MemberSeries* __restrict__ S,
-                         MemberForcing* __restrict__ F, const StepState* __restrict__ st, double dT,
-                         float* __restrict__ PARF, uint32_t* err) {
-    const int m = blockIdx.y;
-    if (m >= nm || stopped(err)) return;
-    const MemberSeries& s = S[m];
-    const MemberDev& M = md[m];
-    const double tm = st->t, tc = (double)st->call_step * dT;
+// The step's prologue in one launch (grid: x blocks, members), each block its share of a member:
+//  - update!'s forcing selection (Simulation/update.jl:14-26) for members with device-resident
+//    series, from model.t before the step (or the step index of the call with time_offset). Every
+//    block works it out from the tables; the first thread of block x = 0 writes it down, and only
+//    the entries that no other block reads here;
+//  - the surface PAR snapshot;
+//  - vel½ = (vel₀ + vel₁) * 0.5 (time_step.jl:17-19) when the two are different fields;
+//  - zeros in the per-cell counts (a memset and two kernels were three launches: 12 µs of a small
+//    model's step).
+struct BeginArgs {
+    const MemberDev* md;
+    const MemberSeries* S;
+    MemberForcing* F;
+    StepState* st;
+    double dT;
+    float* PARF;
+    int* pop;
+    int* pop_sp;               // nsp × Gtot or null
+    uint32_t *segdiv, *segfree;
+    int nsp;
+    long long Gtot;
+    uint32_t* err;
+};
+__global__ void k32_begin(BeginArgs a) {
+    const int mi = blockIdx.y;
     const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
-    if (lead) {
-        MemberForcing f = F[m];
-        if (s.has_series) {
-            if (s.has_vel) {
-                const long long tv = snap_index(tm, tc, s.time_offset & 1, s.dT_vel, s.nvel, err, true);
-                for (int c = 0; c < 3; ++c) f.vel1[c] = s.vel + (tv * 3 + c) * M.G;
-            }
-            f.temp = s.temp + snap_index(tm, tc, s.time_offset & 4, s.dT_temp, s.ntemp, err, true) * M.G;
+    const bool live = !stopped(a.err);
+    if (lead && mi == 0) a.st->live = live;
+    if (!live) return;
+    if (blockIdx.x == 0)
+        for (int q = mi * a.nsp + threadIdx.x; q < (mi + 1) * a.nsp; q += blockDim.x) {
+            a.segfree[q] -= a.segdiv[q];        // the slots taken in the step before
+            a.segdiv[q] = 0u;
         }
-        for (int c = 0; c < 3; ++c) f.velh[c] = (f.vel0[c] == f.vel1[c]) ? f.vel1[c] : s.velh_buf[c];
-        F[m] = f;
+    const MemberSeries& s = a.S[mi];
+    const MemberDev& M = a.md[mi];
+    const MemberForcing& F = a.F[mi];
+    const double tm = a.st->t, tc = (double)a.st->call_step * a.dT;
+    const long long t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x, nt = (long long)gridDim.x * blockDim.x;
+    const float *v0[3], *v1[3], *temp = nullptr;
+    for (int c = 0; c < 3; ++c) v0[c] = F.vel0[c];
+    if (s.has_series && s.has_vel) {
+        const long long tv = snap_index(tm, tc, s.time_offset & 1, s.dT_vel, s.nvel, a.err, lead);
+        for (int c = 0; c < 3; ++c) v1[c] = s.vel + (tv * 3 + c) * M.G;
+    } else {
+        for (int c = 0; c < 3; ++c) v1[c] = F.vel1[c];
+    }
+    if (s.has_series) temp = s.temp + snap_index(tm, tc, s.time_offset & 4, s.dT_temp, s.ntemp, a.err, lead) * M.G;
+    if (lead) {
+        MemberForcing& W = a.F[mi];
+        if (s.has_series && s.has_vel) for (int c = 0; c < 3; ++c) W.vel1[c] = v1[c];
+        if (s.has_series) W.temp = temp;
+        for (int c = 0; c < 3; ++c) W.velh[c] = v0[c] == v1[c] ? v1[c] : s.velh_buf[c];
+    }
+    // members start on multiples of 64 cells, so the counts are cleared 16 bytes at a time
+    const long long n4 = (M.G + 3) >> 2;
+    for (int p = -1; p < (a.pop_sp ? a.nsp : 0); ++p) {
+        int4* z = reinterpret_cast<int4*>((p < 0 ? a.pop : a.pop_sp + p * a.Gtot) + M.cell_off);
+        for (long long q = t0; q < n4; q += nt) z[q] = make_int4(0, 0, 0, 0);
+    }
+    if (v0[0] != v1[0]) {
+        float *h0 = s.velh_buf[0], *h1 = s.velh_buf[1], *h2 = s.velh_buf[2];
+        for (long long q = t0; q < M.G; q += nt) {
+            h0[q] = (v0[0][q] + v1[0][q]) * 0.5f;
+            h1[q] = (v0[1][q] + v1[1][q]) * 0.5f;
+            h2[q] = (v0[2][q] + v1[2][q]) * 0.5f;
+        }
     }
     if (!s.has_series) return;
-    const long long tp = snap_index(tm, tc, s.time_offset & 2, s.dT_PAR, s.npar, err, lead);
+    const long long tp = snap_index(tm, tc, s.time_offset & 2, s.dT_PAR, s.npar, a.err, lead);
     const long long n = (long long)M.Nx * M.Ny;
     const float* src = s.parf + tp * n;
-    for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x)
-        PARF[M.col_off + q] = src[q];
-}
-
-// vel½ = (vel₀ + vel₁) * 0.5 (time_step.jl:17-19) for members whose two fields differ.
-// Grid: (x blocks, members).
-__global__ void k32_velhalf(const MemberDev* __restrict__ md, const MemberForcing* __restrict__ F,
-                            const uint32_t* err) {
-    const int m = blockIdx.y;
-    if (stopped(err)) return;
-    const MemberForcing& f = F[m];
-    if (f.velh[0] == f.vel1[0]) return;
-    const long long G = md[m].G;
-    float* h0 = (float*)f.velh[0];
-    float* h1 = (float*)f.velh[1];
-    float* h2 = (float*)f.velh[2];
-    for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < G; q += (long long)gridDim.x * blockDim.x) {
-        h0[q] = (f.vel0[0][q] + f.vel1[0][q]) * 0.5f;
-        h1[q] = (f.vel0[1][q] + f.vel1[1][q]) * 0.5f;
-        h2[q] = (f.vel0[2][q] + f.vel1[2][q]) * 0.5f;
-    }
+    for (long long q = t0; q < n; q += nt) a.PARF[M.col_off + q] = src[q];
 }
 
 // ------------------------------------------------------------------------------------------
@@ -476,9 +499,15 @@ __device__ __forceinline__ MoveOut move_one(const MoveArgs& a, const MemberDev& 
     return out;
 }
 
-// k32_move's grid sums of one warp (segment s of one member): one atomic per run of a cell
-__device__ __forceinline__ void scatter_move(const MoveArgs& a, int s, const MoveOut& o) {
+// k32_move's grid sums of one warp (segment s of one member): one atomic per run of a cell; and the
+// segment's dividers and newly freed slots
+__device__ __forceinline__ void scatter_move(const MoveArgs& a, int s, int seg, const MoveOut& o) {
     if (__all_sync(0xffffffffu, o.cq < 0)) return;      // a warp of inactive slots adds nothing
+    const unsigned dv = __ballot_sync(0xffffffffu, o.cnt >> 24 != 0), fr = __ballot_sync(0xffffffffu, (o.cnt & 0xffff00u) != 0);
+    if ((threadIdx.x & 31) == 0) {
+        if (dv) atomicAdd(&a.P.segdiv[seg], __popc(dv));
+        if (fr) atomicAdd(&a.P.segfree[seg], __popc(fr));
+    }
     const WarpRuns R = warp_runs(o.cq);
     const uint32_t c = run_sum(o.cnt, R);
     const unsigned long long chl = run_sum(o.chl, R);
@@ -519,7 +548,7 @@ __global__ void __launch_bounds__(256, MINB) k32_move(MoveArgs a) {
             if (p + 1 < ppt) nx = move_state(a.P, base + slot + bs, slot + bs < m.C);
             MoveOut o{-1, 0u, 0ull};
             if (slot < m.C) o = move_one(a, m, sg, mi, s, base + slot, iter, cur);
-            scatter_move(a, s, o);
+            scatter_move(a, s, tl.x, o);
         }
         __syncthreads();
     }
@@ -532,73 +561,127 @@ __global__ void __launch_bounds__(256, MINB) k32_move(MoveArgs a) {
 // For every interior cell holding individuals it also packs the environment physiology gathers
 // (find_NPT!, utils.jl:14-25: NH4, NO3, PO4, DOC, par, temperature, pop) into one 32-byte record,
 // so an individual reads one sector instead of seven.
-#define PAR_CH 8      // levels whose loads are issued together (the column walk is a latency chain)
-__global__ void k32_par(Tab32 T, const float* __restrict__ dzF, const BgcDev32* __restrict__ bgc,
-                        unsigned long long* __restrict__ chl_acc, float* __restrict__ PARF,
-                        float* __restrict__ par, float* __restrict__ diag_par, const float* __restrict__ tr,
-                        long long Gtot, const MemberForcing* __restrict__ F, const int* __restrict__ pop,
-                        float4* __restrict__ env, const uint32_t* err) {
-    if (stopped(err)) return;
-    const int lane = threadIdx.x & 31;
-    const int nw = (gridDim.x * blockDim.x) >> 5;
-    for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < T.nicol; w += nw) {
-        const int4 it = T.icol[w];
-        const MemberDev& m = T.md[it.x];
-        const int i = it.y + lane, j = it.z;     // 1-based interior column
-        if (i > m.Nx) continue;
-        const float kc = bgc[it.x].kc, kw = bgc[it.x].kw;
-        const long long fcol = m.col_off + (i - 1) + (long long)m.Nx * (j - 1);
-        float parf = PARF[fcol];
-        const long long c1 = m.cell_off + gid3(m, i + m.Hx, j + m.Hy, 1 + m.Hz);
-        const long long slab = (long long)m.Gx * m.Gy;
-        const float* __restrict__ temp = F[it.x].temp;
-        const float areaf = m.dx * m.dy;
-        for (int k0 = 1; k0 <= m.Nz; k0 += PAR_CH) {
-            // the loads of PAR_CH levels first (only PARF carries down the column)
+//
+// One thread walking a column waits for memory level by level, and 32 columns are one warp (ncu on
+// 128×128×64: 5 % of the warps resident, 34 µs at 9 % of DRAM). So 1, 2, 4 or 8 warps take the same 32
+// columns: each forms the attenuation of PAR_CH levels, the first carries the light down through
+// shared memory (one product per level), and all write their levels.
+#define PAR_CH 8
+#define PAR_WARPS 8
+struct ParArgs {
+    Tab32 T;
+    const float* dzF;
+    const BgcDev32* bgc;
+    unsigned long long* chl_acc;
+    float* PARF;
+    float* par;
+    float* diag_par;
+    const float* tr;
+    long long Gtot;
+    const MemberForcing* F;
+    const int* pop;
+    float4* env;
+    const StepState* st;
+    int lw;                    // warps per 32 columns: 1, 2, 4 or 8
+    int maxNz;
+};
+// the 32-column items of one block of PAR_WARPS warps
+__device__ __forceinline__ void par_columns(const ParArgs& a, int block) {
+    __shared__ float sEx[PAR_WARPS * PAR_CH][32], sIn[PAR_WARPS * PAR_CH][32];
+    if (!a.st->live) return;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, lw = a.lw;
+    const int part = wid & (lw - 1), row0 = wid * PAR_CH;           // rows of this warp in shared memory
+    const int w = block * (PAR_WARPS / lw) + wid / lw;
+    const bool has = w < a.T.nicol;
+    const int4 it = a.T.icol[has ? w : 0];
+    const MemberDev& m = a.T.md[it.x];
+    const int Nz = m.Nz, Hz = m.Hz;
+    const int i = it.y + lane, j = it.z;                            // 1-based interior column
+    const bool col = has && i <= m.Nx;
+    const float kc = a.bgc[it.x].kc, kw = a.bgc[it.x].kw;
+    const long long fcol = m.col_off + (i - 1) + (long long)m.Nx * (j - 1);
+    const int q1 = gid3(m, i + m.Hx, j + m.Hy, 1 + Hz), slab = m.Gx * m.Gy;
+    const long long off = m.cell_off;
+    const double chl_unit = m.chl_unit;
+    const float areaf = m.dx * m.dy;
+    const float* dzp = a.dzF + m.dz_off + Hz;
+    const float* temp = a.F[it.x].temp;
+    const int* pop = a.pop + off;
+    const float* tr = a.tr + off;
+    unsigned long long* chl_acc = a.chl_acc + off;
+    float *par = a.par + off, *diag = a.diag_par + off;
+    float4* env = a.env + 2 * off;
+    float parf = col && part == 0 ? a.PARF[fcol] : 0.0f;
+    for (int kc0 = 0; kc0 < a.maxNz; kc0 += PAR_CH * lw) {          // same trip count for every warp
+        const int k0 = kc0 + part * PAR_CH;                         // 0-based levels k0 .. k0 + PAR_CH - 1
+        float ex[PAR_CH], at[PAR_CH];
+        int pp[PAR_CH];
+        if (col) {
             long long v[PAR_CH];
-            int pp[PAR_CH];
-            float dp[PAR_CH], dz[PAR_CH];
 #pragma unroll
             for (int e = 0; e < PAR_CH; ++e) {
-                const int k = k0 + e;
-                const long long c = c1 + (k - 1) * slab;
-                const bool in = k <= m.Nz;
-                v[e] = in ? (long long)chl_acc[c] : 0;
-                pp[e] = in ? pop[c] : 0;
-                dp[e] = in ? diag_par[c] : 0.0f;
-                dz[e] = in ? dzF[m.dz_off + k + m.Hz - 1] : 1.0f;
+                const bool in = k0 + e < Nz;
+                const int q = q1 + (k0 + e) * slab;
+                v[e] = in ? (long long)chl_acc[q] : 0;
+                pp[e] = in ? __ldg(pop + q) : 0;
             }
-            float pvs[PAR_CH];
 #pragma unroll
             for (int e = 0; e < PAR_CH; ++e) {
-                const int k = k0 + e;
-                if (k > m.Nz) { pvs[e] = 0.0f; continue; }
-                const long long c = c1 + (k - 1) * slab;
-                if (v[e]) chl_acc[c] = 0ull;
-                const float chl = (float)((double)v[e] * m.chl_unit);
-                const float volk = areaf * dz[e];
-                const float atten = (chl / volk * kc + kw) * dz[e];
-                const float ex = expf(-atten);
-                const float pv = parf * (1.0f - ex) / atten;
-                par[c] = pv;
-                parf = parf * ex;
-                diag_par[c] = dp[e] + pv;
-                pvs[e] = pv;
-            }
-            // environment records of the occupied cells of these levels
-#pragma unroll
-            for (int e = 0; e < PAR_CH; ++e) {
-                const int k = k0 + e;
-                if (k > m.Nz || pp[e] <= 0) continue;
-                const long long c = c1 + (k - 1) * slab;
-                env[2 * c] = make_float4(tr[PI_NH4 * Gtot + c], tr[PI_NO3 * Gtot + c], tr[PI_PO4 * Gtot + c],
-                                         tr[PI_DOC * Gtot + c]);
-                env[2 * c + 1] = make_float4(pvs[e], temp[c - m.cell_off], (float)pp[e], 0.0f);
+                if (k0 + e >= Nz) continue;
+                if (v[e]) chl_acc[q1 + (k0 + e) * slab] = 0ull;
+                const float dz = __ldg(dzp + k0 + e);
+                const float chl = (float)((double)v[e] * chl_unit);
+                at[e] = (chl / (areaf * dz) * kc + kw) * dz;
+                ex[e] = expf(-at[e]);
+                sEx[row0 + e][lane] = ex[e];
             }
         }
-        PARF[fcol] = parf;
+        __syncthreads();
+        if (part == 0 && col) {
+            const int n = min(PAR_CH * lw, Nz - kc0);
+            for (int e = 0; e < n; ++e) {
+                sIn[row0 + e][lane] = parf;
+                parf = parf * sEx[row0 + e][lane];
+            }
+        }
+        __syncthreads();
+        if (col) {
+            // four levels' loads (diagnostics, and the environment of occupied cells) at a time
+#pragma unroll
+            for (int g = 0; g < PAR_CH; g += 4) {
+                float dp[4];
+                float4 nv[4];
+                float tv[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int q = q1 + (k0 + g + e) * slab;
+                    dp[e] = k0 + g + e < Nz ? diag[q] : 0.0f;
+                    if (pp[g + e] > 0) {
+                        nv[e] = make_float4(__ldg(tr + PI_NH4 * a.Gtot + q), __ldg(tr + PI_NO3 * a.Gtot + q),
+                                            __ldg(tr + PI_PO4 * a.Gtot + q), __ldg(tr + PI_DOC * a.Gtot + q));
+                        tv[e] = __ldg(temp + q);
+                    }
+                }
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    if (k0 + g + e >= Nz) continue;
+                    const int q = q1 + (k0 + g + e) * slab;
+                    const float pv = sIn[row0 + g + e][lane] * (1.0f - ex[g + e]) / at[g + e];
+                    par[q] = pv;
+                    diag[q] = dp[e] + pv;
+                    if (pp[g + e] > 0) {
+                        env[2 * q] = nv[e];
+                        env[2 * q + 1] = make_float4(pv, tv[e], (float)pp[g + e], 0.0f);
+                    }
+                }
+            }
+        }
+        __syncthreads();
     }
+    if (col && part == 0) a.PARF[fcol] = parf;
 }
+
+__global__ void __launch_bounds__(32 * PAR_WARPS, 3) k32_par(ParArgs a) { par_columns(a, blockIdx.x); }
 
 // ------------------------------------------------------------------------------------------
 // (e) division: k-th divider (logical slot order) → k-th free logical slot (findall(!ac),
@@ -792,8 +875,41 @@ __global__ void k32_assign(Tab32 T, IndDev32 P, const unsigned long long* __rest
     }
 }
 
-// copy_daughter_individuals! and divide_to_half! (division_death.jl:28-63). The lists hold logical
-// slots; phys gives where each is stored. Grid: (x, segments).
+// copy_daughter_individuals! and divide_to_half! (division_death.jl:28-63) of one divider and its
+// daughter's slot (logical slots of segment base; phys gives where each is stored).
+__device__ __forceinline__ void daughter_one(const IndDev32& P, const MemberDev& m, int s, long long base, int pl, int dl,
+                                             uint32_t* err) {
+    if (pl < 0 || pl >= m.C || dl < 0 || dl >= m.C) { seterr(err, F32_ERR_LISTS); return; }
+    const int pp = P.phys[base + pl], dp = P.phys[base + dl];
+    if (pp < 0 || pp >= m.C || dp < 0 || dp >= m.C) { seterr(err, F32_ERR_LISTS); return; }
+    const long long p = base + pp, d = base + dp;
+    // all reads first: the mother's and the daughter's slots are different
+    const int32_t cd = P.cell[d], cp = P.cell[p];
+    const float ox = P.ox[p], oy = P.oy[p], oz = P.oz[p];
+    const float Bm = P.Bm[p] * 0.5f, Cq = P.Cq[p] * 0.5f, Nq = P.Nq[p] * 0.5f, Pq = P.Pq[p] * 0.5f;
+    const float Chl = P.Chl[p] * 0.5f, gen = P.gen[p] + 1.0f;
+    const float aged = P.age[d] * 0.0f, agep = P.age[p] * 0.0f;
+    const uint8_t std_ = P.stat[d];
+    // the daughter's slot keeps the cell find_inds! gave it this step
+    int32_t sc;
+    if (cd < 0) sc = pack_halo(m, m.Hx, m.Hy, m.Hz);
+    else { int a0, a1, a2; unpack_int(m, cd, a0, a1, a2); sc = pack_halo(m, a0 + 1 + m.Hx, a1 + 1 + m.Hy, a2 + 1 + m.Hz); }
+    P.scell[d] = sc;
+    P.cell[d] = cp;
+    P.ox[d] = ox; P.oy[d] = oy; P.oz[d] = oz;
+    P.Bm[d] = Bm; P.Cq[d] = Cq; P.Nq[d] = Nq; P.Pq[d] = Pq; P.Chl[d] = Chl; P.gen[d] = gen;
+    P.age[d] = aged;
+    P.Bm[p] = Bm; P.Cq[p] = Cq; P.Nq[p] = Nq; P.Pq[p] = Pq; P.Chl[p] = Chl; P.gen[p] = gen;
+    P.age[p] = agep;
+    P.flags[d] = F32_AC | F32_DVID;
+    P.stat[d] = (uint8_t)((std_ & F32_ST_AC0) | F32_ST_STALE);
+    long long w;
+    uint32_t bit;
+    slot_bit(m, s, dl, w, bit);
+    atomicAnd(&P.freebits[w], ~bit);
+}
+
+// Grid: (x, segments).
 __global__ void k32_daughters(Tab32 T, IndDev32 P, const int* __restrict__ divlist,
                               const int* __restrict__ freelist, const uint32_t* __restrict__ ndiv,
                               uint32_t* err) {
@@ -805,31 +921,99 @@ __global__ void k32_daughters(Tab32 T, IndDev32 P, const int* __restrict__ divli
     const long long base = m.slot_off + (long long)s * m.C;
     const uint32_t n = ndiv[seg];
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        const int pl = divlist[base + k], dl = freelist[base + k];
-        if (k >= (uint32_t)m.C || pl < 0 || pl >= m.C || dl < 0 || dl >= m.C) { seterr(err, F32_ERR_LISTS); continue; }
-        const int pp = P.phys[base + pl], dp = P.phys[base + dl];
-        if (pp < 0 || pp >= m.C || dp < 0 || dp >= m.C) { seterr(err, F32_ERR_LISTS); continue; }
-        const long long p = base + pp, d = base + dp;
-        // the daughter's slot keeps the cell find_inds! gave it this step
-        const int32_t cd = P.cell[d];
-        int32_t sc;
-        if (cd < 0) sc = pack_halo(m, m.Hx, m.Hy, m.Hz);
-        else { int a0, a1, a2; unpack_int(m, cd, a0, a1, a2); sc = pack_halo(m, a0 + 1 + m.Hx, a1 + 1 + m.Hy, a2 + 1 + m.Hz); }
-        P.scell[d] = sc;
-        P.cell[d] = P.cell[p];
-        P.ox[d] = P.ox[p]; P.oy[d] = P.oy[p]; P.oz[d] = P.oz[p];
-        const float Bm = P.Bm[p] * 0.5f, Cq = P.Cq[p] * 0.5f, Nq = P.Nq[p] * 0.5f, Pq = P.Pq[p] * 0.5f;
-        const float Chl = P.Chl[p] * 0.5f, gen = P.gen[p] + 1.0f;
-        P.Bm[d] = Bm; P.Cq[d] = Cq; P.Nq[d] = Nq; P.Pq[d] = Pq; P.Chl[d] = Chl; P.gen[d] = gen;
-        P.age[d] = P.age[d] * 0.0f;
-        P.Bm[p] = Bm; P.Cq[p] = Cq; P.Nq[p] = Nq; P.Pq[p] = Pq; P.Chl[p] = Chl; P.gen[p] = gen;
-        P.age[p] = P.age[p] * 0.0f;
-        P.flags[d] = F32_AC | F32_DVID;
-        P.stat[d] = (uint8_t)((P.stat[d] & F32_ST_AC0) | F32_ST_STALE);
-        long long w;
-        uint32_t bit;
-        slot_bit(m, s, dl, w, bit);
-        atomicAnd(&P.freebits[w], ~bit);
+        if (k >= (uint32_t)m.C) { seterr(err, F32_ERR_LISTS); continue; }
+        daughter_one(P, m, s, base, divlist[base + k], freelist[base + k], err);
+    }
+}
+
+// Division of a whole segment by one block (DIV_WARPS warps): k32_count_tiles, k32_scan_tiles,
+// k32_assign and k32_daughters in one, for segments of at most DIV_WORDS bitmap words. Each warp
+// counts a run of words, the warps' counts are added up in shared memory, and each warp walks its
+// run again to list its dividers and the free slots they take.
+#define DIV_WARPS 8
+#define DIV_WORDS 8192
+struct DivArgs {
+    Tab32 T;
+    IndDev32 P;
+    int* divlist;
+    int* freelist;
+    int nseg;
+    StepState* st;
+    uint32_t* err;
+};
+__device__ __forceinline__ void divide_segment(const DivArgs& a, int seg) {
+    __shared__ uint32_t shd[DIV_WARPS], shf[DIV_WARPS];
+    const IndDev32& P = a.P;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    int mi, s;
+    seg_of(a.T, seg, mi, s);
+    const MemberDev& m = a.T.md[mi];
+    const long long base = m.slot_off + (long long)s * m.C, wbase = m.woff + (long long)s * m.wps;
+    const uint32_t tdiv = P.segdiv[seg];
+    // the capacity check (plankton_update.jl:18-22): the step divides in every segment or in none,
+    // so every block looks at all of them (k32_move's counts, which nothing changes here)
+    bool over = false;
+    for (int q = threadIdx.x; q < a.nseg; q += blockDim.x) over |= P.segdiv[q] > P.segfree[q];
+    if (__syncthreads_or(over)) {
+        if (threadIdx.x == 0 && tdiv > P.segfree[seg] && !(atomicOr(a.err, F32_ERR_CAPACITY) & F32_ERR_CAPACITY)) {
+            a.st->err_iter = a.st->iteration + 1;
+            a.st->err_member = mi;
+        }
+        return;
+    }
+    if (tdiv == 0) return;
+    const int words = (int)m.wps, run = (words / 32 + DIV_WARPS - 1) / DIV_WARPS * 32;
+    const int w0 = min(wid * run, words), w1 = min(w0 + run, words);
+    unsigned nd = 0, nf = 0;
+#pragma unroll 4
+    for (int w = w0; w < w1; w += 32) {
+        nd += (unsigned)__popc(P.dvbits[wbase + w + lane]);
+        nf += (unsigned)__popc(P.freebits[wbase + w + lane]);
+    }
+    nd = __reduce_add_sync(0xffffffffu, nd);
+    nf = __reduce_add_sync(0xffffffffu, nf);
+    if (lane == 0) { shd[wid] = nd; shf[wid] = nf; }
+    __syncthreads();
+    unsigned cdiv = 0, cfree = 0, dbefore = 0, fbefore = 0;
+#pragma unroll
+    for (int q = 0; q < DIV_WARPS; ++q) {
+        if (q < wid) { dbefore += shd[q]; fbefore += shf[q]; }
+        cdiv += shd[q]; cfree += shf[q];
+    }
+    if (cdiv != tdiv || tdiv > cfree) {           // the bitmaps hold what k32_move counted
+        if (threadIdx.x == 0) seterr(a.err, F32_ERR_LISTS);
+        return;
+    }
+    for (int w = w0; w < w1 && (nd || fbefore < tdiv); w += 32) {
+        uint32_t dw = nd ? P.dvbits[wbase + w + lane] : 0u, fw = fbefore < tdiv ? P.freebits[wbase + w + lane] : 0u;
+        if (dw) P.dvbits[wbase + w + lane] = 0u;
+        const unsigned cd = (unsigned)__popc(dw), cf = (unsigned)__popc(fw);
+        unsigned rd = dbefore + warp_exscan(cd), rf = fbefore + warp_exscan(cf);
+        dbefore += __reduce_add_sync(0xffffffffu, cd);
+        fbefore += __reduce_add_sync(0xffffffffu, cf);
+        const int L0 = (w + lane) * 32;
+        while (dw) {
+            a.divlist[base + rd++] = L0 + __ffs(dw) - 1;
+            dw &= dw - 1u;
+        }
+        while (fw && rf < tdiv) {
+            a.freelist[base + rf++] = L0 + __ffs(fw) - 1;
+            fw &= fw - 1u;
+        }
+    }
+    __syncthreads();
+    for (unsigned k = threadIdx.x; k < tdiv; k += blockDim.x)
+        daughter_one(P, m, s, base, a.divlist[base + k], a.freelist[base + k], a.err);
+}
+
+// Division and light depend on k32_move only and touch different arrays, so small models run both
+// in one launch: blocks 0 .. nseg - 1 divide a segment each, the others take the columns. Both go by
+// the step's `live` mark: a step that a dividing block stops still has its light.
+__global__ void __launch_bounds__(32 * DIV_WARPS, 3) k32_par_divide(ParArgs pa, DivArgs da) {
+    if ((int)blockIdx.x < da.nseg) {
+        if (da.st->live) divide_segment(da, blockIdx.x);
+    } else {
+        par_columns(pa, blockIdx.x - da.nseg);
     }
 }
 
