@@ -83,7 +83,7 @@ struct Tuning {
     int lz = 32;                              // levels walked by a z thread (8, 16, 32 or 64)
     int wpb_par = 0;                          // warps per 32 columns of k32_par (0: by the levels)
     int occ_move = 2, occ_phys = 4;           // register fit of k32_move / k32_physiology (blocks of 256 per SM)
-    int concurrent = 0;                       // k32_xy on a second branch beside the particle kernels
+    int concurrent = -1;                      // k32_xy on a second branch beside the particle kernels (-1: by its size)
     int fused = 0;                            // k32_tracer when the batch allows it (the autotuner
                                               // picks it where it beats k32_xy + k32_ztail + halo fill)
     int lz_fused = 32;                        // levels finished per k32_tracer block
@@ -514,7 +514,10 @@ pi_status enqueue_step(pi_batch* b, double dT, int cur) {
         else if (ty == 8) k32_xy<8><<<grid, 32 * 12, xy_smem(8), st>>>(a);
         else k32_xy<4><<<grid, 32 * 8, xy_smem(4), st>>>(a);
     };
-    const bool branch = !fused && b->tune.concurrent;
+    // beside the particle kernels when it leaves at least half of the SMs to them (measured per
+    // step: 0D parcel 38.6 -> 34.3 µs, 128×128×1 gyre 49.9 -> 45.1, 64 parcels 93.6 -> 89.0; no gain
+    // at 96×80×24 (114.5 -> 116.9) and above, where the two compete)
+    const bool branch = !fused && (b->tune.concurrent < 0 ? 2 * b->nxy_items <= b->nsm : b->tune.concurrent);
     if (branch) {
         BK(cudaEventRecord(b->ev_fork, s), "fork");
         BK(cudaStreamWaitEvent(b->s2, b->ev_fork, 0), "fork");
