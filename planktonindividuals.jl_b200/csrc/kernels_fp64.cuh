@@ -1022,163 +1022,6 @@ __device__ __forceinline__ FaceCoef face_coef(double vel, double area, double dx
     f.hm = 0.5 * (tr - fabs(tr));
     return f;
 }
-__device__ __forceinline__ double psi_c(const FaceCoef& f, double th) {
-    return jl_max(0.0, jl_min(jl_min(1.0, f.d0c + f.d1c * th), th * f.omc / f.cpe));
-}
-// adv_flux_x / adv_flux_y at face i from c[i-2], c[i-1], c[i], c[i+1]
-__device__ __forceinline__ double flux_xy_c(const FaceCoef& f, double cm2, double cm1, double c0, double cp1,
-                                            int lm2, int lm1, int l0, int lp1) {
-    double d0 = jl_mulb(jl_mulb(c0 - cm1, l0), lm1);
-    double dm = jl_mulb(jl_mulb(cm1 - cm2, lm1), lm2);
-    double dp = jl_mulb(jl_mulb(cp1 - c0, lp1), l0);
-    double psp = psi_c(f, theta(dm, d0));
-    double psm = psi_c(f, theta(dp, d0));
-    return f.hp * (cm1 + psp * d0) + f.hm * (c0 - psm * d0);
-}
-// adv_flux_z at face k from c[k-2], c[k-1], c[k], c[k+1] (index grows downward)
-__device__ __forceinline__ double flux_z_c(const FaceCoef& f, double cm2, double cm1, double c0, double cp1,
-                                           int lm2, int lm1, int l0, int lp1) {
-    double d0 = jl_mulb(jl_mulb(cm1 - c0, l0), lm1);
-    double dm = jl_mulb(jl_mulb(cm2 - cm1, lm1), lm2);
-    double dp = jl_mulb(jl_mulb(c0 - cp1, lp1), l0);
-    double psp = psi_c(f, theta(dm, d0));
-    double psm = psi_c(f, theta(dp, d0));
-    return f.hp * (c0 + psm * d0) + f.hm * (cm1 - psp * d0);
-}
-
-// x sweep (calc_Gcˣ + fill_halo_Gcs + multi_dim_x on tracer_temp = tracer). Each warp owns 31
-// cells of one row and 32 faces: lane l computes the flux of face i0 + l once, and the east-face
-// flux of its cell comes from lane l + 1 by shuffle. The face after the last interior cell follows
-// fill_halo_Gcs!: the periodic image of face H+1, or zero when Bounded.
-#define SWX_WARPS 4
-template <bool LL>
-__global__ void __launch_bounds__(32 * SWX_WARPS) k_sweep_x(DGrid g, const double* __restrict__ tr,
-                                                            double* __restrict__ tta,
-                                                            const double* __restrict__ u, double dT,
-                                                            const uint32_t* err) {
-    if (*err & PI_DEVERR_CAPACITY) return;
-    const int lane = threadIdx.x & 31;
-    const int wid = blockIdx.x * SWX_WARPS + (threadIdx.x >> 5);
-    const int i0 = wid * 31 + 1 + g.Hx;
-    if (i0 > g.Nx + g.Hx) return;                    // uniform per warp
-    const int j = blockIdx.y + 1 + g.Hy, k = blockIdx.z + 1 + g.Hz;
-    const int f = i0 + lane;                         // this lane's face (west face of cell f)
-    const int last = g.Nx + g.Hx;
-    const bool has_face = f <= last + 1;
-    const bool has_cell = lane < 31 && f <= last;
-    const bool special = f == last + 1;
-    const bool zero_face = !has_face || (special && g.tx != PI_PERIODIC);
-    const int fs = special ? g.Hx + 1 : f;           // face whose stencil gives the flux
-    const long long G = g.G;
-    const double ax = g.dy * dzF1(g, k);             // Ax of a RectilinearGrid
-    const int qf = gidx(g, has_face ? fs : i0, j, k);
-    FaceCoef fc{};
-    int lm2 = 1, lm1 = 1, l0 = 1, lp1 = 1;
-    if (!zero_face) {
-        fc = face_coef(u[qf], LL ? Axm<LL>(g, fs, j, k) : ax, dxCm<LL>(g, fs, j), dT);
-        lm2 = lmask(g, fs - 2, j, k); lm1 = lmask(g, fs - 1, j, k); l0 = lmask(g, fs, j, k); lp1 = lmask(g, fs + 1, j, k);
-    }
-    const int qc = gidx(g, has_cell ? f : i0, j, k);
-    double ftr = 0.0, dtv = 0.0;
-    int cl0 = 1, clp = 1;
-    if (has_cell) {
-        cl0 = lmask(g, f, j, k); clp = lmask(g, f + 1, j, k);
-        ftr = jl_mulb(jl_mulb((LL ? Axm<LL>(g, f + 1, j, k) : ax) * u[qc + 1] - (LL ? Axm<LL>(g, f, j, k) : ax) * u[qc], clp), cl0);
-        dtv = dT / vol<LL>(g, f, j, k);
-    }
-#pragma unroll 2
-    for (int n = 0; n < PI_NTRACERS; ++n) {
-        const double* c = tr + n * G;
-        double F = zero_face ? 0.0 : flux_xy_c(fc, c[qf - 2], c[qf - 1], c[qf], c[qf + 1], lm2, lm1, l0, lp1);
-        double Fe = __shfl_down_sync(0xffffffffu, F, 1);
-        if (has_cell) {
-            double c0 = c[qc];
-            double dG = jl_mulb(jl_mulb(Fe - F, clp), cl0);
-            tta[n * G + qc] = c0 - dtv * (dG - c0 * ftr);
-        }
-    }
-}
-
-// y sweep on tracer_temp after x (multi_dim_y, original tracer in the update term). Each thread
-// walks SWY_L cells along y carrying the face flux (each face computed once, plus one shared face
-// per segment), tracer by tracer so a thread holds one running flux; lanes run along x for
-// coalesced access. Rows outside the interior are read through the periodic or clamped map the
-// halo fill of tracer_temp produces.
-#define SWY_L 8
-#define SWY_TY 4
-template <bool LL>
-__device__ __forceinline__ double yface_flux(const DGrid& g, const double* __restrict__ c,
-                                             const double* __restrict__ v, int i, int f, int k,
-                                             double ay, double dT) {
-    const bool special = f == g.Ny + g.Hy + 1;
-    if (special && g.ty != PI_PERIODIC) return 0.0;            // fill_halo_north_Gc! (Bounded)
-    const int fs = special ? g.Hy + 1 : f;                      // periodic: Gc[N+H+1] = Gc[H+1]
-    FaceCoef fc = face_coef(v[gidx(g, i, fs, k)], LL ? Aym<LL>(g, i, fs, k) : ay, dyCm<LL>(g, i, fs), dT);
-    int r0 = gidx(g, i, wrap_axis(fs - 2, g.Ny, g.Hy, g.ty), k), r1 = gidx(g, i, wrap_axis(fs - 1, g.Ny, g.Hy, g.ty), k);
-    int r2 = gidx(g, i, wrap_axis(fs, g.Ny, g.Hy, g.ty), k), r3 = gidx(g, i, wrap_axis(fs + 1, g.Ny, g.Hy, g.ty), k);
-    return flux_xy_c(fc, c[r0], c[r1], c[r2], c[r3], lmask(g, i, fs - 2, k), lmask(g, i, fs - 1, k),
-                     lmask(g, i, fs, k), lmask(g, i, fs + 1, k));
-}
-
-template <bool LL>
-__global__ void __launch_bounds__(32 * SWY_TY, 8) k_sweep_y(DGrid g, const double* __restrict__ tr,
-                                                         const double* __restrict__ tta,
-                                                         double* __restrict__ ttb,
-                                                         const double* __restrict__ v, double dT,
-                                                         const uint32_t* err) {
-    if (*err & PI_DEVERR_CAPACITY) return;
-    const int i = blockIdx.x * 32 + threadIdx.x + 1 + g.Hx;
-    const int j0 = (blockIdx.y * SWY_TY + threadIdx.y) * SWY_L + 1 + g.Hy;
-    const int k = blockIdx.z + 1 + g.Hz;
-    if (i > g.Nx + g.Hx || j0 > g.Ny + g.Hy) return;
-    const int jend = min(j0 + SWY_L - 1, g.Ny + g.Hy);
-    const long long G = g.G;
-    // the face area and ΔT/volume of a RectilinearGrid are the same for every row
-    const double ay = g.dx * dzF1(g, k);
-    const double dtv0 = dT / vol<false>(g, i, j0, k);
-#pragma unroll 1
-    for (int t = 0; t < PI_NTRACERS; ++t) {
-        const double* c = tta + t * G;
-        double Ft = yface_flux<LL>(g, c, v, i, j0, k, ay, dT);
-        for (int jj = j0; jj <= jend; ++jj) {
-            double Fb = yface_flux<LL>(g, c, v, i, jj + 1, k, ay, dT);
-            const int q = gidx(g, i, jj, k);
-            const int cl0 = lmask(g, i, jj, k), clp = lmask(g, i, jj + 1, k);
-            const double dtv = LL ? dT / vol<LL>(g, i, jj, k) : dtv0;
-            const double ayp = LL ? Aym<LL>(g, i, jj + 1, k) : ay, ay0 = LL ? Aym<LL>(g, i, jj, k) : ay;
-            const double ftr = jl_mulb(jl_mulb(ayp * v[q + g.Gx] - ay0 * v[q], clp), cl0);
-            double dG = jl_mulb(jl_mulb(Fb - Ft, clp), cl0);
-            ttb[t * G + q] = c[q] - dtv * (dG - tr[t * G + q] * ftr);
-            Ft = Fb;
-        }
-    }
-}
-
-struct ZFinalArgs {
-    DGrid g;
-    const double* gadv;      // 14 × G, advective tendency from k_sweep_z
-    const double* tr;        // 14 × G, current tracers
-    const double* ttb;       // 14 × G, tracer_temp after x and y
-    double* tr_next;         // 14 × G
-    const double* w;
-    double dT;
-    pi_bgc_params b;
-    int diffuse;             // κh or κv nonzero
-    int any_bc;
-    const FluxBCDev* bcs;    // [14][6]
-    int64_t iter;
-    // particle contributions (plk)
-    const SpcDev* spc;
-    long long C;
-    const uint32_t* off;
-    const uint32_t* gid_sorted;
-    const uint8_t* evk;
-    const double* loss;
-    const double* contrib;
-    int nsp;
-    const uint32_t* err;
-};
-
 __device__ __forceinline__ double getbc_dev(const FluxBCDev& b, int a, int c, int64_t it) {
     if (b.kind == PI_BC_CONST) return b.v[0];
     if (b.kind == PI_BC_ARRAY2D) return b.v[(a - 1) + (long long)b.n1 * (c - 1)];
@@ -1186,201 +1029,8 @@ __device__ __forceinline__ double getbc_dev(const FluxBCDev& b, int a, int c, in
     return b.v[(a - 1) + (long long)b.n1 * ((c - 1) + (long long)b.n2 * (t - 1))];
 }
 
-#define SWZ_L 8
-#define SWZ_TZ 4
-// z sweep of multi_dim_z then calc_tracer_tendency!: Gc_adv = tracer_temp - tracer, written to
-// `gadv`. Each thread walks SWZ_L levels of one column carrying the z face flux, tracer by tracer;
-// levels outside the interior are read through the clamped map of the Bounded halo fill.
-__device__ __forceinline__ double zface_flux(const DGrid& g, const double* __restrict__ c,
-                                             const double* __restrict__ w, int i, int j, int f,
-                                             int qcol, int slab, double az, double dT) {
-    if (f == g.Nz + g.Hz + 1) return 0.0;                      // fill_halo_bottom_Gc! (Bounded)
-    FaceCoef fc = face_coef(w[qcol + (f - 1) * slab], az, dzC1(g, f), dT);
-    auto lev = [&](int kk) { return qcol + (wrap_axis(kk, g.Nz, g.Hz, PI_BOUNDED) - 1) * slab; };
-    return flux_z_c(fc, c[lev(f - 2)], c[lev(f - 1)], c[lev(f)], c[lev(f + 1)], lmask(g, i, j, f - 2),
-                    lmask(g, i, j, f - 1), lmask(g, i, j, f), lmask(g, i, j, f + 1));
-}
-
-template <bool LL>
-__global__ void __launch_bounds__(32 * SWZ_TZ, 8) k_sweep_z(DGrid g, const double* __restrict__ tr,
-                                                         const double* __restrict__ ttb,
-                                                         double* __restrict__ gadv,
-                                                         const double* __restrict__ w, double dT,
-                                                         const uint32_t* err) {
-    if (*err & PI_DEVERR_CAPACITY) return;
-    const int i = blockIdx.x * 32 + threadIdx.x + 1 + g.Hx;
-    const int j = blockIdx.y + 1 + g.Hy;
-    const int k0 = (blockIdx.z * SWZ_TZ + threadIdx.y) * SWZ_L + 1 + g.Hz;
-    if (i > g.Nx + g.Hx || k0 > g.Nz + g.Hz) return;
-    const int kend = min(k0 + SWZ_L - 1, g.Nz + g.Hz);
-    const long long G = g.G;
-    const double az = Azm<LL>(g, i, j);
-    const int slab = g.Gx * g.Gy;
-    const int qcol = gidx(g, i, j, 1);
-#pragma unroll 1
-    for (int t = 0; t < PI_NTRACERS; ++t) {
-        const double* c = ttb + t * G;
-        double Ft = zface_flux(g, c, w, i, j, k0, qcol, slab, az, dT);
-        for (int k = k0; k <= kend; ++k) {
-            double Fb = zface_flux(g, c, w, i, j, k + 1, qcol, slab, az, dT);
-            const int q = qcol + (k - 1) * slab;
-            const int cl0 = lmask(g, i, j, k), clp = lmask(g, i, j, k + 1);
-            const double ftr = jl_mulb(jl_mulb(az * w[q] - az * w[q + slab], clp), cl0);
-            const double dG = jl_mulb(jl_mulb(Ft - Fb, clp), cl0);
-            const double cc = tr[t * G + q];
-            const double ct = c[q] - dT / vol<LL>(g, i, j, k) * (dG - cc * ftr);
-            gadv[t * G + q] = ct - cc;                          // calc_tracer_tendency!
-            Ft = Fb;
-        }
-    }
-}
-
-template <bool LL, bool IRON>
-__device__ __forceinline__ void z_final_cell(const ZFinalArgs& a, int i, int j, int k, int q, double volk, double* Gc);
-
-// Per interior cell: diffusion, sinking, forcing, flux BCs, particle terms and apply_tendency!
-// on top of the advective tendency of k_sweep_z (tracer_update.jl:22-43).
-template <bool LL, bool IRON = false>
-__global__ void __launch_bounds__(128, 6) k_tracer_tail(ZFinalArgs a) {
-    const DGrid& g = a.g;
-    if (*a.err & PI_DEVERR_CAPACITY) return;
-    const int i = blockIdx.x * 128 + threadIdx.x + 1 + g.Hx;
-    const int j = blockIdx.y + 1 + g.Hy;
-    const int k = blockIdx.z + 1 + g.Hz;
-    if (i > g.Nx + g.Hx) return;
-    const int q = gidx(g, i, j, k);
-    const long long G = g.G;
-    double Gc[PI_NTRACERS];
-#pragma unroll
-    for (int t = 0; t < PI_NTRACERS; ++t) Gc[t] = a.gadv[t * G + q];
-    z_final_cell<LL, IRON>(a, i, j, k, q, vol<LL>(g, i, j, k), Gc);
-}
-
-// The rest of tracer_update! for one interior cell, given its advective tendency Gc.
-template <bool LL, bool IRON>
-__device__ __forceinline__ void z_final_cell(const ZFinalArgs& a, int i, int j, int k, int q, double volk, double* Gc) {
-    const DGrid& g = a.g;
-    const long long G = g.G;
-    const double dT = a.dT;
-    const double az = Azm<LL>(g, i, j);
-    const int slab = g.Gx * g.Gy;
-    const pi_bgc_params& b = a.b;
-    // tracer_diffusion! (κ∇², tracer_diffusion.jl:1-21) on the original tracer
-    if (a.diffuse) {
-        double kx = b.kappa_h, ky = b.kappa_h, kz = b.kappa_v;
-        int li = lmask(g, i, j, k);
-#pragma unroll
-        for (int n = 0; n < PI_NTRACERS; ++n) {
-            const double* c = a.tr + n * G;
-            auto dx0 = [&](int ii) { return jl_mulb(jl_mulb(c[gidx(g, ii, j, k)] - c[gidx(g, ii - 1, j, k)], lmask(g, ii, j, k)), lmask(g, ii - 1, j, k)); };
-            auto dy0 = [&](int jj) { return jl_mulb(jl_mulb(c[gidx(g, i, jj, k)] - c[gidx(g, i, jj - 1, k)], lmask(g, i, jj, k)), lmask(g, i, jj - 1, k)); };
-            auto dz0 = [&](int kk) { return jl_mulb(jl_mulb(c[gidx(g, i, j, kk - 1)] - c[gidx(g, i, j, kk)], lmask(g, i, j, kk)), lmask(g, i, j, kk - 1)); };
-            double fx1 = kx * Axm<LL>(g, i + 1, j, k) * (dx0(i + 1) / dxFm<LL>(g, i + 1, j)), fx0 = kx * Axm<LL>(g, i, j, k) * (dx0(i) / dxFm<LL>(g, i, j));
-            double fy1 = ky * Aym<LL>(g, i, j + 1, k) * (dy0(j + 1) / dyFm<LL>(g, i, j + 1)), fy0 = ky * Aym<LL>(g, i, j, k) * (dy0(j) / dyFm<LL>(g, i, j));
-            double fz0 = kz * az * (dz0(k) / dzF1(g, k)), fz1 = kz * az * (dz0(k + 1) / dzF1(g, k + 1));
-            double ax_ = jl_mulb(jl_mulb(fx1 - fx0, lmask(g, i + 1, j, k)), li);
-            double ay_ = jl_mulb(jl_mulb(fy1 - fy0, lmask(g, i, j + 1, k)), li);
-            double az_ = jl_mulb(jl_mulb(fz0 - fz1, lmask(g, i, j, k + 1)), li);
-            double lap = 1.0 / volk * (ax_ + ay_ + az_);
-            Gc[n] = Gc[n] + lap * dT;
-        }
-    }
-    // tracer_sinking! (tracer_sinking.jl:1-42); flux_sink is zero on k <= Hz and k >= Nz+Hz
-    {
-        auto sink = [&](int n, double ws) {
-            const double* c = a.tr + n * G;
-            double fup = (k - 1 <= g.Hz || k - 1 >= g.Nz + g.Hz) ? 0.0 : ws * c[q - slab];
-            double fdn = (k >= g.Nz + g.Hz) ? 0.0 : ws * c[q];
-            return (fup - fdn) / dzC1(g, k - g.Hz) * dT;
-        };
-        Gc[PI_PFe_inorg] = Gc[PI_PFe_inorg] + sink(PI_PFe_inorg, b.w_sink_inorg);
-        Gc[PI_Dust] = Gc[PI_Dust] + sink(PI_Dust, b.w_sink_inorg);
-        Gc[PI_PFe_bio] = Gc[PI_PFe_bio] + sink(PI_PFe_bio, b.w_sink_org);
-    }
-    // tracer_forcing! (tracer_forcings.jl:2-50) on max(0, tracer)
-    {
-        double T[PI_NTRACERS];
-#pragma unroll
-        for (int n = 0; n < PI_NTRACERS; ++n) T[n] = jl_max(0.0, a.tr[n * G + q]);
-        Gc[PI_DIC] = Gc[PI_DIC] + T[PI_DOC] * b.kDOC * dT;
-        Gc[PI_DOC] = Gc[PI_DOC] - T[PI_DOC] * b.kDOC * dT + T[PI_POC] * b.kPOC * dT;
-        Gc[PI_POC] = Gc[PI_POC] - T[PI_POC] * b.kPOC * dT;
-        Gc[PI_NH4] = Gc[PI_NH4] + T[PI_DON] * b.kDON * dT - T[PI_NH4] * b.Nit * dT;
-        Gc[PI_NO3] = Gc[PI_NO3] + T[PI_NH4] * b.Nit * dT;
-        Gc[PI_DON] = Gc[PI_DON] - T[PI_DON] * b.kDON * dT + T[PI_PON] * b.kPON * dT;
-        Gc[PI_PON] = Gc[PI_PON] - T[PI_PON] * b.kPON * dT;
-        Gc[PI_PO4] = Gc[PI_PO4] + T[PI_DOP] * b.kDOP * dT;
-        Gc[PI_DOP] = Gc[PI_DOP] - T[PI_DOP] * b.kDOP * dT + T[PI_POP] * b.kPOP * dT;
-        Gc[PI_POP] = Gc[PI_POP] - T[PI_POP] * b.kPOP * dT;
-        Gc[PI_DFe] = Gc[PI_DFe] + T[PI_PFe_bio] * b.kPOC * dT
-                   - (b.lambda_POC * T[PI_POC] + b.lambda_min + b.lambda_dust * T[PI_Dust]) * T[PI_DFe] * b.DFeFrac * dT
-                   + T[PI_PFe_inorg] * b.kdiss * dT
-                   - jl_max((T[PI_DFe] - b.ligand), 0.0) * T[PI_DFe] * b.DFeFrac * b.lambda_Fe * dT;
-        Gc[PI_PFe_bio] = Gc[PI_PFe_bio] + T[PI_POC] * T[PI_DFe] * b.DFeFrac * b.lambda_POC * dT
-                       - b.kPOC * T[PI_PFe_bio] * dT;
-        Gc[PI_PFe_inorg] = Gc[PI_PFe_inorg] - T[PI_PFe_inorg] * b.kdiss * dT
-                         + (b.lambda_min + b.lambda_dust * T[PI_Dust]) * T[PI_DFe] * b.DFeFrac * dT
-                         + jl_max((T[PI_DFe] - b.ligand), 0.0) * T[PI_DFe] * b.DFeFrac * b.lambda_Fe * dT;
-    }
-    // apply_bcs! (apply_bcs.jl:4-98), faces in the reference's order
-    if (a.any_bc) {
-        int ii = i - g.Hx, jj = j - g.Hy, kk = k - g.Hz;
-        double axk = Axm<LL>(g, i, j, k), ayk = Aym<LL>(g, i, j, k);
-#pragma unroll
-        for (int n = 0; n < PI_NTRACERS; ++n) {
-            const FluxBCDev* B = a.bcs + n * 6;
-            if (B[PI_WEST].kind && i == 1 + g.Hx) Gc[n] += getbc_dev(B[PI_WEST], jj, kk, a.iter) * dT * axk / volk;
-            if (B[PI_EAST].kind && i == g.Nx + g.Hx) Gc[n] -= getbc_dev(B[PI_EAST], jj, kk, a.iter) * dT * axk / volk;
-            if (B[PI_SOUTH].kind && j == 1 + g.Hy) Gc[n] += getbc_dev(B[PI_SOUTH], ii, kk, a.iter) * dT * ayk / volk;
-            if (B[PI_NORTH].kind && j == g.Ny + g.Hy) Gc[n] -= getbc_dev(B[PI_NORTH], ii, kk, a.iter) * dT * ayk / volk;
-            if (B[PI_BOTTOM].kind && k == g.Nz + g.Hz) Gc[n] += getbc_dev(B[PI_BOTTOM], ii, jj, a.iter) * dT * az / volk;
-            if (B[PI_TOP].kind && k == 1 + g.Hz) Gc[n] -= getbc_dev(B[PI_TOP], ii, jj, a.iter) * dT * az / volk;
-        }
-    }
-    // plk: per-cell particle losses and consumption in reference summation order
-    double plk_DIC = 0.0, plk_NH4 = 0.0, plk_NO3 = 0.0, plk_PO4 = 0.0, plk_DOC = 0.0;
-    double plk_DON = 0.0, plk_DOP = 0.0, plk_POC = 0.0, plk_PON = 0.0, plk_POP = 0.0;
-    double plk_DFe = 0.0, plk_PFe = 0.0;         // IronEnergyMode only
-    {
-        uint32_t p0 = a.off[q], p1 = a.off[q + 1];
-        uint32_t p = p0;
-        while (p < p1) {
-            uint32_t s = a.gid_sorted[p] / (uint32_t)a.C;
-            uint32_t e = p;
-            while (e < p1 && a.gid_sorted[e] / (uint32_t)a.C == s) ++e;
-            for (int pass = 1; pass <= 2; ++pass)
-                for (uint32_t r = p; r < e; ++r)
-                    if (a.evk[r] == pass) {
-                        if (IRON) {                  // NH4, NO3, DOC, DON, DOP, DFe, POC, PON, POP, PFe_bio
-                            const double* L = a.loss + (long long)r * 10;
-                            plk_NH4 += L[0]; plk_NO3 += L[1]; plk_DOC += L[2]; plk_DON += L[3]; plk_DOP += L[4];
-                            plk_DFe += L[5]; plk_POC += L[6]; plk_PON += L[7]; plk_POP += L[8]; plk_PFe += L[9];
-                        } else {
-                            const double* L = a.loss + (long long)r * 6;
-                            plk_DOC += L[0]; plk_DON += L[1]; plk_DOP += L[2];
-                            plk_POC += L[3]; plk_PON += L[4]; plk_POP += L[5];
-                        }
-                    }
-            for (uint32_t r = p; r < e; ++r) {
-                const double* K = a.contrib + (long long)r * 5;
-                if (IRON) { plk_DIC += K[0]; plk_NH4 += K[1]; plk_NO3 += K[2]; plk_PO4 += K[3]; plk_DFe += K[4]; }
-                else { plk_DIC += K[0]; plk_DOC += K[1]; plk_NH4 += K[2]; plk_NO3 += K[3]; plk_PO4 += K[4]; }
-            }
-            p = e;
-        }
-    }
-    // apply_tendency!: tracer += Gc + plk / volume
-#pragma unroll
-    for (int n = 0; n < PI_NTRACERS; ++n) {
-        double pk = n == PI_DIC ? plk_DIC : n == PI_NH4 ? plk_NH4 : n == PI_NO3 ? plk_NO3 : n == PI_PO4 ? plk_PO4
-                  : n == PI_DOC ? plk_DOC : n == PI_DON ? plk_DON : n == PI_DOP ? plk_DOP : n == PI_POC ? plk_POC
-                  : n == PI_PON ? plk_PON : n == PI_POP ? plk_POP
-                  : (IRON && n == PI_DFe) ? plk_DFe : (IRON && n == PI_PFe_bio) ? plk_PFe : 0.0;
-        a.tr_next[n * G + q] = a.tr[n * G + q] + (Gc[n] + pk / volk);
-    }
-}
-
-// fill_halo_tracer! in three passes (x, y, z). Each thread owns one line along the axis and
+// fill_halo_tracer! in three passes (x, y, z), where a periodic axis has fewer cells than halo points
+// (k64_halo otherwise). Each thread owns one line along the axis and
 // reads all its source values before writing, as Julia's broadcast unaliases views.
 template <int AXIS>
 __global__ void k_halo(DGrid g, double* __restrict__ f, int nfields, const uint32_t* err) {

@@ -8,10 +8,11 @@
 //   k_setpos             position of each individual in the cell-sorted list
 //   k_par                Chl per cell, calc_par! down each column, PAR diagnostic
 //   per species:         k_decide → scan(flags) → k_lists → k_daughters → k_physiology
-//   k_sweep_x/y          DST3FL sweeps on tracer_temp
-//   k_sweep_z            z sweep and the advective tendency
-//   k_tracer_tail        diffusion, sinking, forcing, BCs, particle terms, apply_tendency!
-//   k_halo<x,y,z>        fill_halo_tracer! on the new tracers
+//   k64_plk              particle terms of the occupied cells
+//   k64_xy               DST3FL x and y sweeps
+//   k64_ztail            z sweep, diffusion, sinking, forcing, BCs, particle terms, apply_tendency!
+//   k64_halo             fill_halo_tracer! on the new tracers (k_halo<x,y,z> where a periodic axis
+//                        has fewer cells than halo points)
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 
@@ -23,6 +24,7 @@
 #include <vector>
 
 #include "kernels_fp64.cuh"
+#include "kernels_fp64_tracer.cuh"
 #include "kernels_abiotic.cuh"
 #include "kernels_iron.cuh"
 #include "host_common.h"
@@ -73,8 +75,8 @@ struct pi_model {
     SpcDev* d_spc = nullptr;
     double* tr = nullptr;        // 14 × G
     double* tr_next = nullptr;   // 14 × G
-    double* tta = nullptr;       // 14 × G
-    double* ttb = nullptr;       // 14 × G
+    double* ttb = nullptr;       // 14 × G, tracer_temp after the x and y sweeps
+    double* plk = nullptr;       // 14 × G, particle terms of the occupied cells
     double* velbuf[2][3] = {{nullptr}};
     const double* vel0[3] = {nullptr, nullptr, nullptr};
     const double* vel1[3] = {nullptr, nullptr, nullptr};
@@ -373,6 +375,21 @@ pi_status enqueue_abiotic_exchange(pi_model* m, double dT) {
 }
 
 // Enqueues one TimeStep! on the model's stream (no synchronisation).
+// Rows or levels walked by a block of a tracer kernel (a power of two up to `most`): two blocks fit an
+// SM, a walk of n costs about n + over (the rows it reads beside its own, or the set-up), and the
+// length with the shortest waves × walk is taken. On 128×128×1 that is 4 rows (160 blocks), on
+// 128×128×64 16.
+template <class B>
+int walk_length(int most, int over, B blocks) {
+    int best = most;
+    long long cost = -1;
+    for (int n = most; n >= 1; n /= 2) {
+        const long long c = (n + over) * ((blocks(n) + 2 * 148 - 1) / (2 * 148));
+        if (cost < 0 || c < cost) { cost = c; best = n; }
+    }
+    return best;
+}
+
 pi_status enqueue_step(pi_model* m, double dT) {
     // getbc(bc, i, j, t) of a time-dependent flux reads bc[i, j, iteration] (boundary_conditions.jl:44-52)
     for (int n = 0; n < PI_NTRACERS; ++n)
@@ -490,36 +507,39 @@ pi_status enqueue_step(pi_model* m, double dT) {
     }
     if (m->nsa) { pi_status e = enqueue_abiotic_exchange(m, dT); if (e) return e; }
     {
-        { ProfScope ps_(m, "k_sweep_x");
-        (ll ? k_sweep_x<true> : k_sweep_x<false>)<<<dim3(nblk(nblk(g.Nx, 31), SWX_WARPS), g.Ny, g.Nz), 32 * SWX_WARPS, 0, st>>>(g, m->tr, m->tta, m->vel1[0], dT, sb.err);
-        CK(cudaGetLastError(), "k_sweep_x"); }
-        { ProfScope ps_(m, "k_sweep_y");
-        (ll ? k_sweep_y<true> : k_sweep_y<false>)<<<dim3(nblk(g.Nx, 32), nblk(nblk(g.Ny, SWY_L), SWY_TY), g.Nz), dim3(32, SWY_TY), 0, st>>>(g, m->tr, m->tta, m->ttb, m->vel1[1], dT, sb.err);
-        CK(cudaGetLastError(), "k_sweep_y"); }
-        ZFinalArgs za;
-        za.g = g; za.tr = m->tr; za.ttb = m->ttb; za.tr_next = m->tr_next; za.w = m->vel1[2];
-        za.dT = dT; za.b = m->bgc;
-        za.diffuse = (m->bgc.kappa_h != 0.0 || m->bgc.kappa_v != 0.0);
-        za.any_bc = m->any_bc; za.bcs = m->d_bcs; za.iter = m->iteration;
-        za.spc = m->d_spc; za.C = C; za.off = sb.off; za.gid_sorted = sb.gid_sorted; za.evk = sb.evk;
-        za.loss = sb.loss; za.contrib = sb.contrib; za.nsp = m->nsp; za.err = sb.err;
-        za.gadv = m->tta;      // the x-sweep output is no longer needed
-        { ProfScope ps_(m, "k_sweep_z");
-        (ll ? k_sweep_z<true> : k_sweep_z<false>)<<<dim3(nblk(g.Nx, 32), g.Ny, nblk(nblk(g.Nz, SWZ_L), SWZ_TZ)), dim3(32, SWZ_TZ), 0, st>>>(
-            g, m->tr, m->ttb, m->tta, m->vel1[2], dT, sb.err);
-        CK(cudaGetLastError(), "k_sweep_z"); }
-        { ProfScope ps_(m, "k_tracer_tail");
-        (m->iron ? (ll ? k_tracer_tail<true, true> : k_tracer_tail<false, true>)
-                 : (ll ? k_tracer_tail<true, false> : k_tracer_tail<false, false>))<<<dim3(nblk(g.Nx, 128), g.Ny, g.Nz), 128, 0, st>>>(za);
-        CK(cudaGetLastError(), "k_tracer_tail"); }
+        const bool lm = !g.all_water;
+        { ProfScope ps_(m, "k64_plk");
+        PlkArgs pa{ g, C, sb.off, sb.gid_sorted, sb.evk, sb.loss, sb.contrib, m->plk, sb.err };
+        (m->iron ? k64_plk<true> : k64_plk<false>)<<<nblk((long long)g.Nx * g.Ny * g.Nz, 128), 128, 0, st>>>(pa);
+        CK(cudaGetLastError(), "k64_plk"); }
+        { ProfScope ps_(m, "k64_xy");
+        const int rows = walk_length(XY64_MAXROWS, 8, [&](int r) { return (long long)nblk(g.Nx, 31) * nblk(g.Ny, r) * g.Nz; });
+        (ll ? (lm ? k64_xy<true, true> : k64_xy<true, false>) : (lm ? k64_xy<false, true> : k64_xy<false, false>))
+            <<<dim3(nblk(g.Nx, 31), nblk(g.Ny, rows), g.Nz), dim3(32, PI_NTRACERS), xy64_smem(rows), st>>>(
+                g, m->tr, m->ttb, m->vel1[0], m->vel1[1], dT, rows, sb.err);
+        CK(cudaGetLastError(), "k64_xy"); }
+        { ProfScope ps_(m, "k64_ztail");
+        const int levels = walk_length(Z64_MAXLEV, 3, [&](int l) { return (long long)nblk(g.Nx, 32) * g.Ny * nblk(g.Nz, l); });
+        Z64Args za{ g, m->tr, m->ttb, m->tr_next, m->plk, sb.off, m->vel1[2], dT, m->bgc,
+                    m->bgc.kappa_h != 0.0 || m->bgc.kappa_v != 0.0, m->any_bc, m->d_bcs, m->iteration, levels, sb.err };
+        (m->iron ? (ll ? (lm ? k64_ztail<true, true, true> : k64_ztail<true, false, true>)
+                       : (lm ? k64_ztail<false, true, true> : k64_ztail<false, false, true>))
+                 : (ll ? (lm ? k64_ztail<true, true, false> : k64_ztail<true, false, false>)
+                       : (lm ? k64_ztail<false, true, false> : k64_ztail<false, false, false>)))
+            <<<dim3(nblk(g.Nx, 32), g.Ny, nblk(g.Nz, levels)), dim3(32, PI_NTRACERS), z64_smem(levels), st>>>(za);
+        CK(cudaGetLastError(), "k64_ztail"); }
         // tracers are only replaced when the step completed (a capacity error leaves them)
         { ProfScope ps_(m, "k_halo");
-        k_halo<0><<<dim3(nblk(g.Gy, 64), g.Gz, PI_NTRACERS), 64, 0, st>>>(g, m->tr_next, PI_NTRACERS, sb.err);
-        k_halo<1><<<dim3(nblk(g.Gx, 64), g.Gz, PI_NTRACERS), 64, 0, st>>>(g, m->tr_next, PI_NTRACERS, sb.err);
-        k_halo<2><<<dim3(nblk(g.Gx, 64), g.Gy, PI_NTRACERS), 64, 0, st>>>(g, m->tr_next, PI_NTRACERS, sb.err);
+        if ((g.tx == PI_PERIODIC && g.Nx < g.Hx) || (g.ty == PI_PERIODIC && g.Ny < g.Hy)) {
+            k_halo<0><<<dim3(nblk(g.Gy, 64), g.Gz, PI_NTRACERS), 64, 0, st>>>(g, m->tr_next, PI_NTRACERS, sb.err);
+            k_halo<1><<<dim3(nblk(g.Gx, 64), g.Gz, PI_NTRACERS), 64, 0, st>>>(g, m->tr_next, PI_NTRACERS, sb.err);
+            k_halo<2><<<dim3(nblk(g.Gx, 64), g.Gy, PI_NTRACERS), 64, 0, st>>>(g, m->tr_next, PI_NTRACERS, sb.err);
+            k_copy_if_err<<<148 * 4, 256, 0, st>>>(m->tr_next, m->tr, PI_NTRACERS * G, sb.err);
+        } else {
+            const long long nh = G - (long long)g.Nx * g.Ny * g.Nz;
+            k64_halo<<<dim3(std::min<unsigned>(nblk(nh, 256), 148), PI_NTRACERS), 256, 0, st>>>(g, m->tr_next, m->tr, sb.err);
+        }
         CK(cudaGetLastError(), "k_halo"); }
-        k_copy_if_err<<<148 * 4, 256, 0, st>>>(m->tr_next, m->tr, PI_NTRACERS * G, sb.err);
-        CK(cudaGetLastError(), "k_copy_if_err");
         if (m->tr_mask) {
             k_diag_tracers<<<148 * 4, 256, 0, st>>>(m->diag_tr, m->tr_next, m->tr_mask, G, sb.err);
             CK(cudaGetLastError(), "k_diag_tracers");
@@ -685,7 +705,7 @@ pi_status pi_create(const pi_grid* grid, const pi_bgc_params* bgc, const pi_quot
         for (int e = 0; e < 3; ++e) std::copy(a3[e], a3[e] + G, m->met_host.begin() + 5 * G2 + e * G);
     }
     ALB(m->tr, PI_NTRACERS * G); ALB(m->tr_next, PI_NTRACERS * G);
-    ALB(m->tta, PI_NTRACERS * G); ALB(m->ttb, PI_NTRACERS * G);
+    ALB(m->plk, PI_NTRACERS * G); ALB(m->ttb, PI_NTRACERS * G);
     for (int b = 0; b < 2; ++b) for (int c = 0; c < 3; ++c) ALB(m->velbuf[b][c], G);
     ALB(m->stage, 3 * G);
     for (int c = 0; c < 3; ++c) ALB(m->velh[c], G);
@@ -715,7 +735,7 @@ pi_status pi_create(const pi_grid* grid, const pi_bgc_params* bgc, const pi_quot
     if (m->met)
         ok = ok && cudaMemcpyAsync(m->met, m->met_host.data(), m->met_host.size() * sizeof(double), cudaMemcpyHostToDevice, s0) == cudaSuccess;
     ok = ok && cudaMemcpyAsync(m->d_spc, m->h_spc.data(), nspecies * sizeof(SpcDev), cudaMemcpyHostToDevice, s0) == cudaSuccess;
-    for (void* p : { (void*)m->tr, (void*)m->tr_next, (void*)m->tta, (void*)m->ttb })
+    for (void* p : { (void*)m->tr, (void*)m->tr_next, (void*)m->ttb })
         ok = ok && cudaMemsetAsync(p, 0, PI_NTRACERS * G * sizeof(double), s0) == cudaSuccess;
     for (int b = 0; b < 2; ++b) for (int c = 0; c < 3; ++c)
         ok = ok && cudaMemsetAsync(m->velbuf[b][c], 0, G * sizeof(double), s0) == cudaSuccess;
@@ -742,6 +762,12 @@ pi_status pi_create(const pi_grid* grid, const pi_bgc_params* bgc, const pi_quot
         ok = ok && cudaStreamSynchronize(s0) == cudaSuccess;
     }
     if (!ok) { m->err = "pi_create: device initialisation failed"; return bail(PI_ERR_CUDA); }
+    // dynamic shared memory of the tracer kernels above the default limit
+    for (auto* f : { k64_xy<false, false>, k64_xy<false, true>, k64_xy<true, false>, k64_xy<true, true> })
+        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)xy64_smem(XY64_MAXROWS));
+    for (auto* f : { k64_ztail<false, false, false>, k64_ztail<false, true, false>, k64_ztail<true, false, false>, k64_ztail<true, true, false>,
+                     k64_ztail<false, false, true>, k64_ztail<false, true, true>, k64_ztail<true, false, true>, k64_ztail<true, true, true> })
+        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)z64_smem(Z64_MAXLEV));
     // vel₀ = vel₁ = 0 until set (timestepper.jl:24-26)
     for (int c = 0; c < 3; ++c) { m->vel0[c] = m->velbuf[0][c]; m->vel1[c] = m->velbuf[1][c]; }
     m->vel1_buf = 1;
