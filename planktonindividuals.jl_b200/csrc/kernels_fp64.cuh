@@ -265,37 +265,77 @@ __global__ void k_setpos(const uint32_t* __restrict__ off, long long G,
 // PAR: calc_par! down each column (Individuals/utils.jl:55-63, time_step.jl:63-67) with the Chl
 // of acc_chl! (utils.jl:33-36) summed per cell in species-then-slot order, and
 // diags.tracer.PAR .+= par (time_step.jl:167).
+//
+// `lw` warps (a power of two) share 32 columns: each sums the Chl of PAR64_CH levels and forms their
+// attenuation, the first carries the light down through shared memory, all write their levels. One
+// thread per column waited for the gathered Chl cell by cell: 207 µs on 128×128×64 with 6 % of the
+// warps resident.
 // ------------------------------------------------------------------------------------------
+#define PAR64_CH 4
+#define PAR64_WARPS 16
 template <bool LL>
-__global__ void k_par(DGrid g, const SpcDev* __restrict__ spc, long long C,
+__global__ void __launch_bounds__(32 * PAR64_WARPS, 2) k64_par(DGrid g, const SpcDev* __restrict__ spc, long long C,
                       const uint32_t* __restrict__ off, const uint32_t* __restrict__ gid_sorted,
-                      double* __restrict__ PARF, const double* __restrict__ PARF_src,
-                      double* __restrict__ par, double* __restrict__ diag_par, double kc, double kw,
-                      const uint32_t* err) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
-    int j = blockIdx.y + 1;
-    if (i > g.Nx) return;
+                      double* __restrict__ PARF, double* __restrict__ par, double* __restrict__ diag_par, double kc, double kw,
+                      int lw, const uint32_t* err) {
+    __shared__ double sEx[PAR64_WARPS * PAR64_CH][32], sIn[PAR64_WARPS * PAR64_CH][32];
     if (*err & PI_DEVERR_CAPACITY) return;
-    int f = (i - 1) + g.Nx * (j - 1);
-    double parf = PARF_src[f];
-    int ii = i + g.Hx, jj = j + g.Hy;
-    for (int k = 1; k <= g.Nz; ++k) {
-        int kk = k + g.Hz;
-        int c = gidx(g, ii, jj, kk);
-        double chl = 0.0;
-        for (uint32_t p = off[c]; p < off[c + 1]; ++p) {
-            uint32_t gd = gid_sorted[p];
-            int s = (int)(gd / C);
-            chl += spc[s].Chl[gd - (long long)s * C];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, part = wid & (lw - 1), row0 = wid * PAR64_CH;
+    const int nx32 = (g.Nx + 31) / 32, w = blockIdx.x * ((blockDim.x >> 5) / lw) + wid / lw;
+    const int i = (w % nx32) * 32 + lane + 1, j = w / nx32 + 1;
+    const bool col = j <= g.Ny && i <= g.Nx;
+    const int ii = i + g.Hx, jj = j + g.Hy, slab = g.Gx * g.Gy;
+    const int f = (i - 1) + g.Nx * (j - 1);
+    const int q1 = col ? gidx(g, ii, jj, 1 + g.Hz) : 0;
+    double parf = col && part == 0 ? PARF[f] : 0.0;
+    for (int kc0 = 0; kc0 < g.Nz; kc0 += PAR64_CH * lw) {
+        const int k0 = kc0 + part * PAR64_CH;                   // 0-based levels k0 .. k0 + PAR64_CH - 1
+        double ex[PAR64_CH], at[PAR64_CH];
+        if (col) {
+            uint32_t p0[PAR64_CH], p1[PAR64_CH];
+#pragma unroll
+            for (int e = 0; e < PAR64_CH; ++e) {
+                const bool in = k0 + e < g.Nz;
+                const int c = q1 + (k0 + e) * slab;
+                p0[e] = in ? off[c] : 0u; p1[e] = in ? off[c + 1] : 0u;
+            }
+#pragma unroll
+            for (int e = 0; e < PAR64_CH; ++e) {
+                if (k0 + e >= g.Nz) continue;
+                double chl = 0.0;
+                for (uint32_t p = p0[e]; p < p1[e]; ++p) {
+                    const uint32_t gd = gid_sorted[p];
+                    const int s = (int)(gd / (uint32_t)C);
+                    chl += spc[s].Chl[gd - (uint32_t)s * (uint32_t)C];
+                }
+                const int kk = k0 + e + 1 + g.Hz;
+                at[e] = (chl / vol<LL>(g, ii, jj, kk) * kc + kw) * dzF1(g, kk);
+                ex[e] = pi_exp(-at[e]);
+                sEx[row0 + e][lane] = ex[e];
+            }
         }
-        double atten = (chl / vol<LL>(g, ii, jj, kk) * kc + kw) * dzF1(g, kk);
-        double e = pi_exp(-atten);
-        double pv = parf * (1.0 - e) / atten;
-        par[c] = pv;
-        parf = parf * e;
-        diag_par[c] = diag_par[c] + pv;
+        __syncthreads();
+        if (part == 0 && col) {
+            const int n = min(PAR64_CH * lw, g.Nz - kc0);
+            for (int e = 0; e < n; ++e) {
+                sIn[row0 + e][lane] = parf;
+                parf = parf * sEx[row0 + e][lane];
+            }
+        }
+        __syncthreads();
+        if (col) {
+#pragma unroll
+            for (int e = 0; e < PAR64_CH; ++e) {
+                if (k0 + e >= g.Nz) continue;
+                const int c = q1 + (k0 + e) * slab;
+                const double pv = sIn[row0 + e][lane] * (1.0 - ex[e]) / at[e];
+                par[c] = pv;
+                diag_par[c] = diag_par[c] + pv;
+            }
+        }
+        __syncthreads();
     }
-    PARF[f] = parf;
+    if (col && part == 0) PARF[f] = parf;
 }
 
 // ------------------------------------------------------------------------------------------
@@ -500,24 +540,26 @@ __device__ __forceinline__ double shape_inc(double x, double xmax, double k, int
     double reg = pi_pow_int(fx, pw) / (k + pi_pow_int(fx, pw));
     return 1.0 - reg;
 }
-__device__ __forceinline__ double tempFunc_PS(double T, const pi_quota_params& p) {
+// tempFunc's normaliser exp(-Ea / (R (Topt + 273.15))), a constant of the species formed on the host
+// (pi_exp has the same bits there) and passed as OGT_rate
+template <class P>
+inline double ogt_rate(const P& p) { return pi_exp(-p.Ea / (F_RGAS * (p.Topt + F_T0))); }
+__device__ __forceinline__ double tempFunc_PS(double T, const pi_quota_params& p, double OGT_rate) {
     double x = T - p.Topt, xmax = p.Tmax - p.Topt;
     double regT = shape_dec(x, xmax, F_4em2, 4);
     double k = pi_exp(-p.Ea / (F_RGAS * (T + F_T0))) * regT;
     k = jl_max(0.0, k);
-    double OGT_rate = pi_exp(-p.Ea / (F_RGAS * (p.Topt + F_T0)));
     return jl_min(1.0, k / OGT_rate);
 }
-__device__ __forceinline__ double tempFunc(double T, const pi_quota_params& p) {
+__device__ __forceinline__ double tempFunc(double T, const pi_quota_params& p, double OGT_rate) {
     double k = pi_exp(-p.Ea / (F_RGAS * (T + F_T0)));
     k = jl_max(0.0, k);
-    double OGT_rate = pi_exp(-p.Ea / (F_RGAS * (p.Topt + F_T0)));
     return jl_min(1.0, k / OGT_rate);
 }
 
 struct TracerPtrs { const double* c[PI_NTRACERS]; };
 
-__global__ void k_physiology(DGrid g, SpcDev P, pi_quota_params p, long long C, int s,
+__global__ void k_physiology(DGrid g, SpcDev P, pi_quota_params p, double ogt, long long C, int s,
                              double dT, double t, uint64_t seed, uint32_t iter, int shared_graz,
                              const double* __restrict__ NH4f, const double* __restrict__ NO3f,
                              const double* __restrict__ PO4f, const double* __restrict__ DOCf,
@@ -559,9 +601,10 @@ __global__ void k_physiology(DGrid g, SpcDev P, pi_quota_params p, long long C, 
     }
     double Bm = P.Bm[slot], Cq = P.Cq[slot], Nq = P.Nq[slot], Pq = P.Pq[slot], Chl = P.Chl[slot];
     double age = P.age[slot];
+    const double tf = tempFunc(T, p, ogt);
     // calc_inorganic_uptake_kernel! (growth_kernels.jl:48-56)
     double aI = parv * p.alpha * p.Phi;
-    double PCm = p.PCmax * tempFunc_PS(T, p);
+    double PCm = p.PCmax * tempFunc_PS(T, p, ogt);
     double PS = PCm * (1.0 - pi_exp(-aI / jl_max(F_1em30, PCm) * Chl / jl_max(F_1em30, Bm))) * Bm;
     PS = jl_mulb(PS, ac);
     double VNH4, VNO3, VPO4;
@@ -570,9 +613,9 @@ __global__ void k_physiology(DGrid g, SpcDev P, pi_quota_params p, long long C, 
         double Qp = (Pq + Bm * p.R_PC) / jl_max(F_1em30, Bm + Cq);
         double regQN = shape_dec(Qn, p.Nqmax, F_1em4, 4);
         double regQP = shape_dec(Qp, p.Pqmax, F_1em4, 4);
-        double a = jl_mulb(p.VNH4max * regQN * NH4 / jl_max(F_1em30, NH4 + p.KsatNH4) * tempFunc(T, p) * Bm, ac);
-        double b = jl_mulb(p.VNO3max * regQN * NO3 / jl_max(F_1em30, NO3 + p.KsatNO3) * tempFunc(T, p) * Bm, ac);
-        double cc = jl_mulb(p.VPO4max * regQP * PO4 / jl_max(F_1em30, PO4 + p.KsatPO4) * tempFunc(T, p) * Bm, ac);
+        double a = jl_mulb(p.VNH4max * regQN * NH4 / jl_max(F_1em30, NH4 + p.KsatNH4) * tf * Bm, ac);
+        double b = jl_mulb(p.VNO3max * regQN * NO3 / jl_max(F_1em30, NO3 + p.KsatNO3) * tf * Bm, ac);
+        double cc = jl_mulb(p.VPO4max * regQP * PO4 / jl_max(F_1em30, PO4 + p.KsatPO4) * tf * Bm, ac);
         VNH4 = jl_min(a, NH4 / dT / jl_max(1.0, pop));
         VNO3 = jl_min(b, NO3 / dT / jl_max(1.0, pop));
         VPO4 = jl_min(cc, PO4 / dT / jl_max(1.0, pop));
@@ -586,7 +629,7 @@ __global__ void k_physiology(DGrid g, SpcDev P, pi_quota_params p, long long C, 
     {
         double Qc = Cq / jl_max(F_1em30, Bm + Cq);
         double regQ = shape_dec(Qc, p.Cqmax, F_1em4, 4);
-        double VN = p.VDOCmax * regQ * DOC / jl_max(F_1em30, DOC + p.KsatDOC) * tempFunc(T, p) * Bm;
+        double VN = p.VDOCmax * regQ * DOC / jl_max(F_1em30, DOC + p.KsatDOC) * tf * Bm;
         VDOC = jl_mulb(jl_min(VN, DOC / dT / jl_max(1.0, pop)), ac);
         VDOC = jl_mulb(VDOC, jl_isless(F_1em2, PS / (VDOC + PS)));
     }
@@ -595,7 +638,7 @@ __global__ void k_physiology(DGrid g, SpcDev P, pi_quota_params p, long long C, 
                                   jl_max(F_1em30, parv * p.alpha * p.Phi * Chl / Bm),
                                   jl_isless(F_1em1, parv)), ac);
     // calc_respir_kernel! (:105-108)
-    double resp = jl_mulb(p.respir * Bm * tempFunc(T, p), ac);
+    double resp = jl_mulb(p.respir * Bm * tf, ac);
     // update_quotas_2_kernel! (:117-124)
     Cq = Cq + (VDOC - resp) * dT;
     Bm = Bm - jl_max(0.0, (0.0 - Cq));
@@ -655,18 +698,16 @@ __global__ void k_physiology(DGrid g, SpcDev P, pi_quota_params p, long long C, 
 // CarbonMode physiology — CarbonMode/plankton_growth.jl:2-29, growth_kernels.jl:2-120,
 // division_death_probability.jl:7-107, calc_consume! (consume_loss.jl:2-5)
 // ------------------------------------------------------------------------------------------
-__device__ __forceinline__ double c_tempFunc_PS(double T, const pi_carbon_params& p) {
+__device__ __forceinline__ double c_tempFunc_PS(double T, const pi_carbon_params& p, double OGT_rate) {
     double x = T - p.Topt, xmax = p.Tmax - p.Topt;
     double regT = shape_dec(x, xmax, F_1em1, 4);
     double k = pi_exp(-p.Ea / (F_RGAS * (T + F_T0))) * regT;
     k = jl_max(0.0, k);
-    double OGT_rate = pi_exp(-p.Ea / (F_RGAS * (p.Topt + F_T0)));
     return jl_min(1.0, k / OGT_rate);
 }
-__device__ __forceinline__ double c_tempFunc(double T, const pi_carbon_params& p) {
+__device__ __forceinline__ double c_tempFunc(double T, const pi_carbon_params& p, double OGT_rate) {
     double k = pi_exp(-p.Ea / (F_RGAS * (T + F_T0)));
     k = jl_max(0.0, k);
-    double OGT_rate = pi_exp(-p.Ea / (F_RGAS * (p.Topt + F_T0)));
     return jl_min(1.0, k / OGT_rate);
 }
 // gamma_alloc (growth_kernels.jl:22-26)
@@ -675,7 +716,7 @@ __device__ __forceinline__ double c_gamma(double Bm, double Bd, const pi_carbon_
     return jl_mulb(jl_min(1.0, gm), p.thermal == 1.0);
 }
 
-__global__ void k_physiology_carbon(DGrid g, SpcDev P, pi_carbon_params p, long long C, int s,
+__global__ void k_physiology_carbon(DGrid g, SpcDev P, pi_carbon_params p, double ogt, long long C, int s,
                                     double dT, double t, uint64_t seed, uint32_t iter, int shared_graz,
                                     const double* __restrict__ par, const double* __restrict__ temp,
                                     const uint32_t* __restrict__ off, const uint32_t* __restrict__ gid_sorted,
@@ -722,9 +763,10 @@ __global__ void k_physiology_carbon(DGrid g, SpcDev P, pi_carbon_params p, long 
         }
     }
     double Bm = P.Bm[slot], Bd = P.Bd[slot], Chl = P.Chl[slot], age = P.age[slot];
+    const double tf = c_tempFunc(T, p, ogt);
     // calc_PS! (calc_photosynthesis, growth_kernels.jl:29-36)
     double aI = parv * p.alpha * p.Phi;
-    double PCm = p.PCmax * (c_tempFunc(T, p) * p.thermal + c_tempFunc_PS(T, p) * (1.0 - p.thermal));
+    double PCm = p.PCmax * (tf * p.thermal + c_tempFunc_PS(T, p, ogt) * (1.0 - p.thermal));
     double light = 1.0 - pi_exp(-aI / jl_max(F_1em30, PCm) * Chl / jl_max(F_1em30, Bm));
     double PS = jl_mulb(PCm * jl_max(0.0, Bm - Bd) * (light * (1.0 - p.is_bact) + p.is_bact), ac);
     // calc_BS!, calc_repair! (:55-64), calc_thermal_damage! (:69-75), calc_respir! (:82-85)
@@ -733,7 +775,7 @@ __global__ void k_physiology_carbon(DGrid g, SpcDev P, pi_carbon_params p, long 
     double TD = jl_mulb(jl_mulb(jl_mulb((T - p.Topt) * p.f_T2B * (Bm - Bd), jl_isless(p.Topt, T)),
                                 jl_isless(Bd, Bm)), p.thermal == 1.0);
     TD = jl_max(0.0, jl_min(TD, (Bm - Bd) / dT));
-    double RS = jl_mulb(p.respir * Bm * c_tempFunc(T, p), ac);
+    double RS = jl_mulb(p.respir * Bm * tf, ac);
     // update_quotas! (:92-97), update_cellsize! (:104-108)
     Bm += (BS - RS) * dT;
     Bd += (TD - RP) * dT;
@@ -776,24 +818,22 @@ __global__ void k_physiology_carbon(DGrid g, SpcDev P, pi_carbon_params p, long 
 // MacroMolecularMode physiology — MacroMolecularMode/plankton_growth.jl:2-28, growth_kernels.jl:1-200,
 // division_death_probability.jl:37-40, 49-52, 84-107, calc_consume! (consume_loss.jl:2-9)
 // ------------------------------------------------------------------------------------------
-__device__ __forceinline__ double m_tempFunc_PS(double T, const pi_macro_params& p) {
+__device__ __forceinline__ double m_tempFunc_PS(double T, const pi_macro_params& p, double OGT_rate) {
     double x = T - p.Topt, xmax = p.Tmax - p.Topt;
     double regT = shape_dec(x, xmax, F_4em2, 4);
     double k = pi_exp(-p.Ea / (F_RGAS * (T + F_T0))) * regT;
     k = jl_max(0.0, k);
-    double OGT_rate = pi_exp(-p.Ea / (F_RGAS * (p.Topt + F_T0)));
     return jl_min(1.0, k / OGT_rate);
 }
-__device__ __forceinline__ double m_tempFunc(double T, const pi_macro_params& p) {
+__device__ __forceinline__ double m_tempFunc(double T, const pi_macro_params& p, double OGT_rate) {
     double k = pi_exp(-p.Ea / (F_RGAS * (T + F_T0)));
     k = jl_max(0.0, k);
-    double OGT_rate = pi_exp(-p.Ea / (F_RGAS * (p.Topt + F_T0)));
     return jl_min(1.0, k / OGT_rate);
 }
 // Every slot is updated: the synthesis and exudation terms carry no ac, so the state of an
 // inactive slot keeps changing as in the reference, from zero light, temperature and nutrients
 // unless it was active when they were gathered (an individual grazed or dead in this step).
-__global__ void k_physiology_macro(DGrid g, SpcDev P, pi_macro_params p, long long C, int s,
+__global__ void k_physiology_macro(DGrid g, SpcDev P, pi_macro_params p, double ogt, long long C, int s,
                                    double dT, uint64_t seed, uint32_t iter, int shared_graz,
                                    const double* __restrict__ NH4f, const double* __restrict__ NO3f,
                                    const double* __restrict__ PO4f, const double* __restrict__ DOCf,
@@ -824,16 +864,17 @@ __global__ void k_physiology_macro(DGrid g, SpcDev P, pi_macro_params p, long lo
     }
     double PRO = P.PRO[slot], DNA = P.DNA[slot], RNA = P.RNA[slot], CH = P.CH[slot];
     double NST = P.NST[slot], PST = P.PST[slot], Chl = P.Chl[slot], age = P.age[slot];
+    const double tf = m_tempFunc(T, p, ogt);
     // calc_inorganic_uptake_kernel! (growth_kernels.jl:45-54): calc_PS (:20-25), calc_NP_uptake (:28-42)
     double aI = parv * p.alpha * p.Phi;
-    double PCm = p.PCmax * m_tempFunc_PS(T, p);
+    double PCm = p.PCmax * m_tempFunc_PS(T, p, ogt);
     double PS = jl_mulb(PCm * (1.0 - pi_exp(-aI / jl_max(F_1em30, PCm) * Chl / jl_max(F_1em30, PRO))) * PRO, ac);
     double R_NST = NST / jl_max(F_1em30, m_totN(PRO, DNA, RNA, NST, Chl, p));
     double R_PST = PST / jl_max(F_1em30, m_totP(DNA, RNA, PST, p));
     double regQN = shape_dec(R_NST, p.NSTmax, F_1em4, 4), regQP = shape_dec(R_PST, p.PSTmax, F_1em4, 4);
-    double VNH4 = jl_mulb(p.VNH4max * regQN * NH4 / jl_max(F_1em30, NH4 + p.KsatNH4) * m_tempFunc(T, p) * PRO, ac);
-    double VNO3 = jl_mulb(p.VNO3max * regQN * NO3 / jl_max(F_1em30, NO3 + p.KsatNO3) * m_tempFunc(T, p) * PRO, ac);
-    double VPO4 = jl_mulb(p.VPO4max * regQP * PO4 / jl_max(F_1em30, PO4 + p.KsatPO4) * m_tempFunc(T, p) * PRO, ac);
+    double VNH4 = jl_mulb(p.VNH4max * regQN * NH4 / jl_max(F_1em30, NH4 + p.KsatNH4) * tf * PRO, ac);
+    double VNO3 = jl_mulb(p.VNO3max * regQN * NO3 / jl_max(F_1em30, NO3 + p.KsatNO3) * tf * PRO, ac);
+    double VPO4 = jl_mulb(p.VPO4max * regQP * PO4 / jl_max(F_1em30, PO4 + p.KsatPO4) * tf * PRO, ac);
     VNH4 = jl_min(VNH4, NH4 / dT / jl_max(1.0, pop));
     VNO3 = jl_min(VNO3, NO3 / dT / jl_max(1.0, pop));
     VPO4 = jl_min(VPO4, PO4 / dT / jl_max(1.0, pop));
@@ -842,20 +883,19 @@ __global__ void k_physiology_macro(DGrid g, SpcDev P, pi_macro_params p, long lo
     // calc_organic_uptake_kernel! (:82-90), calc_DOC_uptake (:73-80)
     double R_CH = CH / jl_max(F_1em30, m_totC(PRO, DNA, RNA, CH, Chl));
     double regQ = shape_dec(R_CH, p.CHmax, F_1em4, 4);
-    double VN = p.VDOCmax * regQ * DOC / jl_max(F_1em30, DOC + p.KsatDOC) * m_tempFunc(T, p) * PRO;
+    double VN = p.VDOCmax * regQ * DOC / jl_max(F_1em30, DOC + p.KsatDOC) * tf * PRO;
     double VDOC = jl_mulb(jl_min(VN, DOC / dT / jl_max(1.0, pop)), ac);
     VDOC = jl_mulb(VDOC, jl_isless(F_5em2, PS / (VDOC + PS)));
     // calc_ρChl_kernel! (:98-103), calc_respir_kernel! (:111-114)
     double rChl = jl_mulb(jl_mulb(PS / jl_max(F_1em30, PRO) / jl_max(F_1em30, parv * p.alpha * p.Phi * Chl / jl_max(F_1em30, PRO)),
                                   jl_isless(F_1em1, parv)), ac);
-    double resp = jl_mulb(p.respir * PRO * m_tempFunc(T, p), ac);
+    double resp = jl_mulb(p.respir * PRO * tf, ac);
     // update_quotas_2_kernel! (:124-130)
     CH = CH + (VDOC - resp) * dT;
     PRO = PRO - jl_max(0.0, 0.0 - CH);
     NST = NST + jl_max(0.0, 0.0 - CH) * p.R_NC_PRO;
     CH = CH + jl_max(0.0, 0.0 - CH);
     // calc_BS_kernel! (:136-152)
-    double tf = m_tempFunc(T, p);
     double limit_PRO = jl_min(CH / (CH + p.k_sat_pro * p.Nsuper), NST / (NST + p.k_sat_pro * p.Nsuper * p.R_NC_PRO));
     double limit_DNA = jl_min(jl_min(CH / (CH + p.k_sat_dna * p.Nsuper), NST / (NST + p.k_sat_dna * p.Nsuper * p.R_NC_DNA)),
                               PST / (PST + p.k_sat_dna * p.Nsuper * p.R_PC_DNA));

@@ -7,22 +7,22 @@
 
 namespace pib {
 
-__device__ __forceinline__ double i_tempFunc(double T, const pi_iron_params& p) {      // growth_kernels.jl:12-17
+__device__ __forceinline__ double i_tempFunc(double T, const pi_iron_params& p, double OGT_rate) {      // growth_kernels.jl:12-17
     double k = jl_max(0.0, pi_exp(-p.Ea / (F_RGAS * (T + F_T0))));
-    return jl_min(1.0, k / pi_exp(-p.Ea / (F_RGAS * (p.Topt + F_T0))));
+    return jl_min(1.0, k / OGT_rate);
 }
-__device__ __forceinline__ double i_tempFunc_CF(double T, const pi_iron_params& p) {   // :2-9
+__device__ __forceinline__ double i_tempFunc_CF(double T, const pi_iron_params& p, double OGT_rate) {   // :2-9
     double x = T - p.Topt, xmax = p.Tmax - p.Topt;
     double k = pi_exp(-p.Ea / (F_RGAS * (T + F_T0))) * shape_dec(x, xmax, F_4em2, 4);
     k = jl_max(0.0, k);
-    return jl_min(1.0, k / pi_exp(-p.Ea / (F_RGAS * (p.Topt + F_T0))));
+    return jl_min(1.0, k / OGT_rate);
 }
 
 // Every slot is updated: the light reaction, the iron allocation and the dark clock carry no ac,
 // so the state of an inactive slot keeps changing as in the reference, from zero light,
 // temperature and nutrients unless it was active when they were gathered (find_NPT!, with the
 // change of PAR since the previous step).
-__global__ void k_physiology_iron(DGrid g, SpcDev P, pi_iron_params p, long long C, int s,
+__global__ void k_physiology_iron(DGrid g, SpcDev P, pi_iron_params p, double ogt, long long C, int s,
                                   double dT, double t, uint64_t seed, uint32_t iter, int shared_graz,
                                   const double* __restrict__ NH4f, const double* __restrict__ NO3f,
                                   const double* __restrict__ PO4f, const double* __restrict__ DFef,
@@ -51,23 +51,24 @@ __global__ void k_physiology_iron(DGrid g, SpcDev P, pi_iron_params p, long long
             pop = (double)n;
         }
     }
+    const double tf = i_tempFunc(T, p, ogt);
     const double nfx = p.is_croc + p.is_tric;
     const double Bm = P.Bm[slot], Sz = P.Sz[slot], Chl = P.Chl[slot], tdark = P.tdark[slot];
     double CH = P.CH[slot], qNH4 = P.qNH4[slot], qNO3 = P.qNO3[slot], qP = P.qP[slot], qFe = P.qFe[slot];
     const double qFePS = P.qFePS[slot], qFeNR = P.qFeNR[slot], qFeNF = P.qFeNF[slot];
     // calc_trs_uptake_kernel! (growth_kernels.jl:56-66) with calc_NH4/NO3/P/Fe_uptake (:20-53)
     double reg = shape_dec(qNH4 / jl_max(F_1em30, Bm + CH), p.qNH4max, F_1em4, 2);
-    double VNH4 = jl_mulb(p.VNH4max * reg * NH4 / jl_max(F_1em30, NH4 + p.KsatNH4) * i_tempFunc(T, p) * Bm, ac);
+    double VNH4 = jl_mulb(p.VNH4max * reg * NH4 / jl_max(F_1em30, NH4 + p.KsatNH4) * tf * Bm, ac);
     VNH4 = jl_min(VNH4, NH4 / dT / jl_max(1.0, pop)) * p.is_nr;
     reg = shape_dec(qNO3 / jl_max(F_1em30, Bm + CH), p.qNO3max, F_1em4, 2);
-    double VNO3 = jl_mulb(p.VNO3max * reg * NO3 / jl_max(F_1em30, NO3 + p.KsatNO3) * i_tempFunc(T, p) * Bm, ac);
+    double VNO3 = jl_mulb(p.VNO3max * reg * NO3 / jl_max(F_1em30, NO3 + p.KsatNO3) * tf * Bm, ac);
     VNO3 = jl_min(VNO3, NO3 / dT / jl_max(1.0, pop)) * p.is_nr;
     reg = shape_dec((qP + Bm * p.R_PC) / jl_max(F_1em30, Bm + CH), p.qPmax, F_1em4, 2);
-    double VPO4 = jl_mulb(p.VPO4max * reg * PO4 / jl_max(F_1em30, PO4 + p.KsatPO4) * i_tempFunc(T, p) * Bm, ac);
+    double VPO4 = jl_mulb(p.VPO4max * reg * PO4 / jl_max(F_1em30, PO4 + p.KsatPO4) * tf * Bm, ac);
     VPO4 = jl_min(VPO4, PO4 / dT / jl_max(1.0, pop));
     reg = shape_dec((qFe + qFePS + qFeNF + qFeNR) / jl_max(F_1em30, Bm + CH), p.qFemax, F_1em4, 2);
     const double SA = p.SA * pi_pow(Sz, (double)(2.0f / 3.0f));
-    double VFe = jl_mulb(p.KSAFe * SA * DFe * reg * p.Nsuper * i_tempFunc(T, p), ac);
+    double VFe = jl_mulb(p.KSAFe * SA * DFe * reg * p.Nsuper * tf, ac);
     VFe = jl_min(VFe, DFe / dT / jl_max(1.0, pop));
     // update_state_1_kernel! (:73-79)
     qP += VPO4 * dT; qNO3 += VNO3 * dT; qNH4 += VNH4 * dT; qFe += VFe * dT;
@@ -76,22 +77,22 @@ __global__ void k_physiology_iron(DGrid g, SpcDev P, pi_iron_params p, long long
     const double Qfe_ps = qFePS / jl_max(F_1em30, Bm + CH);
     const double PS = p.PCmax * (1.0 - pi_exp(-aI)) * Bm * (Qfe_ps / jl_max(F_1em30, Qfe_ps + p.KfePS));
     // calc_respir (:106-111)
-    double RS = jl_mulb(CH * p.k_rs * i_tempFunc(T, p), ac);
+    double RS = jl_mulb(CH * p.k_rs * tf, ac);
     RS = jl_min(RS, CH / dT);
     double ERS = jl_mulb(RS * p.e_rs, ac);
     // calc_CF (:125-131)
     reg = shape_dec(CH / jl_max(F_1em30, Bm + CH), p.CHmax, F_1em4, 2);
-    double CF = jl_mulb(p.k_cf * reg * i_tempFunc_CF(T, p) * Bm, ac);
+    double CF = jl_mulb(p.k_cf * reg * i_tempFunc_CF(T, p, ogt) * Bm, ac);
     double ECF = jl_mulb(CF * p.e_cf, ac);
     // calc_NR (:145-155) and calc_NF (:167-176), both regulated by the same NH4 quota
     reg = shape_dec(qNH4 / jl_max(F_1em30, Bm + CH), p.qNH4max, F_1em4, 2);
     const double Qfe_NR = qFeNR / jl_max(F_1em30, Bm + CH);
-    double NR = jl_mulb(p.k_nr * reg * qNO3 * (Qfe_NR / jl_max(F_1em30, Qfe_NR + p.KfeNR)) * i_tempFunc(T, p), ac);
+    double NR = jl_mulb(p.k_nr * reg * qNO3 * (Qfe_NR / jl_max(F_1em30, Qfe_NR + p.KfeNR)) * tf, ac);
     NR = jl_min(NR, qNO3 / dT);
     double ENR = jl_mulb(NR * p.e_nr, ac);
     NR = NR * p.is_nr; ENR = ENR * p.is_nr;
     const double Qfe_NF = qFeNF / jl_max(F_1em30, Bm + CH);
-    double NF = jl_mulb(p.k_nf * reg * (Qfe_NF / jl_max(F_1em30, Qfe_NF + p.KfeNF)) * i_tempFunc(T, p) * Bm, ac);
+    double NF = jl_mulb(p.k_nf * reg * (Qfe_NF / jl_max(F_1em30, Qfe_NF + p.KfeNF)) * tf * Bm, ac);
     double ENF = jl_mulb(NF * p.e_nf, ac);
     NF = NF * nfx; ENF = ENF * nfx;
     // energy_alloc (:190-197), energy_allocation_kernel! (:198-206)

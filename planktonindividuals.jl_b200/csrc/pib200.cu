@@ -6,7 +6,7 @@
 //   scan(cnt) → off      cell offsets of the binned individuals
 //   radix sort           (cell, species·C + slot) order = the order of a sequential reference run
 //   k_setpos             position of each individual in the cell-sorted list
-//   k_par                Chl per cell, calc_par! down each column, PAR diagnostic
+//   k64_par              Chl per cell, calc_par! down each column, PAR diagnostic
 //   per species:         k_decide → scan(flags) → k_lists → k_daughters → k_physiology
 //   k64_plk              particle terms of the occupied cells
 //   k64_xy               DST3FL x and y sweeps
@@ -442,11 +442,13 @@ pi_status enqueue_step(pi_model* m, double dT) {
     k_setpos<<<nblk(NC, BS), BS, 0, st>>>(sb.off, G, sb.gid_sorted, sb.pos, NC, sb.err);
     CK(cudaGetLastError(), "k_setpos"); }
     {
-        dim3 grid(nblk(g.Nx, 128), g.Ny);
-        ProfScope ps_(m, "k_par");
-        (ll ? k_par<true> : k_par<false>)<<<grid, 128, 0, st>>>(g, m->d_spc, C, sb.off, sb.gid_sorted, m->PARF, m->PARF, m->par,
-                                    m->diag_par, m->bgc.kc, m->bgc.kw, sb.err);
-        CK(cudaGetLastError(), "k_par");
+        // as many warps per 32 columns as the levels give work to, in blocks of at least four
+        const int lw = g.Nz <= PAR64_CH ? 1 : g.Nz <= 2 * PAR64_CH ? 2 : g.Nz <= 4 * PAR64_CH ? 4 : g.Nz <= 8 * PAR64_CH ? 8 : 16;
+        const int wpb = std::max(lw, 4);
+        ProfScope ps_(m, "k64_par");
+        (ll ? k64_par<true> : k64_par<false>)<<<nblk((long long)nblk(g.Nx, 32) * g.Ny * lw, wpb), 32 * wpb, 0, st>>>(
+            g, m->d_spc, C, sb.off, sb.gid_sorted, m->PARF, m->par, m->diag_par, m->bgc.kc, m->bgc.kw, lw, sb.err);
+        CK(cudaGetLastError(), "k64_par");
     }
     const int shared = m->bgc.shared_graz == 1.0;
     for (int s = 0; s < m->nsp; ++s) {
@@ -469,26 +471,26 @@ pi_status enqueue_step(pi_model* m, double dT) {
         CK(cudaGetLastError(), "k_daughters"); }
         const double* trp = m->tr;
         if (m->iron) { ProfScope ps_(m, "k_physiology");
-        k_physiology_iron<<<nblk(C, BS), BS, 0, st>>>(g, m->h_spc[s], m->ipp[s], C, s, dT, m->t, m->seed, iter, shared,
+        k_physiology_iron<<<nblk(C, BS), BS, 0, st>>>(g, m->h_spc[s], m->ipp[s], ogt_rate(m->ipp[s]), C, s, dT, m->t, m->seed, iter, shared,
                                                       trp + PI_NH4 * G, trp + PI_NO3 * G, trp + PI_PO4 * G,
                                                       trp + PI_DFe * G, m->par, m->par0, m->temp, sb.off, sb.gid_sorted,
                                                       sb.pos, sb.contrib, dsp + 0 * G,
                                                       m->proc_mask ? m->procv : nullptr, sb.err);
         CK(cudaGetLastError(), "k_physiology_iron"); } else
         if (m->macro) { ProfScope ps_(m, "k_physiology");
-        k_physiology_macro<<<nblk(C, BS), BS, 0, st>>>(g, m->h_spc[s], m->mp[s], C, s, dT, m->seed, iter, shared,
+        k_physiology_macro<<<nblk(C, BS), BS, 0, st>>>(g, m->h_spc[s], m->mp[s], ogt_rate(m->mp[s]), C, s, dT, m->seed, iter, shared,
                                                        trp + PI_NH4 * G, trp + PI_NO3 * G, trp + PI_PO4 * G,
                                                        trp + PI_DOC * G, m->par, m->temp, sb.off, sb.gid_sorted,
                                                        sb.pos, sb.contrib, dsp + 0 * G,
                                                        m->proc_mask ? m->procv : nullptr, sb.err);
         CK(cudaGetLastError(), "k_physiology_macro"); } else
         if (m->carbon) { ProfScope ps_(m, "k_physiology");
-        k_physiology_carbon<<<nblk(C, BS), BS, 0, st>>>(g, m->h_spc[s], m->cp[s], C, s, dT, m->t, m->seed, iter,
+        k_physiology_carbon<<<nblk(C, BS), BS, 0, st>>>(g, m->h_spc[s], m->cp[s], ogt_rate(m->cp[s]), C, s, dT, m->t, m->seed, iter,
                                                         shared, m->par, m->temp, sb.off, sb.gid_sorted, sb.pos,
                                                         sb.contrib, dsp + 0 * G, m->proc_mask ? m->procv : nullptr, sb.err);
         CK(cudaGetLastError(), "k_physiology_carbon"); } else
         { ProfScope ps_(m, "k_physiology");
-        k_physiology<<<nblk(C, BS), BS, 0, st>>>(g, m->h_spc[s], m->sp[s], C, s, dT, m->t, m->seed, iter,
+        k_physiology<<<nblk(C, BS), BS, 0, st>>>(g, m->h_spc[s], m->sp[s], ogt_rate(m->sp[s]), C, s, dT, m->t, m->seed, iter,
                                                  shared, trp + PI_NH4 * G, trp + PI_NO3 * G,
                                                  trp + PI_PO4 * G, trp + PI_DOC * G, m->par, m->temp,
                                                  sb.off, sb.gid_sorted, sb.pos, sb.contrib,
