@@ -69,25 +69,35 @@ __device__ __forceinline__ double bc_pos(double x, double xr, int topo) {
     return x;
 }
 
-// Trilinear interpolation in grid-index units (u_itpl/v_itpl/w_itpl). HALF = 1 samples
-// vel½ = (vel₀ + vel₁) * 0.5 corner by corner, which is the array time_step.jl:17-19 builds.
-template <int COMP, int HALF, bool LL>
-__device__ __forceinline__ double itpl(const DGrid& g, const double* __restrict__ f0,
-                                       const double* __restrict__ f1, double x, double y,
-                                       double z, int ac, uint32_t* err) {
-    double fx = jl_mulb(COMP == 0 ? x + 1.0 : x + 0.5, ac);
-    double fy = jl_mulb(COMP == 1 ? y + 1.0 : y + 0.5, ac);
-    double fz = jl_mulb(COMP == 2 ? z + 1.0 : z + 0.5, ac);
-    double xd = jl_mod1(fx), yd = jl_mod1(fy), zd = jl_mod1(fz);
-    int i = clamp_idx(jl_trunc(fx) + g.Hx, 1, g.Gx - 1, err);
-    int j = clamp_idx(jl_trunc(fy) + g.Hy, 1, g.Gy - 1, err);
-    int k = clamp_idx(jl_trunc(fz) + g.Hz, 1, g.Gz - 1, err);
-    int q000 = gidx(g, i, j, k);
-    int sx = 1, sy = g.Gx, sz = g.Gx * g.Gy;
-    auto F = [&](int q) -> double { return HALF ? (f0[q] + f1[q]) * 0.5 : f0[q]; };
-    double c000 = F(q000), c001 = F(q000 + sz), c010 = F(q000 + sy), c011 = F(q000 + sy + sz);
-    double c100 = F(q000 + sx), c101 = F(q000 + sx + sz), c110 = F(q000 + sx + sy);
-    double c111 = F(q000 + sx + sy + sz);
+// Index (base corner) and offset of one axis of the interpolation from f = x + 1 or x + ½: trunc(f) + H
+// clamped into 1 .. G - 1, and mod(f, 1). Out of line: NaN and positions outside the grid.
+__device__ __noinline__ double index_axis_any(double f, int H, int G, int* idx, uint32_t* err) {
+    *idx = clamp_idx(jl_trunc(f) + H, 1, G - 1, err);
+    return jl_mod1(f);
+}
+__device__ __forceinline__ double index_axis(double f, int H, int G, int& idx, uint32_t* err) {
+    if (f >= 0.0 && f < (double)(G - H)) {            // 0 <= trunc(f) <= G - 1 - H: nothing to clamp
+        const double t = trunc(f);
+        idx = (int)t + H;
+        return f - t;
+    }
+    int i;
+    const double r = index_axis_any(f, H, G, &i, err);
+    idx = i;
+    return r;
+}
+
+// Trilinear interpolation in grid-index units (u_itpl/v_itpl/w_itpl).
+template <int COMP, bool LL>
+__device__ __forceinline__ double itpl(const DGrid& g, const double* __restrict__ f0, double x, double y, double z, uint32_t* err) {
+    int i, j, k;
+    const double xd = index_axis(COMP == 0 ? x + 1.0 : x + 0.5, g.Hx, g.Gx, i, err);
+    const double yd = index_axis(COMP == 1 ? y + 1.0 : y + 0.5, g.Hy, g.Gy, j, err);
+    const double zd = index_axis(COMP == 2 ? z + 1.0 : z + 0.5, g.Hz, g.Gz, k, err);
+    const double* __restrict__ p = f0 + gidx(g, i, j, k);
+    const int sy = g.Gx, sz = g.Gx * g.Gy;
+    double c000 = p[0], c001 = p[sz], c010 = p[sy], c011 = p[sy + sz];
+    double c100 = p[1], c101 = p[1 + sz], c110 = p[1 + sy], c111 = p[1 + sy + sz];
     double w000 = (1.0 - xd) * (1.0 - yd) * (1.0 - zd);
     double w001 = (1.0 - xd) * (1.0 - yd) * zd;
     double w010 = (1.0 - xd) * yd * (1.0 - zd);
@@ -131,49 +141,31 @@ __device__ __forceinline__ void particle_step(const DGrid& g, const PV& P, uint3
                                               const VelPtrs& vel, double kappa_h, double kappa_v,
                                               uint32_t* __restrict__ cnt, uint32_t* __restrict__ key,
                                               uint32_t* err) {
-    const int ac = 1;
     int oxi, oyi, ozi;
     unpack_cell(g, P.cell[slot], oxi, oyi, ozi);
     int kdz = clamp_idx((long long)ozi + g.Hz, 1, g.Gz, err);   // ΔzC at the stored zi + Hz
     const double X = P.x[slot], Y = P.y[slot], Z = P.z[slot];
     const double NX = (double)g.Nx, NY = (double)g.Ny, NZ = (double)g.Nz;
-    // stage 1 at vel₀
-    double u1 = jl_mulb(itpl<0, 0, LL>(g, vel.u0, vel.u0, X, Y, Z, ac, err), ac);
-    double v1 = jl_mulb(itpl<1, 0, LL>(g, vel.v0, vel.v0, X, Y, Z, ac, err), ac);
-    double w1 = jl_mulb(itpl<2, 0, LL>(g, vel.w0, vel.w0, X, Y, Z, ac, err), ac);
-    double u2 = u1, v2 = v1, w2 = w1;
-    double vx = X + jl_mulb(0.5 * u1 * dT, ac);
-    double vy = Y + jl_mulb(0.5 * v1 * dT, ac);
-    double vz = Z - jl_mulb(0.5 * w1 * dT, ac);
-    vx = jl_mulb(bc_pos(vx, NX, g.tx), ac); vy = jl_mulb(bc_pos(vy, NY, g.ty), ac); vz = jl_mulb(bc_pos(vz, NZ, g.tz), ac);
-    // stage 2 at vel½
-    u1 = jl_mulb(itpl<0, 0, LL>(g, vel.uh, vel.uh, vx, vy, vz, ac, err), ac);
-    v1 = jl_mulb(itpl<1, 0, LL>(g, vel.vh, vel.vh, vx, vy, vz, ac, err), ac);
-    w1 = jl_mulb(itpl<2, 0, LL>(g, vel.wh, vel.wh, vx, vy, vz, ac, err), ac);
-    u2 = u2 + u1 * 2.0; v2 = v2 + v1 * 2.0; w2 = w2 + w1 * 2.0;
-    vx = X + jl_mulb(0.5 * u1 * dT, ac);
-    vy = Y + jl_mulb(0.5 * v1 * dT, ac);
-    vz = Z - jl_mulb(0.5 * w1 * dT, ac);
-    vx = jl_mulb(bc_pos(vx, NX, g.tx), ac); vy = jl_mulb(bc_pos(vy, NY, g.ty), ac); vz = jl_mulb(bc_pos(vz, NZ, g.tz), ac);
-    // stage 3 at vel½
-    u1 = jl_mulb(itpl<0, 0, LL>(g, vel.uh, vel.uh, vx, vy, vz, ac, err), ac);
-    v1 = jl_mulb(itpl<1, 0, LL>(g, vel.vh, vel.vh, vx, vy, vz, ac, err), ac);
-    w1 = jl_mulb(itpl<2, 0, LL>(g, vel.wh, vel.wh, vx, vy, vz, ac, err), ac);
-    u2 = u2 + u1 * 2.0; v2 = v2 + v1 * 2.0; w2 = w2 + w1 * 2.0;
-    vx = X + jl_mulb(1.0 * u1 * dT, ac);
-    vy = Y + jl_mulb(1.0 * v1 * dT, ac);
-    vz = Z - jl_mulb(1.0 * w1 * dT, ac);
-    vx = jl_mulb(bc_pos(vx, NX, g.tx), ac); vy = jl_mulb(bc_pos(vy, NY, g.ty), ac); vz = jl_mulb(bc_pos(vz, NZ, g.tz), ac);
-    // stage 4 at vel₁
-    u1 = jl_mulb(itpl<0, 0, LL>(g, vel.u1, vel.u1, vx, vy, vz, ac, err), ac);
-    v1 = jl_mulb(itpl<1, 0, LL>(g, vel.v1, vel.v1, vx, vy, vz, ac, err), ac);
-    w1 = jl_mulb(itpl<2, 0, LL>(g, vel.w1, vel.w1, vx, vy, vz, ac, err), ac);
-    u2 = u2 + u1; v2 = v2 + v1; w2 = w2 + w1;
+    // the four stages at vel₀, vel½, vel½, vel₁: one body, a quarter of the instructions of four
+    // (products by 1.0 are exact)
+    double u2 = 0.0, v2 = 0.0, w2 = 0.0, vx = X, vy = Y, vz = Z;
+#pragma unroll 1
+    for (int st = 0; st < 4; ++st) {
+        const double* __restrict__ fu = st == 0 ? vel.u0 : st == 3 ? vel.u1 : vel.uh;
+        const double* __restrict__ fv = st == 0 ? vel.v0 : st == 3 ? vel.v1 : vel.vh;
+        const double* __restrict__ fw = st == 0 ? vel.w0 : st == 3 ? vel.w1 : vel.wh;
+        const double u1 = itpl<0, LL>(g, fu, vx, vy, vz, err);
+        const double v1 = itpl<1, LL>(g, fv, vx, vy, vz, err);
+        const double w1 = itpl<2, LL>(g, fw, vx, vy, vz, err);
+        const double wt = st == 1 || st == 2 ? 2.0 : 1.0, hs = st < 2 ? 0.5 : 1.0;
+        if (st == 0) { u2 = u1; v2 = v1; w2 = w1; }
+        else { u2 = u2 + u1 * wt; v2 = v2 + v1 * wt; w2 = w2 + w1 * wt; }
+        vx = bc_pos(X + hs * u1 * dT, NX, g.tx); vy = bc_pos(Y + hs * v1 * dT, NY, g.ty); vz = bc_pos(Z - hs * w1 * dT, NZ, g.tz);
+    }
     u2 = u2 / 6.0; v2 = v2 / 6.0; w2 = w2 / 6.0;
-    double x = X + jl_mulb(1.0 * u2 * dT, ac);
-    double y = Y + jl_mulb(1.0 * v2 * dT, ac);
-    double z = Z - jl_mulb(1.0 * w2 * dT, ac);
-    x = jl_mulb(bc_pos(x, NX, g.tx), ac); y = jl_mulb(bc_pos(y, NY, g.ty), ac); z = jl_mulb(bc_pos(z, NZ, g.tz), ac);
+    double x = bc_pos(X + 1.0 * u2 * dT, NX, g.tx);
+    double y = bc_pos(Y + 1.0 * v2 * dT, NY, g.ty);
+    double z = bc_pos(Z - 1.0 * w2 * dT, NZ, g.tz);
     // diffusion: rnd ∈ [0,1) → (rnd - 0.5) * 2 → · √(κΔT) / Δ
     double r0, r1, r2;
     pi_draw3(seed, iter, dsp, purpose, (uint32_t)slot, &r0, &r1, &r2);
@@ -184,13 +176,12 @@ __device__ __forceinline__ void particle_step(const DGrid& g, const PV& P, uint3
     r0 = r0 * sqrt(kappa_h * dT) / dxCm<LL>(g, dxi, dyi);
     r1 = r1 * sqrt(kappa_h * dT) / dyCm<LL>(g, dxi, dyi);
     r2 = r2 * sqrt(kappa_v * dT) / dzC1(g, kdz);
-    x = x + jl_mulb(r0, ac); y = y + jl_mulb(r1, ac); z = z + jl_mulb(r2, ac);
-    x = jl_mulb(bc_pos(x, NX, g.tx), ac); y = jl_mulb(bc_pos(y, NY, g.ty), ac); z = jl_mulb(bc_pos(z, NZ, g.tz), ac);
+    x = bc_pos(x + r0, NX, g.tx); y = bc_pos(y + r1, NY, g.ty); z = bc_pos(z + r2, NZ, g.tz);
     P.x[slot] = x; P.y[slot] = y; P.z[slot] = z;
     // find_inds!
-    int xi = clamp_idx(jl_trunc(jl_mulb(x + 1.0, ac)) + g.Hx, 1, g.Gx, err);
-    int yi = clamp_idx(jl_trunc(jl_mulb(y + 1.0, ac)) + g.Hy, 1, g.Gy, err);
-    int zi = clamp_idx(jl_trunc(jl_mulb(z + 1.0, ac)) + g.Hz, 1, g.Gz, err);
+    int xi = clamp_idx(jl_trunc(x + 1.0) + g.Hx, 1, g.Gx, err);
+    int yi = clamp_idx(jl_trunc(y + 1.0) + g.Hy, 1, g.Gy, err);
+    int zi = clamp_idx(jl_trunc(z + 1.0) + g.Hz, 1, g.Gz, err);
     P.cell[slot] = pack_cell(g, xi, yi, zi);
     if (BIN) {
         int c = gidx(g, xi, yi, zi);
@@ -214,7 +205,10 @@ __global__ void k_particles(DGrid g, const SpcDev* __restrict__ spc, int nsp, lo
     int s = (int)(gid / C);
     long long slot = gid - (long long)s * C;
     const SpcDev& P = spc[s];
+    const uint8_t stt = P.stat[slot];
     if (!(P.flags[slot] & FL_AC)) {
+        if (stt & ST_HOME) return;                    // as this pass left it
+        P.stat[slot] = ST_HOME;
         int oxi, oyi, ozi;
         unpack_cell(g, P.cell[slot], oxi, oyi, ozi);
         clamp_idx((long long)ozi + g.Hz, 1, g.Gz, err);
@@ -225,15 +219,19 @@ __global__ void k_particles(DGrid g, const SpcDev* __restrict__ spc, int nsp, lo
         key[gid] = sentinel;
         return;
     }
-    if (P.stat[slot] & ST_AC0) return;                // moved by k_particles_sorted
+    if (stt & ST_AC0) return;                         // moved by k_particles_sorted
     particle_step<LL>(g, P, (uint32_t)s, PI_DRAW_DIFFUSION, slot, gid, dT, seed, iter, vel, kappa_h, kappa_v, cnt, key,
                       err);
 }
 
 // Cell-order pass: the individuals binned in the previous step (prev_sorted[0 .. off[G]), which
 // were active then) that are still active. Neighbouring threads interpolate in neighbouring cells.
+// Bound by the latency of FP64 chains (96 quotients and as many loads per individual), so warps count
+// more than registers: 110 registers 275 µs, 80 registers 227 µs for 1,048,576 individuals. Dividing
+// by reciprocals with exact remainders was slower than the division (301 µs): the compiler already
+// shares the reciprocal of a divisor.
 template <bool LL>
-__global__ void k_particles_sorted(DGrid g, const SpcDev* __restrict__ spc, long long C,
+__global__ void __launch_bounds__(128, 6) k_particles_sorted(DGrid g, const SpcDev* __restrict__ spc, long long C,
                                    const uint32_t* __restrict__ prev_sorted,
                                    const uint32_t* __restrict__ prev_off, long long Gcells,
                                    double dT, uint64_t seed, uint32_t iter, VelPtrs vel,
@@ -370,7 +368,7 @@ __global__ void k_decide(DGrid g, SpcDev P, pi_quota_params p, pi_macro_params m
     if (*err & PI_DEVERR_CAPACITY) return;
     uint8_t f = P.flags[slot];
     int ac0 = f & FL_AC, gz = (f & FL_GRAZ) != 0, mt = (f & FL_MORT) != 0, dv = (f & FL_DVID) != 0;
-    P.stat[slot] = ac0 ? ST_AC0 : 0;
+    P.stat[slot] = ac0 ? ST_AC0 : (uint8_t)(P.stat[slot] & ST_HOME);
     int ac1 = ac0 && !gz;          // inactivate!(plank, graz): ac &= isless(graz, 1)
     int ac2 = ac1 && !mt;          // inactivate!(plank, mort)
     int dv2 = dv && ac2;           // plank.dvid .*= plank.ac

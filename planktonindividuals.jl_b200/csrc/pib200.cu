@@ -414,11 +414,14 @@ pi_status enqueue_step(pi_model* m, double dT) {
     const int BS = 256;
 
     CK(cudaMemsetAsync(sb.cnt, 0, (G + 1) * sizeof(uint32_t), st), "zero counts");
-    { ProfScope ps_(m, "k_velhalf");
+    // vel½ = (vel₀ + vel₁)·0.5 is vel₁ itself, bit for bit, while vel₀ and vel₁ are the same field
+    const bool steady = m->vel0[0] == m->vel1[0] && m->vel0[1] == m->vel1[1] && m->vel0[2] == m->vel1[2];
+    const double* const* vh = steady ? m->vel1 : (const double* const*)m->velh;
+    if (!steady) { ProfScope ps_(m, "k_velhalf");
     k_velhalf<<<148 * 8, 256, 0, st>>>(G, m->vel0[0], m->vel0[1], m->vel0[2], m->vel1[0], m->vel1[1], m->vel1[2],
                                        m->velh[0], m->velh[1], m->velh[2], sb.err);
     CK(cudaGetLastError(), "k_velhalf"); }
-    VelPtrs vp{m->vel0[0], m->vel0[1], m->vel0[2], m->velh[0], m->velh[1], m->velh[2],
+    VelPtrs vp{m->vel0[0], m->vel0[1], m->vel0[2], vh[0], vh[1], vh[2],
                m->vel1[0], m->vel1[1], m->vel1[2]};
     const bool ll = m->met != nullptr;      // LatLonGrid: the kernels that read grid metrics take their arrays
     if (m->nsa) { pi_status e = enqueue_abiotic_update(m, dT, vp); if (e) return e; }

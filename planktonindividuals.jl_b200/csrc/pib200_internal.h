@@ -49,6 +49,7 @@
 
 // Per-step status byte.
 #define ST_AC0  1u   // active when cells were found (find_inds!/find_NPT! time)
+#define ST_HOME 2u   // inactive, and its position, cell and binning key are those of an inactive slot
 
 // Grid description passed by value to kernels. Indices inside kernels are the reference's
 // 1-based, halo-inclusive (i, j, k).
