@@ -102,7 +102,7 @@ __global__ void k_abio_move(DGrid g, AbioDev A, long long C, int sa, double dT, 
         return;
     }
     particle_step<LL, false>(g, A, (uint32_t)sa, PI_DRAW_ABIO_DIFFUSION, k, 0, dT, seed, iter, vel, kappa_h, kappa_v,
-                             nullptr, nullptr, err);
+                             nullptr, nullptr, nullptr, err);
 }
 
 // sort keys of the active particles: their find_inds! cell (G when inactive), value the slot

@@ -134,13 +134,14 @@ struct VelPtrs { const double *u0, *v0, *w0, *uh, *vh, *wh, *u1, *v1, *w1; };
 // RK4 + diffusion + find_inds! of one active particle at `slot` of the columns x, y, z, cell of P
 // (a phytoplankton species, SpcDev, or an abiotic species, AbioDev, whose steps are the same
 // kernels, time_step.jl:29-38); the diffusion draw is keyed by (dsp, purpose). BIN: writes the
-// binning key and count of a phytoplankton individual.
+// binning key of a phytoplankton individual and its number among those of its cell (in the order
+// of the atomics).
 template <bool LL, bool BIN = true, class PV>
 __device__ __forceinline__ void particle_step(const DGrid& g, const PV& P, uint32_t dsp, uint32_t purpose, long long slot,
                                               long long gid, double dT, uint64_t seed, uint32_t iter,
                                               const VelPtrs& vel, double kappa_h, double kappa_v,
                                               uint32_t* __restrict__ cnt, uint32_t* __restrict__ key,
-                                              uint32_t* err) {
+                                              int32_t* __restrict__ pos, uint32_t* err) {
     int oxi, oyi, ozi;
     unpack_cell(g, P.cell[slot], oxi, oyi, ozi);
     int kdz = clamp_idx((long long)ozi + g.Hz, 1, g.Gz, err);   // ΔzC at the stored zi + Hz
@@ -186,7 +187,7 @@ __device__ __forceinline__ void particle_step(const DGrid& g, const PV& P, uint3
     if (BIN) {
         int c = gidx(g, xi, yi, zi);
         key[gid] = (uint32_t)c;
-        atomicAdd(&cnt[c], 1u);
+        pos[gid] = (int32_t)atomicAdd(&cnt[c], 1u);
     }
 }
 
@@ -198,7 +199,7 @@ template <bool LL>
 __global__ void k_particles(DGrid g, const SpcDev* __restrict__ spc, int nsp, long long C,
                             double dT, uint64_t seed, uint32_t iter, VelPtrs vel,
                             double kappa_h, double kappa_v, uint32_t* __restrict__ cnt,
-                            uint32_t* __restrict__ key, uint32_t sentinel, uint32_t* err) {
+                            uint32_t* __restrict__ key, int32_t* __restrict__ pos, uint32_t sentinel, uint32_t* err) {
     long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (gid >= (long long)nsp * C) return;
     if (*err & PI_DEVERR_CAPACITY) return;
@@ -221,7 +222,7 @@ __global__ void k_particles(DGrid g, const SpcDev* __restrict__ spc, int nsp, lo
     }
     if (stt & ST_AC0) return;                         // moved by k_particles_sorted
     particle_step<LL>(g, P, (uint32_t)s, PI_DRAW_DIFFUSION, slot, gid, dT, seed, iter, vel, kappa_h, kappa_v, cnt, key,
-                      err);
+                      pos, err);
 }
 
 // Cell-order pass: the individuals binned in the previous step (prev_sorted[0 .. off[G]), which
@@ -236,7 +237,7 @@ __global__ void __launch_bounds__(128, 6) k_particles_sorted(DGrid g, const SpcD
                                    const uint32_t* __restrict__ prev_off, long long Gcells,
                                    double dT, uint64_t seed, uint32_t iter, VelPtrs vel,
                                    double kappa_h, double kappa_v, uint32_t* __restrict__ cnt,
-                                   uint32_t* __restrict__ key, uint32_t* err) {
+                                   uint32_t* __restrict__ key, int32_t* __restrict__ pos, uint32_t* err) {
     long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (*err & PI_DEVERR_CAPACITY) return;
     if (p >= (long long)prev_off[Gcells]) return;
@@ -246,17 +247,73 @@ __global__ void __launch_bounds__(128, 6) k_particles_sorted(DGrid g, const SpcD
     const SpcDev& P = spc[s];
     if (!(P.flags[slot] & FL_AC) || !(P.stat[slot] & ST_AC0)) return;
     particle_step<LL>(g, P, (uint32_t)s, PI_DRAW_DIFFUSION, slot, gd, dT, seed, iter, vel, kappa_h, kappa_v, cnt, key,
-                      err);
+                      pos, err);
 }
 
-// pos[gid] = position of gid in the cell-sorted entry list.
-__global__ void k_setpos(const uint32_t* __restrict__ off, long long G,
-                         const uint32_t* __restrict__ gid_sorted, int32_t* __restrict__ pos,
-                         long long n, const uint32_t* err) {
-    long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+// The cell-sorted entry list (cells in order, gid = species·C + slot ascending within a cell, the
+// order of a sequential reference run) from the counting sort that k_particles began: k64_place puts
+// the individuals of a cell together in the order of the atomics, k64_order gives each its rank by
+// gid among them. A cell holds a few individuals, so a rank is a few comparisons; cells with more
+// than ORDER_BIG are left to k64_order_big. The radix sort of all keys took six launches: 35 µs for
+// 32,768 slots, 80 µs for 2,097,152.
+#define ORDER_BIG 2048
+__global__ void k64_place(const uint32_t* __restrict__ off, uint32_t Gcells, const uint32_t* __restrict__ key,
+                          const int32_t* __restrict__ pos, uint32_t* __restrict__ list, long long n, const uint32_t* err) {
+    const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (gid >= n || (*err & PI_DEVERR_CAPACITY)) return;
+    const uint32_t c = key[gid];
+    if (c < Gcells) list[off[c] + (uint32_t)pos[gid]] = (uint32_t)gid;
+}
+__global__ void k64_order(const uint32_t* __restrict__ off, long long G, const uint32_t* __restrict__ key,
+                          const uint32_t* __restrict__ list, uint32_t* __restrict__ gid_sorted, int32_t* __restrict__ pos,
+                          long long n, uint32_t* __restrict__ nbig, uint32_t* __restrict__ big, const uint32_t* err) {
+    const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= n || (*err & PI_DEVERR_CAPACITY) || p >= (long long)off[G]) return;
+    const uint32_t gid = list[p], c = key[gid], p0 = off[c], m = off[c + 1] - p0;
+    if (m > ORDER_BIG) {
+        if (p == (long long)p0) big[atomicAdd(nbig, 1u)] = c;
+        return;
+    }
+    uint32_t r = 0;
+#pragma unroll 4
+    for (uint32_t x = 0; x < m; ++x) r += list[p0 + x] < gid;
+    gid_sorted[p0 + r] = gid;
+    pos[gid] = (int32_t)(p0 + r);
+}
+// A block per crowded cell (0D models: one cell holds every individual): the keys of all slots are in
+// gid order, so the cell's run is the slots with its key one after another. Each warp counts its share
+// of the keys, then writes behind the counts of the warps before it.
+__global__ void __launch_bounds__(1024) k64_order_big(const uint32_t* __restrict__ off, const uint32_t* __restrict__ key, long long n,
+                                                      const uint32_t* __restrict__ nbig, const uint32_t* __restrict__ big,
+                                                      uint32_t* __restrict__ gid_sorted, int32_t* __restrict__ pos,
+                                                      const uint32_t* err) {
+    __shared__ uint32_t sh[32];
     if (*err & PI_DEVERR_CAPACITY) return;
-    if (p >= n || p >= (long long)off[G]) return;
-    pos[gid_sorted[p]] = (int32_t)p;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const long long run = (n + 1023) / 1024 * 32, a = min(n, wid * run), b = min(n, a + run);
+    for (uint32_t t = blockIdx.x; t < *nbig; t += gridDim.x) {
+        const uint32_t c = big[t];
+        uint32_t m = 0;
+#pragma unroll 8
+        for (long long q = a; q < b; q += 32) m += __popc(__ballot_sync(0xffffffffu, q + lane < b && key[q + lane] == c));
+        if (lane == 0) sh[wid] = m;
+        __syncthreads();
+        uint32_t at = off[c];
+        for (int w = 0; w < wid; ++w) at += sh[w];
+        if (m) {
+            for (long long q = a; q < b; q += 32) {
+                const bool in = q + lane < b && key[q + lane] == c;
+                const unsigned mk = __ballot_sync(0xffffffffu, in);
+                if (in) {
+                    const uint32_t e = at + __popc(mk & ((1u << lane) - 1u));
+                    gid_sorted[e] = (uint32_t)(q + lane);
+                    pos[q + lane] = (int32_t)e;
+                }
+                at += __popc(mk);
+            }
+        }
+        __syncthreads();
+    }
 }
 
 // ------------------------------------------------------------------------------------------
@@ -354,21 +411,21 @@ __host__ __device__ __forceinline__ double m_totP(double DNA, double RNA, double
 }
 
 // Applies last step's grazing/mortality decisions, writes the loss contributions of the
-// individuals lost, the division/free flags for the slot scan and the graz/mort/dvid diags.
+// individuals lost, the divider and free-slot bits of 32 slots per word and the graz/mort/dvid diags.
 // mode MODE_CARBON: CarbonMode losses (CarbonMode/consume_loss.jl:12-16), DOC and POC from Bm only;
 // MODE_MACRO: MacroMolecularMode losses (MacroMolecularMode/consume_loss.jl:14-24) from the total
 // C, N and P biomass (mp holds its R_NC_* and R_PC_* ratios).
 __global__ void k_decide(DGrid g, SpcDev P, pi_quota_params p, pi_macro_params mp, pi_iron_params ip, long long C, int s,
                          const int32_t* __restrict__ pos, double* __restrict__ loss,
-                         uint8_t* __restrict__ evk, unsigned long long* __restrict__ flag64,
+                         uint8_t* __restrict__ evk, uint32_t* __restrict__ dvw, uint32_t* __restrict__ frw,
                          double* __restrict__ d_graz, double* __restrict__ d_mort,
                          double* __restrict__ d_dvid, uint32_t* err, int mode) {
     long long slot = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (slot >= C) return;
     if (*err & PI_DEVERR_CAPACITY) return;
-    uint8_t f = P.flags[slot];
+    const bool in = slot < C;
+    uint8_t f = in ? P.flags[slot] : 0;
     int ac0 = f & FL_AC, gz = (f & FL_GRAZ) != 0, mt = (f & FL_MORT) != 0, dv = (f & FL_DVID) != 0;
-    P.stat[slot] = ac0 ? ST_AC0 : (uint8_t)(P.stat[slot] & ST_HOME);
+    if (in) P.stat[slot] = ac0 ? ST_AC0 : (uint8_t)(P.stat[slot] & ST_HOME);
     int ac1 = ac0 && !gz;          // inactivate!(plank, graz): ac &= isless(graz, 1)
     int ac2 = ac1 && !mt;          // inactivate!(plank, mort)
     int dv2 = dv && ac2;           // plank.dvid .*= plank.ac
@@ -431,13 +488,14 @@ __global__ void k_decide(DGrid g, SpcDev P, pi_quota_params p, pi_macro_params m
             }
         }
     }
-    P.flags[slot] = (uint8_t)((ac2 ? FL_AC : 0) | (dv2 ? FL_DVID : 0));
-    flag64[slot] = ((unsigned long long)dv2 << 32) | (unsigned long long)(!ac2);
+    if (in) P.flags[slot] = (uint8_t)((ac2 ? FL_AC : 0) | (dv2 ? FL_DVID : 0));
+    // dividers and free slots, one bit per slot
+    const uint32_t wd = __ballot_sync(0xffffffffu, dv2), wf = __ballot_sync(0xffffffffu, in && !ac2);
+    if ((threadIdx.x & 31) == 0 && in) { dvw[slot >> 5] = wd; frw[slot >> 5] = wf; }
 }
 
-// After the exclusive scan of flag64: the k-th divider (slot order) and the k-th free slot
-// (findall(!ac), ascending) — get_tind!, Individuals/utils.jl:76-86. Checks capacity
-// (plankton_update.jl:18-22).
+// After the exclusive scan of flag64 (abiotic release): the k-th releaser (slot order) and the k-th
+// free slot (findall(!ac), ascending) — get_tind!, Individuals/utils.jl:76-86. Checks capacity.
 __global__ void k_lists(const unsigned long long* __restrict__ flag64,
                         const unsigned long long* __restrict__ rank64, long long C,
                         int32_t* __restrict__ divlist, int32_t* __restrict__ freelist,
@@ -468,59 +526,104 @@ __global__ void k_lists(const unsigned long long* __restrict__ flag64,
 // (division_death.jl:28-63). Other slots are unchanged by divide_to_half (factor 1, +0, ×1).
 // CarbonMode (CarbonMode/division_death.jl:28-57): x, y, z, Sz, Bm, Chl and gen are copied, Bd is
 // not — the daughter halves the damaged biomass its slot held before.
+// the pools of a mode, copied and halved in both
+template <int N>
+__device__ __forceinline__ void halve_pools(double* const (&pools)[N], long long p, long long d) {
+    const double h = (2.0 - 1.0) / 2.0;
+    double v[N];
+#pragma unroll
+    for (int q = 0; q < N; ++q) v[q] = pools[q][p] * h;
+#pragma unroll
+    for (int q = 0; q < N; ++q) { pools[q][d] = v[q]; pools[q][p] = v[q]; }
+}
+// divider p and its daughter's slot d; every mode reads before it writes (the slots are different)
+__device__ __forceinline__ void daughter_pair(const SpcDev& P, long long p, long long d, int mode) {
+    const double h = (2.0 - 1.0) / 2.0;
+    const double x = P.x[p], y = P.y[p], z = P.z[p], gen = P.gen[p];
+    const double aged = P.age[d] * (1.0 - 1.0), agep = P.age[p] * (1.0 - 1.0);
+    P.x[d] = x; P.y[d] = y; P.z[d] = z;
+    P.gen[d] = gen + 1.0; P.age[d] = aged;
+    P.flags[d] = FL_AC | FL_DVID;
+    P.gen[p] = gen + 1.0; P.age[p] = agep;
+    if (mode == MODE_IRON) {
+        // IronEnergyMode/division_death.jl:44-82: x, y, z, tdark and gen copied; Sz, Bm, CH, the
+        // quotas, exEn and Chl copied and halved in both; age not copied
+        P.tdark[d] = P.tdark[p];
+        double* const pools[12] = { P.Sz, P.Bm, P.CH, P.qNO3, P.qNH4, P.qP, P.qFe, P.qFePS, P.qFeNR, P.qFeNF, P.exEn, P.Chl };
+        halve_pools(pools, p, d);
+    } else if (mode == MODE_MACRO) {
+        // MacroMolecularMode/division_death.jl:28-62: the seven pools, x, y, z and gen are
+        // copied and halved in both (not age)
+        double* const pools[7] = { P.PRO, P.DNA, P.RNA, P.CH, P.NST, P.PST, P.Chl };
+        halve_pools(pools, p, d);
+    } else if (mode == MODE_CARBON) {
+        const double bd = P.Bd[d] * h, bp = P.Bd[p] * h;
+        P.Bd[d] = bd; P.Bd[p] = bp;
+        double* const pools[3] = { P.Sz, P.Bm, P.Chl };
+        halve_pools(pools, p, d);
+    } else {
+        double* const pools[6] = { P.Sz, P.Bm, P.Cq, P.Nq, P.Pq, P.Chl };
+        halve_pools(pools, p, d);
+    }
+}
 __global__ void k_daughters(SpcDev P, const int32_t* __restrict__ divlist,
                             const int32_t* __restrict__ freelist, const uint32_t* ndiv,
                             const uint32_t* err, int mode) {
     if (*err & PI_DEVERR_CAPACITY) return;
     uint32_t n = *ndiv;
-    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        long long p = divlist[k], d = freelist[k];
-        const double h = (2.0 - 1.0) / 2.0;
-        if (mode == MODE_IRON) {
-            // IronEnergyMode/division_death.jl:44-82: x, y, z, tdark and gen copied; Sz, Bm, CH, the
-            // quotas, exEn and Chl copied and halved in both; age not copied
-            double* pools[12] = { P.Sz, P.Bm, P.CH, P.qNO3, P.qNH4, P.qP, P.qFe, P.qFePS, P.qFeNR, P.qFeNF, P.exEn, P.Chl };
-            const double gen = P.gen[p];
-            P.x[d] = P.x[p]; P.y[d] = P.y[p]; P.z[d] = P.z[p]; P.tdark[d] = P.tdark[p];
-#pragma unroll
-            for (int q = 0; q < 12; ++q) { const double v = pools[q][p] * h; pools[q][d] = v; pools[q][p] = v; }
-            P.gen[d] = gen + 1.0; P.age[d] = P.age[d] * (1.0 - 1.0);
-            P.flags[d] = FL_AC | FL_DVID;
-            P.gen[p] = gen + 1.0; P.age[p] = P.age[p] * (1.0 - 1.0);
-            continue;
-        }
-        if (mode == MODE_MACRO) {
-            // MacroMolecularMode/division_death.jl:28-62: the seven pools, x, y, z and gen are
-            // copied and halved in both (not age)
-            double* pools[7] = { P.PRO, P.DNA, P.RNA, P.CH, P.NST, P.PST, P.Chl };
-            const double gen = P.gen[p];
-            P.x[d] = P.x[p]; P.y[d] = P.y[p]; P.z[d] = P.z[p];
-#pragma unroll
-            for (int q = 0; q < 7; ++q) { const double v = pools[q][p] * h; pools[q][d] = v; pools[q][p] = v; }
-            P.gen[d] = gen + 1.0; P.age[d] = P.age[d] * (1.0 - 1.0);
-            P.flags[d] = FL_AC | FL_DVID;
-            P.gen[p] = gen + 1.0; P.age[p] = P.age[p] * (1.0 - 1.0);
-            continue;
-        }
-        if (mode == MODE_CARBON) {
-            double Sz = P.Sz[p], Bm = P.Bm[p], Chl = P.Chl[p], gen = P.gen[p];
-            P.x[d] = P.x[p]; P.y[d] = P.y[p]; P.z[d] = P.z[p];
-            P.Sz[d] = Sz * h; P.Bm[d] = Bm * h; P.Bd[d] = P.Bd[d] * h; P.Chl[d] = Chl * h;
-            P.gen[d] = gen + 1.0; P.age[d] = P.age[d] * (1.0 - 1.0);
-            P.flags[d] = FL_AC | FL_DVID;
-            P.Sz[p] = Sz * h; P.Bm[p] = Bm * h; P.Bd[p] = P.Bd[p] * h; P.Chl[p] = Chl * h;
-            P.gen[p] = gen + 1.0; P.age[p] = P.age[p] * (1.0 - 1.0);
-            continue;
-        }
-        double Sz = P.Sz[p], Bm = P.Bm[p], Cq = P.Cq[p], Nq = P.Nq[p], Pq = P.Pq[p], Chl = P.Chl[p];
-        double gen = P.gen[p];
-        P.x[d] = P.x[p]; P.y[d] = P.y[p]; P.z[d] = P.z[p];
-        P.Sz[d] = Sz * h; P.Bm[d] = Bm * h; P.Cq[d] = Cq * h; P.Nq[d] = Nq * h; P.Pq[d] = Pq * h;
-        P.Chl[d] = Chl * h; P.gen[d] = gen + 1.0; P.age[d] = P.age[d] * (1.0 - 1.0);
-        P.flags[d] = FL_AC | FL_DVID;
-        P.Sz[p] = Sz * h; P.Bm[p] = Bm * h; P.Cq[p] = Cq * h; P.Nq[p] = Nq * h; P.Pq[p] = Pq * h;
-        P.Chl[p] = Chl * h; P.gen[p] = gen + 1.0; P.age[p] = P.age[p] * (1.0 - 1.0);
+    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x)
+        daughter_pair(P, divlist[k], freelist[k], mode);
+}
+
+// The k-th divider (slot order) and the k-th free slot (findall(!ac), ascending) — get_tind!,
+// Individuals/utils.jl:76-86 — by one block from k_decide's bits, with the capacity check
+// (plankton_update.jl:18-22): each warp counts a run of words, then lists behind the warps before it,
+// and with `daughters` the block copies and halves them too. A scan of one 64-bit flag per slot and
+// two kernels took 20 µs at any size (the words are a 32nd of the slots: 64 KB for 262,144).
+__global__ void __launch_bounds__(1024) k64_divide(SpcDev P, long long C, const uint32_t* __restrict__ dvw,
+                                                   const uint32_t* __restrict__ frw, int32_t* divlist, int32_t* freelist,
+                                                   uint32_t* ndiv, uint32_t* err, int64_t* err_iter, int64_t iter,
+                                                   int daughters, int mode) {
+    __shared__ uint32_t shd[32], shf[32];
+    if (*err & PI_DEVERR_CAPACITY) return;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const long long words = (C + 31) / 32, run = (words + 1023) / 1024 * 32, w0 = min(words, wid * run), w1 = min(words, w0 + run);
+    uint32_t nd = 0, nf = 0;
+#pragma unroll 4
+    for (long long w = w0 + lane; w < w1; w += 32) { nd += __popc(dvw[w]); nf += __popc(frw[w]); }
+    nd = __reduce_add_sync(0xffffffffu, nd);
+    nf = __reduce_add_sync(0xffffffffu, nf);
+    if (lane == 0) { shd[wid] = nd; shf[wid] = nf; }
+    __syncthreads();
+    uint32_t tdiv = 0, tfree = 0, db = 0, fb = 0;
+    for (int w = 0; w < 32; ++w) {
+        if (w < wid) { db += shd[w]; fb += shf[w]; }
+        tdiv += shd[w]; tfree += shf[w];
     }
+    if (tdiv > tfree) {
+        if (threadIdx.x == 0) { *ndiv = 0; *err_iter = iter; __threadfence(); set_err(err, PI_DEVERR_CAPACITY); }
+        return;
+    }
+    if (threadIdx.x == 0) *ndiv = tdiv;
+    if (tdiv == 0) return;
+    for (long long w = w0; w < w1 && (nd || fb < tdiv); w += 32) {          // uniform over the warp
+        uint32_t dw = nd && w + lane < w1 ? dvw[w + lane] : 0u, fw = fb < tdiv && w + lane < w1 ? frw[w + lane] : 0u;
+        uint32_t cd = __popc(dw), cf = __popc(fw), xd = cd, xf = cf;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t yd = __shfl_up_sync(0xffffffffu, xd, o), yf = __shfl_up_sync(0xffffffffu, xf, o);
+            if (lane >= o) { xd += yd; xf += yf; }
+        }
+        uint32_t rd = db + xd - cd, rf = fb + xf - cf;
+        const int32_t s0 = (int32_t)((w + lane) * 32);
+        while (dw) { divlist[rd++] = s0 + __ffs(dw) - 1; dw &= dw - 1u; }
+        while (fw && rf < tdiv) { freelist[rf++] = s0 + __ffs(fw) - 1; fw &= fw - 1u; }
+        db += __shfl_sync(0xffffffffu, xd, 31);
+        fb += __shfl_sync(0xffffffffu, xf, 31);
+    }
+    if (!daughters) return;
+    __syncthreads();
+    for (uint32_t k = threadIdx.x; k < tdiv; k += blockDim.x) daughter_pair(P, divlist[k], freelist[k], mode);
 }
 
 // ------------------------------------------------------------------------------------------

@@ -4,10 +4,10 @@
 // A step (TimeStep!, src/Model/time_step.jl:12-180) is this sequence of launches:
 //   k_particles          RK4 + diffusion + find_inds! for every species; per-cell counts
 //   scan(cnt) → off      cell offsets of the binned individuals
-//   radix sort           (cell, species·C + slot) order = the order of a sequential reference run
-//   k_setpos             position of each individual in the cell-sorted list
+//   k64_place/order      (cell, species·C + slot) order = the order of a sequential reference run,
+//                        and each individual's position in it
 //   k64_par              Chl per cell, calc_par! down each column, PAR diagnostic
-//   per species:         k_decide → scan(flags) → k_lists → k_daughters → k_physiology
+//   per species:         k_decide → k64_divide (→ k_daughters) → k_physiology
 //   k64_plk              particle terms of the occupied cells
 //   k64_xy               DST3FL x and y sweeps
 //   k64_ztail            z sweep, diffusion, sinking, forcing, BCs, particle terms, apply_tendency!
@@ -105,7 +105,6 @@ struct pi_model {
     double* met = nullptr;           // LatLonGrid metrics: dxC, dyC, dxF, dyF, Az (Gx·Gy each), Ax, Ay, Vol (G each)
     std::vector<double> met_host;    // their host copy, the source of the upload
     StepBufs sb{};
-    uint32_t* iota = nullptr;    // nsp·C
     void* cub_tmp = nullptr;
     size_t cub_bytes = 0;
     int key_bits = 1;
@@ -375,6 +374,11 @@ pi_status enqueue_abiotic_exchange(pi_model* m, double dT) {
 }
 
 // Enqueues one TimeStep! on the model's stream (no synchronisation).
+// Most slots of a species whose daughters k64_divide's one block copies: above, dividers come by the
+// thousand and k_daughters' 592 blocks are faster than one block's waits (the lists alone take one
+// block about 17 µs for 1,048,576 slots, where the scan and list kernels took 19).
+#define DIVIDE_INBLOCK 262144
+
 // Rows or levels walked by a block of a tracer kernel (a power of two up to `most`): two blocks fit an
 // SM, a walk of n costs about n + over (the rows it reads beside its own, or the set-up), and the
 // length with the shortest waves × walk is taken. On 128×128×1 that is 4 rows (160 blocks), on
@@ -413,7 +417,7 @@ pi_status enqueue_step(pi_model* m, double dT) {
     StepBufs& sb = m->sb;
     const int BS = 256;
 
-    CK(cudaMemsetAsync(sb.cnt, 0, (G + 1) * sizeof(uint32_t), st), "zero counts");
+    CK(cudaMemsetAsync(sb.cnt, 0, (G + 2) * sizeof(uint32_t), st), "zero counts");
     // vel½ = (vel₀ + vel₁)·0.5 is vel₁ itself, bit for bit, while vel₀ and vel₁ are the same field
     const bool steady = m->vel0[0] == m->vel1[0] && m->vel0[1] == m->vel1[1] && m->vel0[2] == m->vel1[2];
     const double* const* vh = steady ? m->vel1 : (const double* const*)m->velh;
@@ -427,23 +431,24 @@ pi_status enqueue_step(pi_model* m, double dT) {
     if (m->nsa) { pi_status e = enqueue_abiotic_update(m, dT, vp); if (e) return e; }
     { ProfScope ps_(m, "k_particles_sorted");
     (ll ? k_particles_sorted<true> : k_particles_sorted<false>)<<<nblk(NC, 128), 128, 0, st>>>(g, m->d_spc, C, sb.gid_sorted, sb.off, G, dT, m->seed, iter, vp,
-                                                      m->bgc.kappa_hP, m->bgc.kappa_vP, sb.cnt, sb.key, sb.err);
+                                                      m->bgc.kappa_hP, m->bgc.kappa_vP, sb.cnt, sb.key, sb.pos, sb.err);
     CK(cudaGetLastError(), "k_particles_sorted"); }
     { ProfScope ps_(m, "k_particles");
     (ll ? k_particles<true> : k_particles<false>)<<<nblk(NC, BS), BS, 0, st>>>(g, m->d_spc, m->nsp, C, dT, m->seed, iter, vp,
-                                             m->bgc.kappa_hP, m->bgc.kappa_vP, sb.cnt, sb.key,
+                                             m->bgc.kappa_hP, m->bgc.kappa_vP, sb.cnt, sb.key, sb.pos,
                                              (uint32_t)G, sb.err);
     CK(cudaGetLastError(), "k_particles"); }
     size_t tb = m->cub_bytes;
     { ProfScope ps_(m, "cub_scan_cells");
     CK(cub::DeviceScan::ExclusiveSum(m->cub_tmp, tb, sb.cnt, sb.off, (int)(G + 1), st), "scan counts"); }
-    tb = m->cub_bytes;
-    { ProfScope ps_(m, "cub_sort_cells");
-    CK(cub::DeviceRadixSort::SortPairs(m->cub_tmp, tb, sb.key, sb.key_sorted, m->iota, sb.gid_sorted,
-                                       (int64_t)NC, 0, m->key_bits, st), "sort by cell"); }
-    { ProfScope ps_(m, "k_setpos");
-    k_setpos<<<nblk(NC, BS), BS, 0, st>>>(sb.off, G, sb.gid_sorted, sb.pos, NC, sb.err);
-    CK(cudaGetLastError(), "k_setpos"); }
+    { ProfScope ps_(m, "k64_order");
+    k64_place<<<nblk(NC, BS), BS, 0, st>>>(sb.off, (uint32_t)G, sb.key, sb.pos, sb.list, NC, sb.err);
+    k64_order<<<nblk(NC, BS), BS, 0, st>>>(sb.off, G, sb.key, sb.list, sb.gid_sorted, sb.pos, NC, sb.nbig, sb.big, sb.err);
+    // no cell can be crowded in a model of few slots
+    if (NC > ORDER_BIG)
+        k64_order_big<<<(unsigned)std::min<long long>(148, NC / ORDER_BIG), 1024, 0, st>>>(sb.off, sb.key, NC, sb.nbig, sb.big, sb.gid_sorted,
+                                                                                           sb.pos, sb.err);
+    CK(cudaGetLastError(), "k64_order"); }
     {
         // as many warps per 32 columns as the levels give work to, in blocks of at least four
         const int lw = g.Nz <= PAR64_CH ? 1 : g.Nz <= 2 * PAR64_CH ? 2 : g.Nz <= 4 * PAR64_CH ? 4 : g.Nz <= 8 * PAR64_CH ? 8 : 16;
@@ -460,16 +465,15 @@ pi_status enqueue_step(pi_model* m, double dT) {
         const pi_macro_params mpz = m->macro ? m->mp[s] : pi_macro_params{};
         const pi_iron_params ipz = m->iron ? m->ipp[s] : pi_iron_params{};
         k_decide<<<nblk(C, BS), BS, 0, st>>>(g, m->h_spc[s], m->sp[s], mpz, ipz, C, s, sb.pos, sb.loss, sb.evk,
-                                             sb.flag64, dsp + 1 * G, dsp + 2 * G, dsp + 3 * G, sb.err, m->mode());
+                                             sb.dvw, sb.frw, dsp + 1 * G, dsp + 2 * G, dsp + 3 * G, sb.err, m->mode());
         CK(cudaGetLastError(), "k_decide"); }
-        tb = m->cub_bytes;
-        { ProfScope ps_(m, "cub_scan_slots");
-        CK(cub::DeviceScan::ExclusiveSum(m->cub_tmp, tb, sb.flag64, sb.rank64, (int64_t)C, st), "scan division flags"); }
-        { ProfScope ps_(m, "k_lists");
-        k_lists<<<nblk(C, BS), BS, 0, st>>>(sb.flag64, sb.rank64, C, sb.divlist, sb.freelist, sb.ndiv,
-                                            sb.err, sb.err_iter, m->iteration);
-        CK(cudaGetLastError(), "k_lists"); }
-        { ProfScope ps_(m, "k_daughters");
+        // one block copies the daughters too where they are few
+        const int inblock = C <= DIVIDE_INBLOCK;
+        { ProfScope ps_(m, "k64_divide");
+        k64_divide<<<1, 1024, 0, st>>>(m->h_spc[s], C, sb.dvw, sb.frw, sb.divlist, sb.freelist, sb.ndiv, sb.err, sb.err_iter,
+                                       m->iteration, inblock, m->mode());
+        CK(cudaGetLastError(), "k64_divide"); }
+        if (!inblock) { ProfScope ps_(m, "k_daughters");
         k_daughters<<<148 * 4, 256, 0, st>>>(m->h_spc[s], sb.divlist, sb.freelist, sb.ndiv, sb.err, m->mode());
         CK(cudaGetLastError(), "k_daughters"); }
         const double* trp = m->tr;
@@ -717,11 +721,12 @@ pi_status pi_create(const pi_grid* grid, const pi_bgc_params* bgc, const pi_quot
     ALB(m->zeros, G); ALB(m->par, G); ALB(m->PARF, (long long)hg.Nx * hg.Ny); ALB(m->temp_own, G);
     ALB(m->diag_par, G); ALB(m->diag_sp, 4LL * nspecies * G);
     StepBufs& sb = m->sb;
-    ALB(sb.cnt, G + 1); ALB(sb.off, G + 1); ALB(sb.key, NC); ALB(sb.key_sorted, NC);
+    ALB(sb.cnt, G + 2); ALB(sb.off, G + 1); ALB(sb.key, NC); ALB(sb.list, NC); ALB(sb.big, NC / ORDER_BIG + 1);
+    sb.nbig = sb.cnt + G + 1;
+    ALB(sb.dvw, (C + 31) / 32); ALB(sb.frw, (C + 31) / 32);
     ALB(sb.gid_sorted, NC); ALB(sb.pos, NC); ALB(sb.contrib, 5 * NC); ALB(sb.loss, 6 * NC);
     ALB(sb.evk, NC); ALB(sb.flag64, C); ALB(sb.rank64, C); ALB(sb.divlist, C); ALB(sb.freelist, C);
     ALB(sb.ndiv, 1); ALB(sb.err, 1); ALB(sb.err_iter, 1);
-    ALB(m->iota, NC);
     ALB(m->d_bcs, PI_NTRACERS * 6);
     m->h_spc.resize(nspecies);
     for (int s = 0; s < nspecies; ++s) {
@@ -760,12 +765,7 @@ pi_status pi_create(const pi_grid* grid, const pi_bgc_params* bgc, const pi_quot
         ok = ok && cudaMemsetAsync(P.stat, 0, C, s0) == cudaSuccess;
         ok = ok && cudaMemsetAsync(P.cell, 0, C * sizeof(int32_t), s0) == cudaSuccess;  // (0,0,0) as constructed
     }
-    {
-        std::vector<uint32_t> io(NC);
-        for (long long q = 0; q < NC; ++q) io[q] = (uint32_t)q;
-        ok = ok && cudaMemcpyAsync(m->iota, io.data(), NC * sizeof(uint32_t), cudaMemcpyHostToDevice, s0) == cudaSuccess;
-        ok = ok && cudaStreamSynchronize(s0) == cudaSuccess;
-    }
+    ok = ok && cudaStreamSynchronize(s0) == cudaSuccess;
     if (!ok) { m->err = "pi_create: device initialisation failed"; return bail(PI_ERR_CUDA); }
     // dynamic shared memory of the tracer kernels above the default limit
     for (auto* f : { k64_xy<false, false>, k64_xy<false, true>, k64_xy<true, false>, k64_xy<true, true> })
@@ -779,12 +779,11 @@ pi_status pi_create(const pi_grid* grid, const pi_bgc_params* bgc, const pi_quot
     m->temp = m->temp_own;
     m->key_bits = 1;
     while ((1LL << m->key_bits) <= G) ++m->key_bits;
-    // CUB scratch: the largest of the three uses
-    size_t b1 = 0, b2 = 0, b3 = 0;
+    // CUB scratch: the larger of the two uses
+    size_t b1 = 0, b3 = 0;
     cub::DeviceScan::ExclusiveSum(nullptr, b1, sb.cnt, sb.off, (int)(G + 1), s0);
-    cub::DeviceRadixSort::SortPairs(nullptr, b2, sb.key, sb.key_sorted, m->iota, sb.gid_sorted, (int64_t)NC, 0, m->key_bits, s0);
     cub::DeviceScan::ExclusiveSum(nullptr, b3, sb.flag64, sb.rank64, (int64_t)C, s0);
-    m->cub_bytes = std::max(b1, std::max(b2, b3));
+    m->cub_bytes = std::max(b1, b3);
     st = dalloc(m, (char**)&m->cub_tmp, m->cub_bytes, "cub scratch");
     if (st) return bail(st);
     m->dg = DGrid{hg.Nx, hg.Ny, hg.Nz, hg.Hx, hg.Hy, hg.Hz, hg.Gx, hg.Gy, hg.Gz,

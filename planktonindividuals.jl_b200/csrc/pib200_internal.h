@@ -117,16 +117,21 @@ struct FluxBCDev {
 
 // Per-step work arrays shared by the kernels.
 struct StepBufs {
-    uint32_t* cnt;          // G+1 counts of active individuals per cell
+    uint32_t* cnt;          // G+1 counts of active individuals per cell (then nbig)
     uint32_t* off;          // G+1 exclusive prefix of cnt
     uint32_t* key;          // nsp*C cell key (G-linear) per individual, sentinel when inactive
-    uint32_t* key_sorted;   // nsp*C
+    uint32_t* list;         // nsp*C: the cells' individuals in the order of the atomics
+    uint32_t* nbig;         // cells of more than ORDER_BIG individuals, listed in big
+    uint32_t* big;
     uint32_t* gid_sorted;   // nsp*C: gid = sp*C + slot sorted by (cell, gid)
-    int32_t* pos;           // nsp*C: position of gid in gid_sorted (valid when ST_AC0)
+    int32_t* pos;           // nsp*C: position of gid in gid_sorted (valid when ST_AC0); while binning,
+                            // its number among its cell's individuals
     double* contrib;        // 5 per entry: DIC, DOC, NH4, NO3, PO4 consumption
     double* loss;           // 6 per entry: DOC, DON, DOP, POC, PON, POP loss
     uint8_t* evk;           // per entry: 0 none, 1 grazing loss, 2 mortality loss
-    unsigned long long* flag64;   // C: (is_div << 32) | is_free
+    uint32_t* dvw;          // C/32: one bit per slot, a divider
+    uint32_t* frw;          // C/32: a free slot
+    unsigned long long* flag64;   // C: (releases << 32) | is_free (abiotic release)
     unsigned long long* rank64;   // C: exclusive prefix of flag64
     int32_t* divlist;       // C
     int32_t* freelist;      // C
