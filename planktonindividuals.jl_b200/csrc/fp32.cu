@@ -172,6 +172,8 @@ struct pi_batch {
     // queued steps: the buffer vel₁ is bound to (-1: a series snapshot), whether a setter bound it
     // after the last queued step, and the buffer that is vel₀ of the next step (-1: none)
     std::vector<int> vel1_buf, vel1_pending, vel0_buf;
+    unsigned long long* exp_buf = nullptr;   // columns of pi_batch_get_individuals on their way to the host
+    long long exp_slots = 0;
     double* partial = nullptr;      // budget partials
     unsigned long long* scratch = nullptr;
     // work tables (device) built for the current tuning
@@ -1082,62 +1084,61 @@ pi_status pi_batch_get_individuals(pi_batch* b, int32_t member, int32_t sp, pi_i
     if (e) return e;
     if (!out || sp < 0 || sp >= b->nsp) return bfail(b, PI_ERR_ARG, "pi_get_individuals: bad argument");
     const MemberHost& h = b->mh[member];
-    const HostGrid& g = h.g;
-    const long long C = h.C;
-    const long long g0 = b->mdh[member].slot_off + (long long)sp * C;
-    std::vector<int32_t> cell(C), scell(C), lslot(C);
-    std::vector<float> o[3], f[7];
-    std::vector<uint8_t> flags(C), stat(C);
-    const IndDev32& P = b->P;
-    cudaStream_t s = b->stream;
-    BK(cudaMemcpyAsync(lslot.data(), P.lslot + g0, C * 4, cudaMemcpyDeviceToHost, s), "download individuals");
-    BK(cudaMemcpyAsync(cell.data(), P.cell + g0, C * 4, cudaMemcpyDeviceToHost, s), "download individuals");
-    BK(cudaMemcpyAsync(scell.data(), P.scell + g0, C * 4, cudaMemcpyDeviceToHost, s), "download individuals");
-    const float* od[3] = { P.ox, P.oy, P.oz };
-    for (int a = 0; a < 3; ++a) { o[a].resize(C); BK(cudaMemcpyAsync(o[a].data(), od[a] + g0, C * 4, cudaMemcpyDeviceToHost, s), "download individuals"); }
-    const float* fd[7] = { P.Bm, P.Cq, P.Nq, P.Pq, P.Chl, P.age, P.gen };
-    for (int q = 0; q < 7; ++q) { f[q].resize(C); BK(cudaMemcpyAsync(f[q].data(), fd[q] + g0, C * 4, cudaMemcpyDeviceToHost, s), "download individuals"); }
-    BK(cudaMemcpyAsync(flags.data(), P.flags + g0, C, cudaMemcpyDeviceToHost, s), "download individuals");
-    BK(cudaMemcpyAsync(stat.data(), P.stat + g0, C, cudaMemcpyDeviceToHost, s), "download individuals");
-    BK(cudaStreamSynchronize(s), "synchronize");
+    const MemberDev& md = b->mdh[member];
+    const long long C = h.C, g0 = md.slot_off + (long long)sp * C;
     const pi_quota_params& p = h.sp[sp];
     const float cq_ns = (float)p.Cquota * (float)p.Nsuper;
-    // stored position k holds logical slot lslot[k]: the outputs are in logical order
-    std::vector<char> seen(C, 0);
-    for (long long k = 0; k < C; ++k) {
-        if (lslot[k] < 0 || lslot[k] >= C || seen[lslot[k]]) return bfail(b, PI_ERR_STATE, "pi_get_individuals: storage order corrupted");
-        seen[lslot[k]] = 1;
+    // the columns asked for, in k32_export's order
+    void* const cols[ECOL_AC] = { out->x, out->y, out->z, out->Sz, out->Bm, out->Cq, out->Nq, out->Pq, out->Chl, out->gen, out->age,
+                                  out->graz, out->mort, out->dvid, out->xi, out->yi, out->zi };
+    std::vector<char*> dst;
+    uint32_t mask = 0;
+    for (int q = 0; q < ECOL_AC; ++q)
+        if (cols[q]) { mask |= 1u << q; dst.push_back((char*)cols[q]); }
+    if (out->ac) mask |= 1u << ECOL_AC;
+    // The slots leave storage order on the device, a chunk at a time through one buffer (at most
+    // 2^19 slots, 72 MB): the host only receives columns. Reordering and converting 15 downloaded
+    // columns on one host thread took 17 ms for 2 × 200,000 slots.
+    if (!b->exp_buf) {
+        long long most = 1;
+        for (const auto& mb : b->mh) most = std::max(most, mb.C);
+        b->exp_slots = std::min<long long>(most, 1LL << 19);
+        cudaError_t er = cudaSuccess;
+        for (;; b->exp_slots = (b->exp_slots + 1) / 2) {
+            er = cudaMalloc(&b->exp_buf, (size_t)b->exp_slots * (8 * ECOL_AC + 1) + 8);
+            if (er != cudaErrorMemoryAllocation || b->exp_slots <= 1024) break;
+            cudaGetLastError();
+        }
+        if (er != cudaSuccess) { b->exp_buf = nullptr; return bcuda(b, er, "download individuals"); }
+        b->allocs.push_back(b->exp_buf);
     }
-    for (long long k = 0; k < C; ++k) {
-        const long long i = lslot[k];       // logical slot written from stored position k
-        const uint8_t fl = flags[k];
-        const int32_t code = cell[k];
-        int ci = 0, cj = 0, ck = 0;
-        const MemberDev& md = b->mdh[member];
-        if (code >= 0) f32_unpack(code, md.cbx, md.cby, ci, cj, ck);
-        const double xyz[3] = { code < 0 ? 0.0 : ci + (double)o[0][k], code < 0 ? 0.0 : cj + (double)o[1][k],
-                                code < 0 ? 0.0 : ck + (double)o[2][k] };
-        int64_t xi, yi, zi;
-        if (stat[k] & F32_ST_STALE) {
-            int a0, a1, a2;
-            f32_unpack(scell[k], md.hbx, md.hby, a0, a1, a2);
-            xi = a0; yi = a1; zi = a2;
-        } else if (code < 0) { xi = g.Hx; yi = g.Hy; zi = g.Hz; }
-        else { xi = ci + 1 + g.Hx; yi = cj + 1 + g.Hy; zi = ck + 1 + g.Hz; }
-        if (out->x) out->x[i] = xyz[0];
-        if (out->y) out->y[i] = xyz[1];
-        if (out->z) out->z[i] = xyz[2];
-        if (out->xi) out->xi[i] = xi;
-        if (out->yi) out->yi[i] = yi;
-        if (out->zi) out->zi[i] = zi;
-        double* cols[7] = { out->Bm, out->Cq, out->Nq, out->Pq, out->Chl, out->age, out->gen };
-        for (int q = 0; q < 7; ++q) if (cols[q]) cols[q][i] = (double)f[q][k];
-        if (out->Sz) out->Sz[i] = (double)(f[0][k] / cq_ns);
-        if (out->ac) out->ac[i] = (fl & F32_AC) ? 1 : 0;
-        if (out->graz) out->graz[i] = (fl & F32_GRAZ) ? 1.0 : 0.0;
-        if (out->mort) out->mort[i] = (fl & F32_MORT) ? 1.0 : 0.0;
-        if (out->dvid) out->dvid[i] = (fl & F32_DVID) ? 1.0 : 0.0;
+    cudaStream_t s = b->stream;
+    uint32_t* bad = (uint32_t*)b->scratch;
+    BK(cudaMemsetAsync(bad, 0, sizeof(uint32_t), s), "download individuals");
+    for (long long L0 = 0; L0 < C; L0 += b->exp_slots) {
+        const long long n = std::min(C - L0, b->exp_slots);
+        k32_export<<<nblk(n, 256), 256, 0, s>>>(b->P, md, g0, L0, n, mask, cq_ns, b->exp_buf, bad);
+        BK(cudaGetLastError(), "k32_export");
+        const char* src = (const char*)b->exp_buf;
+        for (size_t q = 0; q < dst.size();) {
+            // columns that follow one another in the caller's memory too are one copy (two page-locked
+            // allocations side by side are not: that copy is refused, and they are copied in turn)
+            size_t r = q + 1;
+            while (n == C && r < dst.size() && dst[r] == dst[r - 1] + C * 8) ++r;
+            if (r > q + 1 && cudaMemcpyAsync(dst[q], src + q * n * 8, (r - q) * n * 8, cudaMemcpyDeviceToHost, s) != cudaSuccess) {
+                cudaGetLastError();
+                r = q + 1;
+            }
+            if (r == q + 1)
+                BK(cudaMemcpyAsync(dst[q] + L0 * 8, src + q * n * 8, n * 8, cudaMemcpyDeviceToHost, s), "download individuals");
+            q = r;
+        }
+        if (out->ac) BK(cudaMemcpyAsync(out->ac + L0, src + dst.size() * n * 8, n, cudaMemcpyDeviceToHost, s), "download individuals");
     }
+    uint32_t hb = 0;
+    BK(cudaMemcpyAsync(&hb, bad, sizeof hb, cudaMemcpyDeviceToHost, s), "download individuals");
+    BK(cudaStreamSynchronize(s), "synchronize");
+    if (hb) return bfail(b, PI_ERR_STATE, "pi_get_individuals: storage order corrupted");
     return PI_OK;
 }
 

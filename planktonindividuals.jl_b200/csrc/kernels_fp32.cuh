@@ -2434,6 +2434,50 @@ __global__ void k32_sort_scatter(Tab32 T, IndDev32 P, IndDev32 Q, unsigned long 
     }
 }
 
+// Slots L0 .. L0 + n - 1 of one segment (logical order) as the boundary's columns: 8-byte columns of n
+// values one after another in `out` (bit q of mask: column q of ECOL_*; xi, yi, zi as int64), then ac
+// as bytes when bit ECOL_AC is set.
+enum { ECOL_X = 0, ECOL_Y, ECOL_Z, ECOL_SZ, ECOL_BM, ECOL_CQ, ECOL_NQ, ECOL_PQ, ECOL_CHL, ECOL_GEN, ECOL_AGE, ECOL_GRAZ,
+       ECOL_MORT, ECOL_DVID, ECOL_XI, ECOL_YI, ECOL_ZI, ECOL_AC };
+__global__ void __launch_bounds__(256) k32_export(IndDev32 P, MemberDev m, long long base, long long L0, long long n, uint32_t mask,
+                                                  float cq_ns, unsigned long long* __restrict__ out, uint32_t* __restrict__ bad) {
+    const long long t = (long long)blockIdx.x * 256 + threadIdx.x;
+    if (t >= n) return;
+    const long long L = L0 + t;
+    const int ph = P.phys[base + L];
+    if (ph < 0 || ph >= m.C || P.lslot[base + ph] != (int)L) { *bad = 1u; return; }
+    const long long g = base + ph;
+    const int32_t code = P.cell[g];
+    const uint8_t fl = P.flags[g];
+    int c[3] = { 0, 0, 0 };
+    if (code >= 0) unpack_int(m, code, c[0], c[1], c[2]);
+    long long at = 0;
+    auto put = [&](int q, double v) { if (mask >> q & 1u) { out[at * n + t] = (unsigned long long)__double_as_longlong(v); ++at; } };
+    const float off[3] = { P.ox[g], P.oy[g], P.oz[g] };
+    for (int a = 0; a < 3; ++a) put(ECOL_X + a, code < 0 ? 0.0 : c[a] + (double)off[a]);
+    const float Bm = P.Bm[g];
+    put(ECOL_SZ, (double)__fdiv_rn(Bm, cq_ns));
+    put(ECOL_BM, (double)Bm);
+    if (mask >> ECOL_CQ & 1u) put(ECOL_CQ, (double)P.Cq[g]);
+    if (mask >> ECOL_NQ & 1u) put(ECOL_NQ, (double)P.Nq[g]);
+    if (mask >> ECOL_PQ & 1u) put(ECOL_PQ, (double)P.Pq[g]);
+    if (mask >> ECOL_CHL & 1u) put(ECOL_CHL, (double)P.Chl[g]);
+    if (mask >> ECOL_GEN & 1u) put(ECOL_GEN, (double)P.gen[g]);
+    if (mask >> ECOL_AGE & 1u) put(ECOL_AGE, (double)P.age[g]);
+    put(ECOL_GRAZ, fl & F32_GRAZ ? 1.0 : 0.0);
+    put(ECOL_MORT, fl & F32_MORT ? 1.0 : 0.0);
+    put(ECOL_DVID, fl & F32_DVID ? 1.0 : 0.0);
+    if (mask >> ECOL_XI & 7u) {
+        const int H[3] = { m.Hx, m.Hy, m.Hz };
+        int x[3];
+        if (P.stat[g] & F32_ST_STALE) unpack_halo(m, P.scell[g], x[0], x[1], x[2]);
+        else for (int a = 0; a < 3; ++a) x[a] = code < 0 ? H[a] : c[a] + 1 + H[a];
+        for (int a = 0; a < 3; ++a)
+            if (mask >> (ECOL_XI + a) & 1u) { out[at * n + t] = (unsigned long long)x[a]; ++at; }
+    }
+    if (mask >> ECOL_AC & 1u) reinterpret_cast<uint8_t*>(out + at * n)[t] = fl & F32_AC ? 1 : 0;
+}
+
 // Storage order equal to the logical order over a slot range (after an upload): lslot and phys
 // are the identity, relative to the segment's first slot.
 __global__ void k32_identity_order(IndDev32 P, long long base, long long C) {
