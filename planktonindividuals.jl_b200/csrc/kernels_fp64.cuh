@@ -1247,7 +1247,25 @@ __global__ void k_halo_vel(DGrid g, double* __restrict__ c, int face_axis) {
     }
 }
 
-// Active individuals of one species (calc_active_individuals, models.jl:157-164).
+// Slots s0 .. s0 + n - 1 of the boundary's columns that are not stored as such: graz, mort and dvid as
+// Float64 and xi, yi and zi as int64 (bits 0-5 of mask), 8-byte columns of n one after another in
+// `out`, then ac as bytes (bit 6).
+__global__ void k64_export(DGrid g, SpcDev P, long long s0, long long n, uint32_t mask, unsigned long long* __restrict__ out) {
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n) return;
+    const uint8_t f = P.flags[s0 + t];
+    int x[3];
+    unpack_cell(g, P.cell[s0 + t], x[0], x[1], x[2]);
+    const uint8_t bits[3] = { FL_GRAZ, FL_MORT, FL_DVID };
+    long long at = 0;
+    for (int q = 0; q < 6; ++q) {
+        if (!(mask >> q & 1u)) continue;
+        out[at * n + t] = q < 3 ? (unsigned long long)__double_as_longlong(f & bits[q] ? 1.0 : 0.0) : (unsigned long long)x[q - 3];
+        ++at;
+    }
+    if (mask >> 6 & 1u) reinterpret_cast<uint8_t*>(out + at * n)[t] = f & FL_AC ? 1 : 0;
+}
+
 // Index of the first non-finite value of a[0, n) (atomicMin into *first, which starts at ~0).
 __global__ void k_first_nonfinite(const double* __restrict__ a, long long n, unsigned long long* first) {
     for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x)
@@ -1322,6 +1340,7 @@ __global__ void __launch_bounds__(256) k_budget_inds_macro(SpcDev s, long long C
     block_sum3(c, n, p, partial);
 }
 
+// Active individuals of one species (calc_active_individuals, models.jl:157-164).
 __global__ void k_count_active(const uint8_t* __restrict__ flags, long long C, unsigned long long* out) {
     unsigned long long n = 0;
     for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < C; q += (long long)gridDim.x * blockDim.x)

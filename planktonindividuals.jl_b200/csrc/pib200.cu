@@ -95,6 +95,8 @@ struct pi_model {
     double* diag_tr = nullptr;   // 14 × G
     double* diag_proc = nullptr; // nsp × PI_MAXPROC × G
     double* procv = nullptr;     // PI_MAXPROC × C values of the species being updated
+    unsigned long long* exp_buf = nullptr;   // columns of pi_get_individuals on their way to the host
+    long long exp_slots = 0;
     double* budget_part = nullptr;   // 3 × 512 block partials of pi_get_budget
     uint32_t *dkey = nullptr, *dkey_s = nullptr, *dval = nullptr, *dval_s = nullptr;
     void* dsort_tmp = nullptr;
@@ -1028,23 +1030,34 @@ pi_status pi_get_individuals(pi_model* m, int32_t sp, pi_individuals* out) {
         for (int q = 0; q < 6; ++q)
             if (mh[q]) CK(cudaMemcpyAsync(mh[q], md[q], C * sizeof(double), cudaMemcpyDeviceToHost, m->stream), "download individuals");
     }
-    std::vector<uint8_t> flags(C);
-    std::vector<int32_t> cell(C);
-    CK(cudaMemcpyAsync(flags.data(), P.flags, C, cudaMemcpyDeviceToHost, m->stream), "download flags");
-    CK(cudaMemcpyAsync(cell.data(), P.cell, C * sizeof(int32_t), cudaMemcpyDeviceToHost, m->stream), "download cells");
-    CK(cudaStreamSynchronize(m->stream), "synchronize");
-    for (long long i = 0; i < C; ++i) {
-        uint8_t f = flags[i];
-        if (out->ac) out->ac[i] = (f & FL_AC) ? 1 : 0;
-        if (out->graz) out->graz[i] = (f & FL_GRAZ) ? 1.0 : 0.0;
-        if (out->mort) out->mort[i] = (f & FL_MORT) ? 1.0 : 0.0;
-        if (out->dvid) out->dvid[i] = (f & FL_DVID) ? 1.0 : 0.0;
-        int xi, yi, zi;
-        unpack_cell(m->dg, cell[i], xi, yi, zi);
-        if (out->xi) out->xi[i] = xi;
-        if (out->yi) out->yi[i] = yi;
-        if (out->zi) out->zi[i] = zi;
+    // decisions, cells and ac are unpacked on the device, a chunk at a time through one buffer (at
+    // most 2^19 slots, 26 MB)
+    void* const cols[6] = { out->graz, out->mort, out->dvid, out->xi, out->yi, out->zi };
+    uint32_t mask = out->ac ? 64u : 0u;
+    for (int q = 0; q < 6; ++q) if (cols[q]) mask |= 1u << q;
+    if (mask && !m->exp_buf) {
+        cudaError_t er = cudaSuccess;
+        for (m->exp_slots = std::min<long long>(C, 1LL << 19);; m->exp_slots = (m->exp_slots + 1) / 2) {
+            er = cudaMalloc(&m->exp_buf, (size_t)m->exp_slots * 49 + 8);
+            if (er != cudaErrorMemoryAllocation || m->exp_slots <= 1024) break;
+            cudaGetLastError();
+        }
+        if (er != cudaSuccess) { m->exp_buf = nullptr; return cuda_fail(m, er, "download individuals"); }
+        m->allocs.push_back(m->exp_buf);
     }
+    for (long long s0 = 0; mask && s0 < C; s0 += m->exp_slots) {
+        const long long n = std::min(C - s0, m->exp_slots);
+        k64_export<<<nblk(n, 256), 256, 0, m->stream>>>(m->dg, P, s0, n, mask, m->exp_buf);
+        CK(cudaGetLastError(), "k64_export");
+        const char* src = (const char*)m->exp_buf;
+        for (int q = 0; q < 6; ++q) {
+            if (!cols[q]) continue;
+            CK(cudaMemcpyAsync((char*)cols[q] + s0 * 8, src, n * 8, cudaMemcpyDeviceToHost, m->stream), "download individuals");
+            src += n * 8;
+        }
+        if (out->ac) CK(cudaMemcpyAsync(out->ac + s0, src, n, cudaMemcpyDeviceToHost, m->stream), "download individuals");
+    }
+    CK(cudaStreamSynchronize(m->stream), "synchronize");
     return PI_OK;
 }
 
