@@ -20,7 +20,7 @@
 //                        forcing, particle terms, apply_tendency! and the halo fill in one walk
 //                        down the levels
 //   (otherwise, and in the first step after a tracer upload, these three:)
-//   k32_xy               DST3FL x and y sweeps of every tracer on level tiles in shared memory
+//   k32_xy               DST3FL x and y sweeps: a warp per tracer pair walks the rows of a level tile
 //   k32_ztail            z sweep walking columns, then diffusion, sinking, forcing, BCs, particle
 //                        terms and apply_tendency!
 //   k32_halo_direct (k32_halo_small, k32_halo<x,y,z>)  fill_halo_tracer!, then vel₀ ← vel₁,
@@ -426,7 +426,7 @@ pi_status build_tables(pi_batch* b) {
         const HostGrid& g = b->mh[m].g;
         for (int L = 1 + g.Hz; L <= g.Nz + g.Hz; ++L)
             for (int j0 = 1 + g.Hy; j0 <= g.Ny + g.Hy; j0 += ty)
-                for (int i0 = 1 + g.Hx; i0 <= g.Nx + g.Hx; i0 += 28) xy.push_back(make_int4(m, i0, j0, L));
+                for (int i0 = 1 + g.Hx; i0 <= g.Nx + g.Hx; i0 += 31) xy.push_back(make_int4(m, i0, j0, L));
         for (int k0 = 1 + g.Hz; k0 <= g.Nz + g.Hz; k0 += lz)
             for (int j = 1 + g.Hy; j <= g.Ny + g.Hy; ++j)
                 for (int i0 = 1 + g.Hx; i0 <= g.Nx + g.Hx; i0 += 32) zz.push_back(make_int4(m, i0, j, k0));
@@ -456,8 +456,6 @@ pi_status build_tables(pi_batch* b) {
     b->tables_ty = ty; b->tables_lz = lz; b->tables_lzf = lzf;
     return PI_OK;
 }
-
-size_t xy_smem(int ty) { return (size_t)(3 * ty + 5) * PI_NTRACERS * 32 * sizeof(float); }
 
 float* velown(pi_batch* b, int m, int buf, int c) { return b->velown + ((long long)(buf * 3 + c)) * b->Gtot + b->mdh[m].cell_off; }
 
@@ -502,19 +500,13 @@ pi_status enqueue_step(pi_batch* b, double dT, int cur) {
         TrArgs a = ta;
         a.items = b->xy_items; a.nitems = b->nxy_items;
         BScope sc(b, "k32_xy", st);
-        // persistent: as many blocks as fit at once, each looping over items with the next
-        // item's loads in flight
-        int per_sm = 1;
         const int ty = b->tune.ty;
-        if (ty == 28) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k32_xy<28>, 32 * 32, xy_smem(28));
-        else if (ty == 16) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k32_xy<16>, 32 * 20, xy_smem(16));
-        else if (ty == 8) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k32_xy<8>, 32 * 12, xy_smem(8));
-        else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k32_xy<4>, 32 * 8, xy_smem(4));
-        const unsigned grid = (unsigned)std::max(1, std::min(b->nxy_items, std::max(1, per_sm) * b->nsm));
-        if (ty == 28) k32_xy<28><<<grid, 32 * 32, xy_smem(28), st>>>(a);
-        else if (ty == 16) k32_xy<16><<<grid, 32 * 20, xy_smem(16), st>>>(a);
-        else if (ty == 8) k32_xy<8><<<grid, 32 * 12, xy_smem(8), st>>>(a);
-        else k32_xy<4><<<grid, 32 * 8, xy_smem(4), st>>>(a);
+        const unsigned grid = (unsigned)std::max(1, b->nxy_items);
+        const dim3 blk(32, TR_PAIRS);
+        if (ty == 28) k32_xy<28><<<grid, blk, xy_smem(28), st>>>(a);
+        else if (ty == 16) k32_xy<16><<<grid, blk, xy_smem(16), st>>>(a);
+        else if (ty == 8) k32_xy<8><<<grid, blk, xy_smem(8), st>>>(a);
+        else k32_xy<4><<<grid, blk, xy_smem(4), st>>>(a);
     };
     // beside the particle kernels when it leaves at least half of the SMs to them (measured per
     // step: 0D parcel 38.6 -> 34.3 µs, 128×128×1 gyre 49.9 -> 45.1, 64 parcels 93.6 -> 89.0; no gain
@@ -590,12 +582,15 @@ pi_status enqueue_step(pi_batch* b, double dT, int cur) {
             a.items = b->z_items; a.nitems = b->nz_items;
             BScope sc(b, "k32_ztail");
             const unsigned grid = (unsigned)std::max(1, b->nz_items);
-            const dim3 blk(32, PI_NTRACERS);
-            const size_t zs = ztail_smem(b->tune.lz);
-            if (b->tune.lz == 8) k32_ztail<8><<<grid, blk, zs, s>>>(a);
-            else if (b->tune.lz == 32) k32_ztail<32><<<grid, blk, zs, s>>>(a);
-            else if (b->tune.lz == 64) k32_ztail<64><<<grid, blk, zs, s>>>(a);
-            else k32_ztail<16><<<grid, blk, zs, s>>>(a);
+            const dim3 blk(32, TR_PAIRS);
+                        bool gen = false;               // a member has tracer diffusion or flux boundary conditions
+            for (int m = 0; m < b->nm; ++m)
+                gen = gen || b->mdh[m].any_bc || (float)b->mh[m].bgc.kappa_h != 0.0f || (float)b->mh[m].bgc.kappa_v != 0.0f;
+            const size_t zs = ztail_smem(b->tune.lz, gen);
+            if (b->tune.lz == 8) (gen ? k32_ztail<8, true> : k32_ztail<8, false>)<<<grid, blk, zs, s>>>(a);
+            else if (b->tune.lz == 32) (gen ? k32_ztail<32, true> : k32_ztail<32, false>)<<<grid, blk, zs, s>>>(a);
+            else if (b->tune.lz == 64) (gen ? k32_ztail<64, true> : k32_ztail<64, false>)<<<grid, blk, zs, s>>>(a);
+            else (gen ? k32_ztail<16, true> : k32_ztail<16, false>)<<<grid, blk, zs, s>>>(a);
         }
         }
     }
@@ -973,10 +968,14 @@ pi_status pi_batch_create(const pi_member* members, int32_t nmembers, int32_t ns
     cudaFuncSetAttribute(k32_xy<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)xy_smem(16));
     cudaFuncSetAttribute(k32_xy<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)xy_smem(8));
     cudaFuncSetAttribute(k32_xy<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)xy_smem(4));
-    cudaFuncSetAttribute(k32_ztail<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ztail_smem(8));
-    cudaFuncSetAttribute(k32_ztail<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ztail_smem(16));
-    cudaFuncSetAttribute(k32_ztail<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ztail_smem(32));
-    cudaFuncSetAttribute(k32_ztail<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ztail_smem(64));
+    cudaFuncSetAttribute(k32_ztail<8, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ztail_smem(8, false));
+    cudaFuncSetAttribute(k32_ztail<8, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ztail_smem(8, true));
+    cudaFuncSetAttribute(k32_ztail<16, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ztail_smem(16, false));
+    cudaFuncSetAttribute(k32_ztail<16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ztail_smem(16, true));
+    cudaFuncSetAttribute(k32_ztail<32, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ztail_smem(32, false));
+    cudaFuncSetAttribute(k32_ztail<32, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ztail_smem(32, true));
+    cudaFuncSetAttribute(k32_ztail<64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ztail_smem(64, false));
+    cudaFuncSetAttribute(k32_ztail<64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ztail_smem(64, true));
     cudaFuncSetAttribute(k32_tracer, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tracer_smem_bytes());
     st = build_tensor_maps(b);
     if (st) return bail(st);

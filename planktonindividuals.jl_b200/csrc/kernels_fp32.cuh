@@ -1340,9 +1340,15 @@ __device__ __forceinline__ FCu fcu(float vel, float area, float rdxc, float dT) 
     f.R = __fdividef(__fsub_rn(1.0f, cfl), __fadd_rn(cfl, EPS20_F));
     return f;
 }
+// max(0, min(|d|, a, b)) with the sign of d on d, a and b: the two cases of δ⁰ in one, five or six
+// operations instead of eight
+__device__ __forceinline__ float limited(float d, float a, float b) {
+    const unsigned sg = __float_as_uint(d) & 0x80000000u;
+    const float as = __uint_as_float(__float_as_uint(a) ^ sg), bs = __uint_as_float(__float_as_uint(b) ^ sg);
+    return __uint_as_float(__float_as_uint(fmaxf(0.0f, fminf(fminf(fabsf(d), as), bs))) | sg);
+}
 __device__ __forceinline__ float psid0(float d0, float dn, const FCu& f) {
-    const float a = __fmaf_rn(f.d0c, d0, __fmul_rn(f.d1c, dn)), b = __fmul_rn(f.R, dn);
-    return d0 >= 0.0f ? fmaxf(0.0f, fminf(fminf(d0, a), b)) : fminf(0.0f, fmaxf(fmaxf(d0, a), b));
+    return limited(d0, __fmaf_rn(f.d0c, d0, __fmul_rn(f.d1c, dn)), __fmul_rn(f.R, dn));
 }
 // one sweep's update v − dtv·(ΔF − c·ftr) (multi_dim_adv.jl:111-135)
 __device__ __forceinline__ float upd_sweep(float v, float dtv, float dF, float c, float ftr) {
@@ -1408,8 +1414,8 @@ __device__ __forceinline__ float getbc32(const FluxBC32& b, int a, int c, int64_
 
 // Pairs of FP32 values — the same cell of tracers 2p and 2p+1 — in one 64-bit register, for the
 // packed FP32 instructions of sm_100 (add/sub/mul/fma .rn.f32x2). Each half is rounded exactly as the
-// scalar __fadd_rn, __fsub_rn, __fmul_rn and __fmaf_rn, so the packed x-y tile gives the same bits
-// as xy_tile while issuing one instruction for two tracers.
+// scalar __fadd_rn, __fsub_rn, __fmul_rn and __fmaf_rn, so the kernels that use them give the same bits
+// as k32_tracer's scalar formulas with one instruction for two tracers.
 typedef unsigned long long fx2;
 __device__ __forceinline__ fx2 fx2_of(float lo, float hi) {
     fx2 r;
@@ -1427,33 +1433,27 @@ __device__ __forceinline__ fx2 fx2_fma(fx2 a, fx2 b, fx2 c) {
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
     return d;
 }
-__device__ __forceinline__ fx2 fx2_neg(fx2 a) { return a ^ 0x8000000080000000ull; }   // exact sign flips
 
 // the face coefficients of one face for both halves
-struct FCu2 { fx2 tr, d0c, d1c, R; bool pos; };
-__device__ __forceinline__ FCu2 fcu2(const FCu& f) {
-    FCu2 g;
-    g.tr = fx2_of(f.tr, f.tr); g.d0c = fx2_of(f.d0c, f.d0c); g.d1c = fx2_of(f.d1c, f.d1c); g.R = fx2_of(f.R, f.R);
-    g.pos = f.tr > 0.0f;
-    return g;
+struct FCu2 { fx2 tr, d0c, d1c, R; };
+// adv_flux at a face for two tracers from the upwind cell B, the cell A behind it and the downwind cell
+// C: flux_h and flux_v select their operands by the sign of the transport; here the caller has, and as
+// the limiter is odd, both signs are the one formula tr·(B + ψ). mAB, mBC: landmask products of the
+// two differences as AND masks (δ·mask = copysign(0, δ) on land), all ones for water.
+__device__ __forceinline__ fx2 flux3(const FCu2& f, fx2 A, fx2 B, fx2 C, bool lm, unsigned mAB, unsigned mBC) {
+    fx2 d = fx2_sub(C, B), dn = fx2_sub(B, A);
+    if (lm) {
+        d &= ((fx2)mBC << 32) | mBC;
+        dn &= ((fx2)mAB << 32) | mAB;
+    }
+    const fx2 a = fx2_fma(f.d0c, d, fx2_mul(f.d1c, dn)), b = fx2_mul(f.R, dn);
+    float dl, dh, al, ah, bl, bh;
+    fx2_split(d, dl, dh); fx2_split(a, al, ah); fx2_split(b, bl, bh);
+    return fx2_mul(f.tr, fx2_add(B, fx2_of(limited(dl, al, bl), limited(dh, ah, bh))));
 }
-// flux_h of an all-water face for two tracers: the upwind operands are selected first (the
-// selected difference and the sum c0 − ψ = c0 + (−ψ) are the same IEEE operations), the limiter
-// (min/max, no packed form) runs per half
-__device__ __forceinline__ fx2 flux_h2(const FCu2& f, fx2 cm2, fx2 cm1, fx2 c0, fx2 cp1) {
-    const fx2 d0 = fx2_sub(c0, cm1);
-    const fx2 dn = f.pos ? fx2_sub(cm1, cm2) : fx2_sub(cp1, c0);
-    const fx2 a = fx2_fma(f.d0c, d0, fx2_mul(f.d1c, dn)), b = fx2_mul(f.R, dn);
-    float d0l, d0h, al, ah, bl, bh;
-    fx2_split(d0, d0l, d0h); fx2_split(a, al, ah); fx2_split(b, bl, bh);
-    const float pl = d0l >= 0.0f ? fmaxf(0.0f, fminf(fminf(d0l, al), bl)) : fminf(0.0f, fmaxf(fmaxf(d0l, al), bl));
-    const float ph = d0h >= 0.0f ? fmaxf(0.0f, fminf(fminf(d0h, ah), bh)) : fminf(0.0f, fmaxf(fmaxf(d0h, ah), bh));
-    const fx2 ps = fx2_of(pl, ph);
-    return fx2_mul(f.tr, f.pos ? fx2_add(cm1, ps) : fx2_add(c0, fx2_neg(ps)));
-}
-// upd_sweep for two tracers: v − dtv·(ΔF − c·ftr)
-__device__ __forceinline__ fx2 upd_sweep2(fx2 v, fx2 ndtv, fx2 dF, fx2 c, fx2 ftr) {
-    return fx2_fma(ndtv, fx2_fma(fx2_neg(c), ftr, dF), v);
+// upd_sweep for two tracers: v − dtv·(ΔF − c·ftr), with −dtv and −ftr given
+__device__ __forceinline__ fx2 upd_sweep2(fx2 v, fx2 ndtv, fx2 dF, fx2 c, fx2 nftr) {
+    return fx2_fma(ndtv, fx2_fma(c, nftr, dF), v);
 }
 
 struct TrArgs {
@@ -1478,241 +1478,225 @@ struct TrArgs {
     const uint32_t* err;
 };
 
-// x and y sweeps of all 14 tracers on one level of a tile of 28 columns × TY rows. Warp w holds
-// row j0-2+w (TY+4 rows: the y sweep reads two rows on each side, outside the domain through the
-// halo-fill map), lane l column i0-2+l (28 cells and two halo columns on each side, exchanged by
-// shuffles). The face coefficients are computed once per face and shared by the 14 tracers.
-// Shared memory [row][tracer][lane]: TA (after x), FY (y face fluxes), TRs (tracer of the rows
-// the y sweep updates).
-// The inputs of one item for this thread (its row and column): u and the 14 tracers of the x
-// sweep, and the y velocities it reads later — v at its y face j0 + wid (x) and at the two faces
-// of its row (y, z; in range whenever the row is updated). A block loops over items and loads the
-// next item's inputs while it works on the current one.
-__device__ __forceinline__ void xy_load(const TrArgs& a, int item, float& u, float* v, float3& vy) {
-    const int4 it = a.items[item];
-    const MemberDev& m = a.T.md[it.x];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int jj = wrap_ax(it.z - 2 + wid, m.Ny, m.Hy, m.ty);
-    const int ic = min(it.y - 2 + lane, m.Gx);
-    const int q = gid3(m, ic, jj, it.w);
-    const MemberForcing& F = a.F[it.x];
-    u = F.vel1[0][q];
-    const float* __restrict__ src = a.tr + m.cell_off + q;
-#pragma unroll
-    for (int n = 0; n < PI_NTRACERS; ++n) v[n] = src[n * a.Gtot];
-    const int f = it.z + wid;
-    const int fs = f == m.Ny + m.Hy + 1 ? m.Hy + 1 : min(f, m.Ny + m.Hy);
-    const int jr = min(f, m.Gy - 1);
-    const float* __restrict__ vv = F.vel1[1];
-    vy.x = vv[gid3(m, ic, fs, it.w)];
-    const int qr = gid3(m, ic, jr, it.w);
-    vy.y = vv[qr];
-    vy.z = vv[qr + m.Gx];
+// The coefficients of a face as the walking kernels keep them in shared memory, doubled on their way to
+// the packed instructions: the copies would halve the accesses' moves, but take shared memory that is
+// then missing as L1 (see k32_ztail).
+__device__ __forceinline__ FCu2 get_fcu(const float4* s, int e, bool& pos) {
+    const float4 a = s[e];
+    pos = a.x > 0.0f;
+    FCu2 f;
+    f.tr = fx2_of(a.x, a.x); f.d0c = fx2_of(a.y, a.y); f.d1c = fx2_of(a.z, a.z); f.R = fx2_of(a.w, a.w);
+    return f;
+}
+// Mask byte of a face and of the cell after it: water on both sides of B-C and of A-B (by the sign of the
+// transport), no flux through the face, water in the cell and beyond its far face, and that sign
+#define MB_BC 1u
+#define MB_AB 2u
+#define MB_ZERO 4u
+#define MB_CELL 8u
+#define MB_POS 16u                    // the transport is positive
+__device__ __forceinline__ unsigned mask_byte(float tr, int lm2, int lm1, int l0, int lp1) {
+    return (l0 & lm1 ? MB_BC : 0u) | ((tr > 0.0f ? lm1 & lm2 : lp1 & l0) ? MB_AB : 0u);
+}
+__device__ __forceinline__ unsigned and_mask(unsigned mb, unsigned bit) { return mb & bit ? 0xffffffffu : 0x80000000u; }
+__device__ __forceinline__ fx2 fx2_and(fx2 v, unsigned m) { return v & (((fx2)m << 32) | m); }
+__device__ __forceinline__ fx2 cell_mask(fx2 v, unsigned mb) { return fx2_and(v, and_mask(mb, MB_CELL)); }
+// The two tracers of a pair: nutrients in the first five pairs, the iron tracers and dust in the last two
+__host__ __device__ constexpr int pair_tracer(int p, int h) {
+    return p == 0 ? (h ? PI_NH4 : PI_DIC) : p == 1 ? (h ? PI_PO4 : PI_NO3) : p == 2 ? (h ? PI_DON : PI_DOC)
+         : p == 3 ? (h ? PI_POC : PI_DOP) : p == 4 ? (h ? PI_POP : PI_PON) : p == 5 ? (h ? PI_PFe_inorg : PI_DFe)
+         : (h ? PI_Dust : PI_PFe_bio);
+}
+#define TR_PAIRS (PI_NTRACERS / 2)
+// threadIdx.y as a value the compiler knows to be the same for the warp, so that what follows from it (the
+// bases of the pair's arrays) can stay in uniform registers
+__device__ __forceinline__ int warp_row() { return __shfl_sync(0xffffffffu, (int)threadIdx.y, 0); }
+// element at a byte offset below 4 GB from a uniform base (a member's field: 14 of them, twice, and the
+// particle sums would not fit the memory beyond that), which needs no 64-bit address arithmetic per access
+__device__ __forceinline__ float ldg_at(const float* base, unsigned byte) {
+    return __ldg(reinterpret_cast<const float*>(reinterpret_cast<const char*>(base) + byte));
+}
+__device__ __forceinline__ void st_at(float* base, unsigned byte, float v) {
+    *reinterpret_cast<float*>(reinterpret_cast<char*>(base) + byte) = v;
 }
 
-template <int TY, bool LM>
-__device__ __forceinline__ void xy_tile(const TrArgs& a, const MemberDev& m, const int4 it, float* sm,
-                                        float& pu, float* pv, float3& pvy, int next) {
-    float* TA = sm;                                        // (TY+4) × 14 × 32
-    float* FY = TA + (TY + 4) * PI_NTRACERS * 32;          // (TY+1) × 14 × 32
-    float* TRs = FY + (TY + 1) * PI_NTRACERS * 32;         // TY × 14 × 32
-    auto at = [](float* base, int r, int n, int l) -> float& { return base[(r * PI_NTRACERS + n) * 32 + l]; };
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const long long G = a.Gtot;
-    const float dT = a.dT;
-    const int i0 = it.y, j0 = it.z, L = it.w;
-    const long long off = m.cell_off;
-    const float dz = a.dzF[m.dz_off + L - 1];
-    const float az = __fmul_rn(m.dx, m.dy), dtv = __fdiv_rn(dT, __fmul_rn(az, dz));
-    // ---- x sweep of row j0-2+wid
-    {
-        const int jj = wrap_ax(j0 - 2 + wid, m.Ny, m.Hy, m.ty);
-        const int i = i0 - 2 + lane;
-        const int ic = min(i, m.Gx);
-        const float ax = __fmul_rn(m.dy, dz);
-        const float uw = pu;
-        const float ue = __shfl_down_sync(0xffffffffu, uw, 1);
-        const FCu fc = fcu(uw, ax, __frcp_rn(m.dx), dT);
-        int l0 = 1, lm1 = 1, lm2 = 1, lp1 = 1;
-        if (LM) {
-            l0 = lm32(m, a.lm, ic, jj, L);
-            lm1 = __shfl_up_sync(0xffffffffu, l0, 1); lm2 = __shfl_up_sync(0xffffffffu, l0, 2);
-            lp1 = __shfl_down_sync(0xffffffffu, l0, 1);
-        }
-        const bool east_zero = i == m.Nx + m.Hx && m.tx != PI_PERIODIC;   // fill_halo_east_Gc! (Bounded)
-        const float ftr = mk<LM>(tdiff(ax, ue, uw), lp1, l0);
-        const bool store_tr = wid >= 2 && wid < TY + 2;
-#pragma unroll
-        for (int n = 0; n < PI_NTRACERS; ++n) {
-            const float v = pv[n];
-            const float cm2 = __shfl_up_sync(0xffffffffu, v, 2), cm1 = __shfl_up_sync(0xffffffffu, v, 1);
-            const float cp1 = __shfl_down_sync(0xffffffffu, v, 1);
-            const float Fw = flux_h<LM>(fc, cm2, cm1, v, cp1, lm2, lm1, l0, lp1);
-            float Fe = __shfl_down_sync(0xffffffffu, Fw, 1);
-            if (east_zero) Fe = 0.0f;
-            at(TA, wid, n, lane) = upd_sweep(v, dtv, mk<LM>(__fsub_rn(Fe, Fw), lp1, l0), v, ftr);
-            if (store_tr) at(TRs, wid - 2, n, lane) = v;
-        }
-    }
-    __syncthreads();
-    // the registers of this item's x inputs are free: start the next item's loads
-    const float3 vy = pvy;
-    if (next < a.nitems) xy_load(a, next, pu, pv, pvy);
-    // ---- y faces j0 + r, r = 0..TY
-    const int i = i0 - 2 + lane;
-    const bool col = lane >= 2 && lane < 30 && i <= m.Nx + m.Hx;
-    const float ay = __fmul_rn(m.dx, dz);
-    if (wid <= TY) {
-        const int r = wid, f = j0 + r;
-        const bool special = f == m.Ny + m.Hy + 1;
-        const bool zero = !col || f > m.Ny + m.Hy + 1 || (special && m.ty != PI_PERIODIC);
-        const int fs = special ? m.Hy + 1 : min(f, m.Ny + m.Hy);
-        const int ic = min(i, m.Gx);
-        const FCu fc = fcu(zero ? 0.0f : vy.x, ay, __frcp_rn(m.dy), dT);
-        int L2 = 1, L1 = 1, L0 = 1, Lp = 1;
-        if (LM) {
-            L2 = lm32(m, a.lm, ic, fs - 2, L); L1 = lm32(m, a.lm, ic, fs - 1, L);
-            L0 = lm32(m, a.lm, ic, fs, L); Lp = lm32(m, a.lm, ic, fs + 1, L);
-        }
-#pragma unroll
-        for (int n = 0; n < PI_NTRACERS; ++n)
-            at(FY, r, n, lane) = zero ? 0.0f : flux_h<LM>(fc, at(TA, r, n, lane), at(TA, r + 1, n, lane), at(TA, r + 2, n, lane),
-                                                          at(TA, r + 3, n, lane), L2, L1, L0, Lp);
-    }
-    __syncthreads();
-    // ---- y update of row j0 + wid
-    if (wid < TY) {
-        const int j = j0 + wid;
-        if (col && j <= m.Ny + m.Hy) {
-            const int q = gid3(m, i, j, L);
-            const int c0m = LM ? lm32(m, a.lm, i, j, L) : 1, cpm = LM ? lm32(m, a.lm, i, j + 1, L) : 1;
-            const float ftr = mk<LM>(tdiff(ay, vy.z, vy.y), cpm, c0m);
-            float* dst = a.tb + off + q;
-#pragma unroll
-            for (int n = 0; n < PI_NTRACERS; ++n) {
-                const float dG = mk<LM>(__fsub_rn(at(FY, wid + 1, n, lane), at(FY, wid, n, lane)), cpm, c0m);
-                dst[n * G] = upd_sweep(at(TA, wid + 2, n, lane), dtv, dG, at(TRs, wid, n, lane), ftr);
-            }
-        }
-    }
-    __syncthreads();
+// x and y sweeps on one level of 31 columns (32 x faces, one per lane) × TY rows: warp p of the block walks
+// the rows of tracer pair p from two above to two below (outside the domain through the halo-fill
+// map). Each row's x sweep gives the tracer_temp row that the y sweep keeps in a window of four
+// registers; a y face's flux is formed once and serves the rows on both sides, so nothing but the
+// face coefficients, formed once for the 14 tracers, goes through shared memory. The x sweep loads a
+// face's three cells in upwind order (no selects), two rows ahead. What bounds it is the latency of
+// those loads and of the limiter's chain, so warps count more than registers: on 256×256×64 309 µs with
+// two pairs per warp (16 warps per SM), 256 µs with one (28 warps), 231 µs at five blocks (35 warps, 56
+// registers); 326 µs when every tile staged its rows, fluxes and intermediate rows in shared memory.
+// Rows per tile (the walk costs TY + 4): at four blocks 363 µs with 8, 256 with 16, 245 with 28, which in
+// turn leaves small models short of blocks (96×80×24: 15.8 µs with 16, 19.5 with 28).
+struct XYRows { float4 *fx, *fy; float *tx, *ty; int* row; uint8_t *mx, *my; };
+__host__ __device__ inline size_t xy_smem(int ty) {
+    return (size_t)(2 * ty + 5) * 32 * (sizeof(float4) + sizeof(float) + 1) + (size_t)(ty + 4) * sizeof(int);
 }
-
-// xy_tile for an all-water member with the 14 tracers handled as 7 packed pairs: the same tile,
-// threads and operations, with shared memory laid out [row][pair][lane] of 64-bit pairs so that a
-// lane reads or writes both tracers of a pair with one access.
-template <int TY>
-__device__ __forceinline__ void xy_tile_pk(const TrArgs& a, const MemberDev& m, const int4 it, float* sm,
-                                           float& pu, float* pv, float3& pvy, int next) {
-    constexpr int NP = PI_NTRACERS / 2;
-    fx2* TA = reinterpret_cast<fx2*>(sm);                 // (TY+4) × 7 × 32
-    fx2* FY = TA + (TY + 4) * NP * 32;                     // (TY+1) × 7 × 32
-    fx2* TRs = FY + (TY + 1) * NP * 32;                    // TY × 7 × 32
-    auto at = [](fx2* base, int r, int p, int l) -> fx2& { return base[(r * NP + p) * 32 + l]; };
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const long long G = a.Gtot;
-    const float dT = a.dT;
-    const int i0 = it.y, j0 = it.z, L = it.w;
-    const long long off = m.cell_off;
+template <bool LM>
+__device__ __forceinline__ void xy_walk(const TrArgs& a, const MemberDev& m, const int4 it, const XYRows& S, int nr, int p) {
+    const int lane = threadIdx.x;
+    const int i0 = it.y, L = it.w, lastx = m.Nx + m.Hx;
     const float dz = a.dzF[m.dz_off + L - 1];
-    const float az = __fmul_rn(m.dx, m.dy), dtv = __fdiv_rn(dT, __fmul_rn(az, dz));
+    const float az = __fmul_rn(m.dx, m.dy), dtv = __fdiv_rn(a.dT, __fmul_rn(az, dz));
     const fx2 ndtv = fx2_of(-dtv, -dtv);
-    // ---- x sweep of row j0-2+wid
-    {
-        const int i = i0 - 2 + lane;
-        const float ax = __fmul_rn(m.dy, dz);
-        const float uw = pu;
-        const float ue = __shfl_down_sync(0xffffffffu, uw, 1);
-        const FCu2 fc = fcu2(fcu(uw, ax, __frcp_rn(m.dx), dT));
-        const bool east_zero = i == m.Nx + m.Hx && m.tx != PI_PERIODIC;   // fill_halo_east_Gc! (Bounded)
-        const float ftr1 = tdiff(ax, ue, uw);
-        const fx2 ftr = fx2_of(ftr1, ftr1);
-        const bool store_tr = wid >= 2 && wid < TY + 2;
-#pragma unroll
-        for (int p = 0; p < NP; ++p) {
-            const float v0 = pv[2 * p], v1 = pv[2 * p + 1];
-            const fx2 v = fx2_of(v0, v1);
-            const fx2 cm2 = fx2_of(__shfl_up_sync(0xffffffffu, v0, 2), __shfl_up_sync(0xffffffffu, v1, 2));
-            const fx2 cm1 = fx2_of(__shfl_up_sync(0xffffffffu, v0, 1), __shfl_up_sync(0xffffffffu, v1, 1));
-            const fx2 cp1 = fx2_of(__shfl_down_sync(0xffffffffu, v0, 1), __shfl_down_sync(0xffffffffu, v1, 1));
-            const fx2 Fw = flux_h2(fc, cm2, cm1, v, cp1);
-            float wl, wh;
-            fx2_split(Fw, wl, wh);
-            fx2 Fe = fx2_of(__shfl_down_sync(0xffffffffu, wl, 1), __shfl_down_sync(0xffffffffu, wh, 1));
-            if (east_zero) Fe = 0ull;
-            at(TA, wid, p, lane) = upd_sweep2(v, ndtv, fx2_sub(Fe, Fw), v, ftr);
-            if (store_tr) at(TRs, wid - 2, p, lane) = v;
+    const int f = i0 + lane;
+    const bool cell = lane < 31 && f <= lastx;
+    const bool nox = f == lastx + 1 && m.tx != PI_PERIODIC;            // fill_halo_east_Gc! (Bounded)
+    const unsigned fx4 = 4u * (unsigned)(min(f, lastx + 1) - 1);       // byte offset of the face's cell in a row
+    const long long oa = pair_tracer(p, 0) * a.Gtot + m.cell_off, ob = pair_tracer(p, 1) * a.Gtot + m.cell_off;
+    const float *ca = a.tr + oa, *cb = a.tr + ob;
+    float *ta = a.tb + oa, *tb = a.tb + ob;
+    // a row's cells in upwind order: behind, upwind and downwind of the face; two rows ahead of the sweep
+    struct In { float a[2], b[2], c[2]; };
+    In I0, I1;
+    auto load = [&](In& I, int r) {
+        if (r >= nr + 4) return;
+        const bool pos = S.mx[r * 32 + lane] & MB_POS;
+        const unsigned qb = 4u * (unsigned)S.row[r] + fx4 - (pos ? 4u : 0u), st = pos ? 0u - 4u : 4u;
+        I.a[0] = ldg_at(ca, qb + st); I.a[1] = ldg_at(cb, qb + st);
+        I.b[0] = ldg_at(ca, qb); I.b[1] = ldg_at(cb, qb);
+        I.c[0] = ldg_at(ca, qb - st); I.c[1] = ldg_at(cb, qb - st);
+    };
+    fx2 T0 = 0ull, T1 = 0ull, T2 = 0ull, T3 = 0ull, g0 = 0ull, g1 = 0ull, g2 = 0ull, Fy = 0ull;
+    auto row = [&](In& I, int r, bool face, bool store) {
+        const int ex = r * 32 + lane;
+        bool pos;
+        const FCu2 fc = get_fcu(S.fx, ex, pos);
+        const float tx = S.tx[ex];
+        const unsigned mx = LM ? S.mx[ex] : 0u;
+        const fx2 A = fx2_of(I.a[0], I.a[1]), B = fx2_of(I.b[0], I.b[1]), C = fx2_of(I.c[0], I.c[1]);
+        load(I, r + 2);
+        fx2 F = flux3(fc, A, B, C, LM, and_mask(mx, MB_AB), and_mask(mx, MB_BC));
+        if (nox) F = 0ull;
+        T0 = T1; T1 = T2; T2 = T3;
+        g0 = g1; g1 = g2; g2 = pos ? C : B;
+        float Fl, Fh;
+        fx2_split(F, Fl, Fh);
+        fx2 dF = fx2_sub(fx2_of(__shfl_down_sync(0xffffffffu, Fl, 1), __shfl_down_sync(0xffffffffu, Fh, 1)), F);
+        if (LM) dF = cell_mask(dF, mx);
+        T3 = upd_sweep2(g2, ndtv, dF, g2, fx2_of(tx, tx));
+        if (!face) return;
+        // y face j0 + r - 3 from rows r - 3 .. r, and the row between it and the face before
+        const int ey = ex - 3 * 32;
+        const FCu2 fy = get_fcu(S.fy, ey, pos);
+        const unsigned my = S.my[ey];
+        fx2 Fn = flux3(fy, pos ? T0 : T3, pos ? T1 : T2, pos ? T2 : T1, LM, and_mask(my, MB_AB), and_mask(my, MB_BC));
+        if (my & MB_ZERO) Fn = 0ull;
+        if (store && cell) {
+            // row j0 + r - 4 is row r - 2 of the walk: window entry 1, its original tracer g0
+            const float ty = S.ty[ey - 32];
+            fx2 dG = fx2_sub(Fn, Fy);
+            if (LM) dG = cell_mask(dG, S.my[ey - 32]);
+            const unsigned q = 4u * (unsigned)S.row[r - 2] + fx4;
+            float lo, hi;
+            fx2_split(upd_sweep2(T1, ndtv, dG, g0, fx2_of(ty, ty)), lo, hi);
+            st_at(ta, q, lo);
+            st_at(tb, q, hi);
         }
+        Fy = Fn;
+    };
+    load(I0, 0);
+    load(I1, 1);
+    row(I0, 0, false, false);
+    row(I1, 1, false, false);
+    row(I0, 2, false, false);
+    row(I1, 3, true, false);
+    int r = 4;
+#pragma unroll 2
+    for (; r + 1 < nr + 4; r += 2) {
+        row(I0, r, true, true);
+        row(I1, r + 1, true, true);
     }
-    __syncthreads();
-    // the registers of this item's x inputs are free: start the next item's loads
-    const float3 vy = pvy;
-    if (next < a.nitems) xy_load(a, next, pu, pv, pvy);
-    // ---- y faces j0 + r, r = 0..TY
-    const int i = i0 - 2 + lane;
-    const bool col = lane >= 2 && lane < 30 && i <= m.Nx + m.Hx;
-    const float ay = __fmul_rn(m.dx, dz);
-    if (wid <= TY) {
-        const int r = wid, f = j0 + r;
-        const bool special = f == m.Ny + m.Hy + 1;
-        const bool zero = !col || f > m.Ny + m.Hy + 1 || (special && m.ty != PI_PERIODIC);
-        const FCu2 fc = fcu2(fcu(zero ? 0.0f : vy.x, ay, __frcp_rn(m.dy), dT));
-#pragma unroll
-        for (int p = 0; p < NP; ++p)
-            at(FY, r, p, lane) = zero ? 0ull : flux_h2(fc, at(TA, r, p, lane), at(TA, r + 1, p, lane), at(TA, r + 2, p, lane),
-                                                      at(TA, r + 3, p, lane));
-    }
-    __syncthreads();
-    // ---- y update of row j0 + wid
-    if (wid < TY) {
-        const int j = j0 + wid;
-        if (col && j <= m.Ny + m.Hy) {
-            const int q = gid3(m, i, j, L);
-            const float ftr1 = tdiff(ay, vy.z, vy.y);
-            const fx2 ftr = fx2_of(ftr1, ftr1);
-            float* dst = a.tb + off + q;
-#pragma unroll
-            for (int p = 0; p < NP; ++p) {
-                const fx2 dG = fx2_sub(at(FY, wid + 1, p, lane), at(FY, wid, p, lane));
-                float lo, hi;
-                fx2_split(upd_sweep2(at(TA, wid + 2, p, lane), ndtv, dG, at(TRs, wid, p, lane), ftr), lo, hi);
-                dst[(2 * p) * G] = lo;
-                dst[(2 * p + 1) * G] = hi;
-            }
-        }
-    }
-    __syncthreads();
+    if (r < nr + 4) row(I0, r, true, true);
 }
 
 template <int TY>
-__global__ void __launch_bounds__(32 * (TY + 4)) k32_xy(TrArgs a) {
+__global__ void __launch_bounds__(32 * TR_PAIRS, 5) k32_xy(TrArgs a) {
     if (stopped(a.err)) return;
-    extern __shared__ float sm[];
-    if ((int)blockIdx.x >= a.nitems) return;
-    float pu, pv[PI_NTRACERS];
-    float3 pvy;
-    xy_load(a, blockIdx.x, pu, pv, pvy);
-    for (int item = blockIdx.x; item < a.nitems; item += gridDim.x) {
-        const int4 it = a.items[item];
-        const MemberDev& m = a.T.md[it.x];
-        const int next = item + gridDim.x;
-        if (m.all_water) xy_tile_pk<TY>(a, m, it, sm, pu, pv, pvy, next);
-        else xy_tile<TY, true>(a, m, it, sm, pu, pv, pvy, next);
+    extern __shared__ __align__(16) unsigned char xsm[];
+    const int4 it = a.items[blockIdx.x];
+    const MemberDev& m = a.T.md[it.x];
+    XYRows S;
+    S.fx = reinterpret_cast<float4*>(xsm);
+    S.fy = S.fx + (TY + 4) * 32;
+    S.tx = reinterpret_cast<float*>(S.fy + (TY + 1) * 32);
+    S.ty = S.tx + (TY + 4) * 32;
+    S.row = reinterpret_cast<int*>(S.ty + (TY + 1) * 32);
+    S.mx = reinterpret_cast<uint8_t*>(S.row + TY + 4);
+    S.my = S.mx + (TY + 4) * 32;
+    const int lane = threadIdx.x, i0 = it.y, j0 = it.z, L = it.w, lastx = m.Nx + m.Hx, lasty = m.Ny + m.Hy;
+    const int nr = min(TY, lasty - j0 + 1);
+    const MemberForcing& F = a.F[it.x];
+    const float *uu = F.vel1[0], *vv = F.vel1[1];
+    const float dz = a.dzF[m.dz_off + L - 1], ax = __fmul_rn(m.dy, dz), ay = __fmul_rn(m.dx, dz);
+    const float rdx = __frcp_rn(m.dx), rdy = __frcp_rn(m.dy);
+    const bool land = !m.all_water;
+    const int f = i0 + lane, fi = min(f, lastx + 1);             // lanes past the last face repeat it
+    // (the velocities are loaded through the read-only path, so that several rows' loads are in flight)
+#pragma unroll 5
+    for (int r = threadIdx.y; r < nr + 4; r += TR_PAIRS) {
+        const int e = r * 32 + lane, j = wrap_ax(j0 - 2 + r, m.Ny, m.Hy, m.ty);
+        const int q = gid3(m, fi, j, L);
+        const float uw = __ldg(uu + q), ue = __ldg(uu + q + 1);
+        const FCu fc = fcu(uw, ax, rdx, a.dT);
+        S.fx[e] = make_float4(fc.tr, fc.d0c, fc.d1c, fc.R);
+        float ftr = tdiff(ax, ue, uw);
+        unsigned mb = fc.tr > 0.0f ? MB_POS : 0u;
+        if (land) {
+            const int l0 = lm32(m, a.lm, fi, j, L), lp1 = lm32(m, a.lm, fi + 1, j, L);
+            mb |= mask_byte(fc.tr, lm32(m, a.lm, fi - 2, j, L), lm32(m, a.lm, fi - 1, j, L), l0, lp1) | (l0 & lp1 ? MB_CELL : 0u);
+            ftr = mk<true>(ftr, lp1, l0);
+        }
+        S.tx[e] = -ftr;
+        S.mx[e] = (uint8_t)mb;
+        if (lane == 0) S.row[r] = gid3(m, 1, j, L);
     }
+#pragma unroll 5
+    for (int r = threadIdx.y; r < nr + 1; r += TR_PAIRS) {
+        const int e = r * 32 + lane, fj = j0 + r, ic = min(f, m.Gx);
+        const bool special = fj == lasty + 1;
+        const bool zero = f > lastx || (special && m.ty != PI_PERIODIC);       // fill_halo_north_Gc! (Bounded)
+        const int fs = special ? m.Hy + 1 : fj;
+        const FCu fc = fcu(zero ? 0.0f : __ldg(vv + gid3(m, ic, fs, L)), ay, rdy, a.dT);
+        S.fy[e] = make_float4(fc.tr, fc.d0c, fc.d1c, fc.R);
+        unsigned mb = zero ? MB_ZERO : 0u;
+        const int jr = min(fj, m.Gy - 1), qr = gid3(m, ic, jr, L);
+        float ftr = tdiff(ay, __ldg(vv + qr + m.Gx), __ldg(vv + qr));
+        if (land) {
+            mb |= mask_byte(fc.tr, lm32(m, a.lm, ic, fs - 2, L), lm32(m, a.lm, ic, fs - 1, L), lm32(m, a.lm, ic, fs, L),
+                            lm32(m, a.lm, ic, fs + 1, L));
+            const int c0 = lm32(m, a.lm, ic, jr, L), cp = lm32(m, a.lm, ic, jr + 1, L);
+            mb |= c0 & cp ? MB_CELL : 0u;
+            ftr = mk<true>(ftr, cp, c0);
+        }
+        S.ty[e] = -ftr;
+        S.my[e] = (uint8_t)mb;
+    }
+    __syncthreads();
+    if (land) xy_walk<true>(a, m, it, S, nr, warp_row());
+    else xy_walk<false>(a, m, it, S, nr, warp_row());
 }
 
-// z sweep and the rest of tracer_update! for LZ levels of 32 columns: warp y of the block takes
-// tracer y and each lane walks its column keeping the 4-level stencil window of tracer_temp and
-// the flux of the face above the current cell. What does not depend on the tracer is formed once
-// per item in shared memory for the 14 tracer warps: the face coefficients, the vertical
-// transport term of each cell, the cell counts and the per-level constants (ΔT/vol, ΔT/ΔzC and
-// the fixed-point unit per volume). As the warps walk the same cells, the forcing terms' reads of
-// the other tracers at a cell hit lines already loaded.
+// z sweep and the rest of tracer_update! for LZ levels of 32 columns: warp p of the block walks tracer
+// pair p down the columns (packed instructions for both tracers) with the 4-level stencil window of
+// tracer_temp and the flux of the face above the current cell in registers, and the inputs of the
+// next two levels on their way. What does not depend on the tracer is formed once per item in
+// shared memory for the 7 warps: the face coefficients, the vertical transport term of each cell, a bit
+// per cell with individuals and the per-level constants (ΔT/vol, ΔT/ΔzC and the fixed-point unit per
+// volume). As the warps walk the same cells, the forcing terms' reads of the other tracers at a cell hit
+// lines already loaded: while they are in L1, which is what shared memory leaves of it. On 256×256×64 the
+// kernel took 368 µs with 49 KB per block (which rounds to all of L1 at four blocks), 284 µs at 48 KB and
+// 260 µs at 23 KB; 337 µs with a warp per pair whose inputs were not fetched ahead. Five blocks (56
+// registers) spill: 309 µs. Levels per walk: 358 µs with 16, 260 with 32, 278 with 64 (each walk reads
+// three levels of tracer_temp more than it writes). Latency bounds what is left.
 struct ZLev {
     float dtv;      // ΔT / (Δx Δy ΔzF[k])
     float sk;       // ΔT / ΔzC (tracer_sinking!)
     float dz;       // ΔzF[k]
-    float dzn;      // ΔzF[k+1]
+    float kzu, kzd; // tracer_diffusion!: κv·ΔT / ΔzF[k]², κv·ΔT / (ΔzF[k]·ΔzF[k+1])
     double fxv;     // mmol per fixed-point unit / (Δx Δy ΔzF[k])
 };
 
@@ -1738,293 +1722,336 @@ __device__ __forceinline__ float fe_forcing(int n, const FeCoef& c, float dfe, f
     return __fadd_rn(__fadd_rn(-diss, __fmul_rn(__fmul_rn(scav, dfe), c.frac)), fe);
 }
 
-// Asynchronous global → shared copies (cp.async): a warp's z walk reads the inputs of each level
-// from a ring of ZS levels filled ahead of it, so ZS - 1 levels of loads are in flight while it
-// computes. A lane reads back only what it copied itself, which wait_group makes visible to it.
-__device__ __forceinline__ void cpa4(unsigned sdst, const float* gsrc) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" :: "r"(sdst), "l"(gsrc) : "memory");
+// tracer_diffusion! (tracer_diffusion.jl:1-21) of one cell for two tracers, with the face areas, widths
+// and ΔT of each axis folded into one coefficient (κh·ΔT/Δx², κh·ΔT/Δy², and per level κv·ΔT/ΔzF[k]² and
+// κv·ΔT/(ΔzF[k]·ΔzF[k+1])): per tracer and cell six differences and as many multiply-adds, where the terms
+// as the reference groups them take seven divisions.
+#define DB_E 1u                       // water in the cell and its eastern neighbour
+#define DB_W 2u                       // … and the western one as well (the x term is masked as a whole by DB_E)
+#define DB_N 4u
+#define DB_S 8u
+#define DB_DN 16u                     // the z term as a whole is masked by the cell below
+#define DB_UP 32u
+struct DifNb { fx2 e, w, n, s, up, dn; };
+__device__ __forceinline__ unsigned dif_bits(const MemberDev& m, const uint8_t* lm, int i, int j, int k) {
+    const int c = lm32(m, lm, i, j, k), e = c & lm32(m, lm, i + 1, j, k), n = c & lm32(m, lm, i, j + 1, k), d = c & lm32(m, lm, i, j, k + 1);
+    return (e ? DB_E : 0u) | (e & lm32(m, lm, i - 1, j, k) ? DB_W : 0u) | (n ? DB_N : 0u) | (n & lm32(m, lm, i, j - 1, k) ? DB_S : 0u)
+         | (d ? DB_DN : 0u) | (d & lm32(m, lm, i, j, k - 1) ? DB_UP : 0u);
 }
-// 8 bytes, or zeros without reading when `on` is false
-__device__ __forceinline__ void cpa8(unsigned sdst, const unsigned long long* gsrc, bool on) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" :: "r"(sdst), "l"(gsrc), "r"(on ? 8 : 0) : "memory");
+template <bool LM>
+__device__ __forceinline__ fx2 z_diffusion(const DifNb& v, fx2 c, unsigned bits, fx2 kx, fx2 ky, float kzu, float kzd) {
+    auto dif = [&](fx2 x, unsigned b) { const fx2 d = fx2_sub(x, c); return LM ? fx2_and(d, and_mask(bits, b)) : d; };
+    const fx2 x = fx2_add(dif(v.e, DB_E), dif(v.w, DB_W)), y = fx2_add(dif(v.n, DB_N), dif(v.s, DB_S));
+    const fx2 z = fx2_fma(fx2_of(kzu, kzu), dif(v.up, DB_UP), fx2_mul(fx2_of(kzd, kzd), dif(v.dn, DB_DN)));
+    return fx2_fma(kx, x, fx2_fma(ky, y, z));
 }
-__device__ __forceinline__ void cpa_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cpa_wait() { asm volatile("cp.async.wait_group %0;\n" :: "n"(N) : "memory"); }
-// shared loads ordered after the wait above (volatile asm keeps program order among them)
-__device__ __forceinline__ float lds_f32(unsigned a) {
-    float v;
-    asm volatile("ld.shared.f32 %0, [%1];\n" : "=f"(v) : "r"(a));
-    return v;
-}
-__device__ __forceinline__ unsigned long long lds_u64(unsigned a) {
-    unsigned long long v;
-    asm volatile("ld.shared.u64 %0, [%1];\n" : "=l"(v) : "r"(a));
-    return v;
+// apply_bcs! (apply_bcs.jl:4-98) of tracer n in a cell on a boundary
+__device__ __forceinline__ float z_fluxes(const TrArgs& a, const MemberDev& md, int n, int i, int j, int k, float dz) {
+    const float dT = a.dT;
+    float Gc = 0.0f;
+    const int64_t itn = a.st->iteration + 1;
+    const FluxBC32* B = a.bcs + md.bc_off + n * 6;
+    const int ii = i - md.Hx, jj = j - md.Hy, kk = k - md.Hz;
+    const float az = md.dx * md.dy, volk = az * dz;
+    const float axk = md.dy * dz, ayk = md.dx * dz;
+    if (B[PI_WEST].kind && i == 1 + md.Hx) Gc += getbc32(B[PI_WEST], jj, kk, itn) * dT * axk / volk;
+    if (B[PI_EAST].kind && i == md.Nx + md.Hx) Gc -= getbc32(B[PI_EAST], jj, kk, itn) * dT * axk / volk;
+    if (B[PI_SOUTH].kind && j == 1 + md.Hy) Gc += getbc32(B[PI_SOUTH], ii, kk, itn) * dT * ayk / volk;
+    if (B[PI_NORTH].kind && j == md.Ny + md.Hy) Gc -= getbc32(B[PI_NORTH], ii, kk, itn) * dT * ayk / volk;
+    if (B[PI_BOTTOM].kind && k == md.Nz + md.Hz) Gc += getbc32(B[PI_BOTTOM], ii, jj, itn) * dT * az / volk;
+    if (B[PI_TOP].kind && k == md.Hz + 1) Gc -= getbc32(B[PI_TOP], ii, jj, itn) * dT * az / volk;
+    return Gc;
 }
 
-#define ZS 4                              // levels of a z walk ring (power of two)
-// One warp's ring: own tracer c, tracer_temp t two levels below, the other tracers the forcing
-// reads and the particle sum of the cell. A nutrient warp uses x[0] and acc; an iron warp reads
-// DFe, POC, Dust, PFe_bio, PFe_inorg into x[0..3] and, for the fifth, the first 512 bytes of acc.
-struct ZRing {
-    float c[ZS][32];
-    float t[ZS][32];
-    float x[4][ZS][32];
-    unsigned long long acc[ZS][32];
-};
-static_assert(ZS == 4 && offsetof(ZRing, t) == 512 && offsetof(ZRing, x) == 1024 && offsetof(ZRing, acc) == 3072 &&
-              sizeof(ZRing) == 4096, "z walk ring layout");
+// Shared memory of an item: coefficients of the faces k0 .. k0 + LZ of the 32 columns, vertical transport
+// terms and populations of the cells, per-level constants, and with land the mask bits of face and cell
+// and of the cell's diffusion.
+struct ZItem { float4* f; float* tr; unsigned* pop; ZLev* lev; uint8_t *m, *d; };
+__host__ __device__ inline size_t ztail_smem(int lz, bool gen) {
+    return (size_t)(lz + 1) * 32 * sizeof(float4) + (size_t)lz * (32 * sizeof(float) + sizeof(unsigned) + sizeof(ZLev))
+         + (size_t)((gen ? 2 : 1) * lz + 1) * 32;
+}
+// add_forcing's coefficients of nutrient tracer n (tracer_forcings.jl:2-50): aS·T(n) + aO·T(other),
+// aO = 0 and other = n where there is no second tracer
+__device__ __forceinline__ int nutrient_forcing(int n, const BgcDev32& b, float dT, float& aS, float& aO) {
+    aS = 0.0f; aO = 0.0f;
+    switch (n) {
+        case PI_DIC: aO = b.kDOC * dT; return PI_DOC;
+        case PI_DOC: aS = -b.kDOC * dT; aO = b.kPOC * dT; return PI_POC;
+        case PI_POC: aS = -b.kPOC * dT; return n;
+        case PI_NH4: aS = -b.Nit * dT; aO = b.kDON * dT; return PI_DON;
+        case PI_NO3: aO = b.Nit * dT; return PI_NH4;
+        case PI_DON: aS = -b.kDON * dT; aO = b.kPON * dT; return PI_PON;
+        case PI_PON: aS = -b.kPON * dT; return n;
+        case PI_PO4: aO = b.kDOP * dT; return PI_DOP;
+        case PI_DOP: aS = -b.kDOP * dT; aO = b.kPOP * dT; return PI_POP;
+        default: aS = -b.kPOP * dT; return n;                     // POP
+    }
+}
+__device__ __forceinline__ fx2 fx2_max0(fx2 v) {
+    float l, h;
+    fx2_split(v, l, h);
+    return fx2_of(fmaxf(0.0f, l), fmaxf(0.0f, h));
+}
 
-// NUT: the ten nutrient tracers (linear forcing, particle sums); otherwise the three iron tracers
-// and dust (iron forcing, sinking). GEN: diffusion or flux boundary conditions are switched on.
-template <int LZ, bool LM, bool NUT, bool GEN>
-__device__ __forceinline__ void z_walk(const TrArgs& a, const MemberDev& md, const int4 it, const float4* sFC,
-                                       const float* sFtr, const int* sPop, const ZLev* sLev, ZRing& R) {
-    const int lane = threadIdx.x, n = threadIdx.y;
+// KIND 0: a nutrient pair (linear forcing, particle sums); 1: DFe and PFe_inorg; 2: PFe_bio and Dust (iron
+// forcing, sinking). GEN: diffusion or flux boundary conditions are switched on.
+template <int LZ, bool LM, int KIND, bool GEN>
+__device__ __forceinline__ void z_walk(const TrArgs& a, const MemberDev& md, const int4 it, const ZItem& S) {
+    const int lane = threadIdx.x, p = warp_row();
+    const int na = pair_tracer(p, 0), nb = pair_tracer(p, 1);
     // member constants in registers: the stores of the walk could otherwise alias them
     const int Nx = md.Nx, Hx = md.Hx, Hz = md.Hz, Gx = md.Gx, Gy = md.Gy;
     const int i = it.y + lane, j = it.z, k0 = it.w;
+    const int top = Hz + 1, bot = md.Nz + Hz, nl = min(LZ, bot - k0 + 1);
     // levels of the walk where any of the 32 columns holds an individual: only those have
-    // particle sums to read and zero (a warp-uniform test; the others skip the sum's copy)
+    // particle sums to read and zero (a warp-uniform test)
     uint64_t occm = 0;
-    if (NUT) {
-#pragma unroll 4
-        for (int l = 0; l < LZ; ++l)
-            if (__ballot_sync(0xffffffffu, sPop[l * 32 + lane] > 0)) occm |= 1ull << l;
+    if (KIND == 0) {
+        for (int l = 0; l < nl; l += 32) occm |= (uint64_t)__ballot_sync(0xffffffffu, l + lane < nl && S.pop[l + lane]) << l;
     }
     if (i > Nx + Hx) return;
     const long long G = a.Gtot, off = md.cell_off;
     const float dT = a.dT;
     const int slab = Gx * Gy;
-    const int top = Hz + 1, bot = md.Nz + Hz;
-    const int kend = min(k0 + LZ - 1, bot);
     const int qcol = (i - 1) + Gx * (j - 1);             // level 1 of the column, member-local
     const BgcDev32& b = a.bgc[it.x];
-    const bool sinks = !NUT && n != PI_DFe;
-    const float ws = n == PI_PFe_bio ? b.w_sink_org : b.w_sink_inorg;
-    // tracer_forcing! of the ten nutrient tracers: aS·T(n) + aO·T(x0) (aO = 0 where there is no
-    // second tracer); of the iron tracers: T of DFe, POC, Dust, PFe_bio, PFe_inorg, each the own
-    // tracer (-1) or one of the four others x0..x3
-    float aS = 0.0f, aO = 0.0f;
-    int xo[5] = { n, PI_POC, PI_Dust, PI_PFe_bio, PI_PFe_inorg };
-    if (NUT) {
-        switch (n) {
-            case PI_DIC: xo[0] = PI_DOC; aO = b.kDOC * dT; break;
-            case PI_DOC: aS = -b.kDOC * dT; xo[0] = PI_POC; aO = b.kPOC * dT; break;
-            case PI_POC: aS = -b.kPOC * dT; break;
-            case PI_NH4: aS = -b.Nit * dT; xo[0] = PI_DON; aO = b.kDON * dT; break;
-            case PI_NO3: xo[0] = PI_NH4; aO = b.Nit * dT; break;
-            case PI_DON: aS = -b.kDON * dT; xo[0] = PI_PON; aO = b.kPON * dT; break;
-            case PI_PON: aS = -b.kPON * dT; break;
-            case PI_PO4: xo[0] = PI_DOP; aO = b.kDOP * dT; break;
-            case PI_DOP: aS = -b.kDOP * dT; xo[0] = PI_POP; aO = b.kPOP * dT; break;
-            case PI_POP: aS = -b.kPOP * dT; break;
-            default: break;
-        }
+    const float* trm = a.tr + off;                        // all tracers of the member
+    const float* ca = trm + na * G;
+    const float* cb = trm + nb * G;
+    const float* ta = a.tb + na * G + off;
+    const float* tb = a.tb + nb * G + off;
+    float* oa = a.tr_next + na * G + off;
+    float* ob = a.tr_next + nb * G + off;
+    unsigned long long* accA = nullptr;
+    unsigned long long* accB = nullptr;
+    // forcing: two other tracers of a nutrient pair (its own where there is none), or POC, DFe and Dust,
+    // PFe_bio for the iron tracers
+    const float *x0 = nullptr, *x1 = nullptr, *x2 = nullptr;
+    bool has0 = true, has1 = true;
+    fx2 aS = 0ull, aO = 0ull;
+    if (KIND == 0) {
+        float sa, oa_, sb, ob_;
+        const int pa = nutrient_forcing(na, b, dT, sa, oa_), pb = nutrient_forcing(nb, b, dT, sb, ob_);
+        aS = fx2_of(sa, sb); aO = fx2_of(oa_, ob_);
+        has0 = pa != na; has1 = pb != nb;
+        x0 = trm + pa * G; x1 = trm + pb * G;
+        accA = a.acc + acc_slot(na) * G + off;
+        accB = a.acc + acc_slot(nb) * G + off;
+    } else if (KIND == 1) {
+        x0 = trm + PI_POC * G; x1 = trm + PI_Dust * G; x2 = trm + PI_PFe_bio * G;
     } else {
-        xo[0] = PI_DFe;
+        x0 = trm + PI_POC * G; x1 = trm + PI_DFe * G;
     }
     const FeCoef fc = fe_coef(b, dT);
-    // POC, PON and POP force on themselves only: their partner term reads the own value (aO = 0)
-    const bool partner = !NUT || xo[0] != n;
-    const float* __restrict__ t = a.tb + n * G + off;
-    const float* __restrict__ c = a.tr + n * G + off;
-    const float* __restrict__ trm = a.tr + off;           // all tracers of the member
-    float* __restrict__ out = a.tr_next + n * G + off;
-    unsigned long long* __restrict__ acc = a.acc + (NUT ? acc_slot(n) : 0) * G + off;
-    const uint8_t* __restrict__ lmc = a.lm + off + qcol;
-    auto tl = [&](int kk) { return qcol + (min(max(kk, top), bot) - 1) * slab; };
-    auto lmk = [&](int kk) -> int { return LM ? (int)lmc[(kk - 1) * slab] : 1; };
-    auto fcz = [&](int l) { const float4 v = sFC[l * 32 + lane]; FCu r; r.tr = v.x; r.d0c = v.y; r.d1c = v.z; r.R = v.w; return r; };
-    // ring addresses of this lane (shared space): stage sl of c at rc + 128 sl, t at rc + 512 +
-    // 128 sl, x[e] at rc + 1024 + 512 e + 128 sl, the particle sum at ra + 256 sl, the fifth
-    // iron tracer at rx4 + 128 sl
-    const unsigned rc = (unsigned)__cvta_generic_to_shared(&R.c[0][lane]);
-    const unsigned ra = (unsigned)__cvta_generic_to_shared(&R.acc[0][lane]);
-    const unsigned rx4 = (unsigned)__cvta_generic_to_shared(&R.acc[0][0]) + 4u * lane;   // iron x[4]: 128 B stages
-    const float* __restrict__ x0p = trm + xo[0] * G;
-    const float* __restrict__ x1p = trm + xo[1] * G;
-    const float* __restrict__ x2p = trm + xo[2] * G;
-    const float* __restrict__ x3p = trm + xo[3] * G;
-    const float* __restrict__ x4p = trm + xo[4] * G;
-    // ring fill of level kk (nothing past the last level: an empty group keeps the wait count)
-    auto issue = [&](int kk) {
-        if (kk <= kend) {                                     // warp-uniform
-            const unsigned so = (unsigned)((kk - k0) & (ZS - 1)) * 128u;
-            const int qq = qcol + (kk - 1) * slab;
-            cpa4(rc + so, c + qq);
-            cpa4(rc + 512u + so, t + tl(kk + 2));
-            if (NUT) {
-                if (partner) cpa4(rc + 1024u + so, x0p + qq);
-                if (occm >> (kk - k0) & 1ull) cpa8(ra + 2u * so, acc + qq, sPop[(kk - k0) * 32 + lane] > 0);
-            } else if (n != PI_Dust) {
-                cpa4(rc + 1024u + so, x0p + qq);
-                cpa4(rc + 1536u + so, x1p + qq);
-                cpa4(rc + 2048u + so, x2p + qq);
-                cpa4(rc + 2560u + so, x3p + qq);
-                cpa4(rx4 + so, x4p + qq);
-            }
+    const float wsa = b.w_sink_org, wsb = b.w_sink_inorg;        // PFe_bio; Dust and PFe_inorg
+    const bool dif = GEN && (b.kappa_h != 0.0f || b.kappa_v != 0.0f), bcs = GEN && md.any_bc;
+    const unsigned slab4 = 4u * (unsigned)slab, q40 = 4u * (unsigned)(qcol + (k0 - 1) * slab);
+    auto tl = [&](int kk) { return 4u * (unsigned)(qcol + (min(max(kk, top), bot) - 1) * slab); };
+    auto ld2 = [](const float* x, const float* y, unsigned q) { return fx2_of(ldg_at(x, q), ldg_at(y, q)); };
+    // inputs of a level: own tracers, tracer_temp two levels below, the others, the particle sums
+    struct In { fx2 c, t; float e0, e1, e2; long long sa, sb; };
+    unsigned qf = q40, qt = tl(k0 + 2);                   // byte offsets of the next level to fetch
+    auto fetch = [&](In& I, int l) {
+        if (l >= nl) {
+            if (GEN && l == nl) I.c = ld2(ca, cb, qf);    // the cell below the last one, for the diffusion
+            return;
         }
-        cpa_commit();
-    };
-#pragma unroll
-    for (int e = 0; e < ZS - 1; ++e) issue(k0 + e);
-    // stencil windows: w (tracer_temp) and mm (land mask) at levels k-1 .. k+2 of the current cell k
-    float w0 = t[tl(k0 - 2)], w1 = t[tl(k0 - 1)], w2 = t[tl(k0)], w3 = t[tl(k0 + 1)];
-    int mm0 = lmk(k0 - 2), mm1 = lmk(k0 - 1), mm2 = lmk(k0), mm3 = lmk(k0 + 1);
-    float Ft = flux_v<LM>(fcz(0), w0, w1, w2, w3, mm0, mm1, mm2, mm3);
-    int q = qcol + (k0 - 1) * slab;
-    float sink_prev = (sinks && k0 - 1 > Hz) ? c[q - slab] : 0.0f;
-    for (int k = k0; k <= kend; ++k, q += slab) {
-        const int l = k - k0;
-        const unsigned so = (unsigned)(l & (ZS - 1)) * 128u;
-        issue(k + ZS - 1);
-        cpa_wait<ZS - 1>();
-        const float cc = lds_f32(rc + so);
-        w0 = w1; w1 = w2; w2 = w3; w3 = lds_f32(rc + 512u + so);
-        if (LM) { mm0 = mm1; mm1 = mm2; mm2 = mm3; mm3 = lmk(k + 2); }
-        const int l1 = mm1, l0 = mm2;                       // land mask of cell k and k+1
-        const float Fb = flux_v<LM>(fcz(l + 1), w0, w1, w2, w3, mm0, mm1, mm2, mm3);   // zero at the bottom
-        const ZLev L = sLev[l];
-        float Gc = __fsub_rn(upd_sweep(w1, L.dtv, mk<LM>(__fsub_rn(Ft, Fb), l0, l1), cc, sFtr[l * 32 + lane]), cc);
-        Ft = Fb;
-        if (GEN) {
-            // tracer_diffusion! (tracer_diffusion.jl:1-21)
-            if (b.kappa_h != 0.0f || b.kappa_v != 0.0f) {
-                const float dz = L.dz, az = md.dx * md.dy, volk = az * dz;
-                const float axk = md.dy * dz, ayk = md.dx * dz;
-                auto lmq = [&](int dq) -> int { return LM ? (int)lmc[(k - 1) * slab + dq] : 1; };
-                auto dif = [&](int dq, int dp) { return mulbf(mulbf(c[q + dq] - c[q + dp], lmq(dq)), lmq(dp)); };
-                const float fx1 = b.kappa_h * axk * (dif(1, 0) / md.dx), fx0 = b.kappa_h * axk * (dif(0, -1) / md.dx);
-                const float fy1 = b.kappa_h * ayk * (dif(Gx, 0) / md.dy), fy0 = b.kappa_h * ayk * (dif(0, -Gx) / md.dy);
-                const float fz0 = b.kappa_v * az * (dif(-slab, 0) / dz), fz1 = b.kappa_v * az * (dif(0, slab) / L.dzn);
-                const float ax_ = mulbf(mulbf(fx1 - fx0, lmq(1)), l1);
-                const float ay_ = mulbf(mulbf(fy1 - fy0, lmq(Gx)), l1);
-                const float az_ = mulbf(mulbf(fz0 - fz1, l0), l1);
-                Gc += 1.0f / volk * (ax_ + ay_ + az_) * dT;
+        I.c = ld2(ca, cb, qf);
+        I.t = ld2(ta, tb, qt);
+        if (KIND == 0) {
+            if (has0) I.e0 = ldg_at(x0, qf);
+            if (has1) I.e1 = ldg_at(x1, qf);
+            if (occm >> l & 1ull) {
+                const bool on = S.pop[l] >> lane & 1u;
+                I.sa = on ? (long long)accA[qf >> 2] : 0;
+                I.sb = on ? (long long)accB[qf >> 2] : 0;
             }
-        }
-        if (NUT) {
-            // tracer_forcing! (tracer_forcings.jl:2-50) on max(0, tracer)
-            Gc = add_forcing(Gc, aS, cc, aO, partner ? lds_f32(rc + 1024u + so) : cc);
         } else {
-            // tracer_sinking! (tracer_sinking.jl:1-42)
-            if (sinks) {
-                const float fup = (k - 1 <= Hz) ? 0.0f : __fmul_rn(ws, sink_prev);
-                const float fdn = (k >= bot) ? 0.0f : __fmul_rn(ws, cc);
-                Gc = add_sinking(Gc, fup, fdn, L.sk);
-                sink_prev = cc;
-            }
-            if (n != PI_Dust) {
-                const float dfe = fmaxf(0.0f, lds_f32(rc + 1024u + so)), poc = fmaxf(0.0f, lds_f32(rc + 1536u + so));
-                const float dust = fmaxf(0.0f, lds_f32(rc + 2048u + so)), pfeb = fmaxf(0.0f, lds_f32(rc + 2560u + so));
-                const float pfei = fmaxf(0.0f, lds_f32(rx4 + so));
-                Gc += fe_forcing(n, fc, dfe, poc, dust, pfeb, pfei);
-            }
+            I.e0 = ldg_at(x0, qf);
+            I.e1 = ldg_at(x1, qf);
+            if (KIND == 1) I.e2 = ldg_at(x2, qf);
         }
-        if (GEN && md.any_bc) {
-            // apply_bcs! (apply_bcs.jl:4-98)
-            const int64_t itn = a.st->iteration + 1;
-            const FluxBC32* B = a.bcs + md.bc_off + n * 6;
-            const int ii = i - Hx, jj = j - md.Hy, kk = k - Hz;
-            const float dz = L.dz, az = md.dx * md.dy, volk = az * dz;
-            const float axk = md.dy * dz, ayk = md.dx * dz;
-            if (B[PI_WEST].kind && i == 1 + Hx) Gc += getbc32(B[PI_WEST], jj, kk, itn) * dT * axk / volk;
-            if (B[PI_EAST].kind && i == Nx + Hx) Gc -= getbc32(B[PI_EAST], jj, kk, itn) * dT * axk / volk;
-            if (B[PI_SOUTH].kind && j == 1 + md.Hy) Gc += getbc32(B[PI_SOUTH], ii, kk, itn) * dT * ayk / volk;
-            if (B[PI_NORTH].kind && j == md.Ny + md.Hy) Gc -= getbc32(B[PI_NORTH], ii, kk, itn) * dT * ayk / volk;
-            if (B[PI_BOTTOM].kind && k == bot) Gc += getbc32(B[PI_BOTTOM], ii, jj, itn) * dT * az / volk;
-            if (B[PI_TOP].kind && k == top) Gc -= getbc32(B[PI_TOP], ii, jj, itn) * dT * az / volk;
+        qf += slab4;
+        if (k0 + l + 2 < bot) qt += slab4;                // the clamped map of the Bounded halo fill
+    };
+    In I0{}, I1{};
+    fetch(I0, 0);
+    fetch(I1, 1);
+    // flux of a face between the cells w1 (above) and w2 (below) of the window: the upwind cell of a
+    // positive (upward) transport is the one below
+    auto zflux = [&](int e, fx2 w0, fx2 w1, fx2 w2, fx2 w3) {
+        bool pos;
+        const FCu2 fcz = get_fcu(S.f, e, pos);
+        const unsigned mb = LM ? S.m[e] : 0u;
+        return flux3(fcz, pos ? w3 : w0, pos ? w2 : w1, pos ? w1 : w2, LM, and_mask(mb, MB_AB), and_mask(mb, MB_BC));
+    };
+    // window of tracer_temp at levels k - 1 .. k + 2 of the current cell k
+    fx2 w0 = ld2(ta, tb, tl(k0 - 2)), w1 = ld2(ta, tb, tl(k0 - 1)), w2 = ld2(ta, tb, tl(k0)), w3 = ld2(ta, tb, tl(k0 + 1));
+    fx2 Ft = zflux(lane, w0, w1, w2, w3);
+    // sinking tracers of the level above: PFe_inorg, or PFe_bio and Dust
+    fx2 above = KIND != 0 && k0 - 1 > Hz ? ld2(ca, cb, tl(k0 - 1)) : 0ull;
+    unsigned q4 = q40;
+    const float khx = GEN ? b.kappa_h * dT / (md.dx * md.dx) : 0.0f, khy = GEN ? b.kappa_h * dT / (md.dy * md.dy) : 0.0f;
+    DifNb nb4;
+    if (GEN) nb4.up = ld2(ca, cb, q40 - slab4);
+    auto level = [&](In& I, const In& next, int l) {
+        const int k = k0 + l, e = l * 32 + lane;
+        const fx2 c = I.c;
+        w0 = w1; w1 = w2; w2 = w3; w3 = I.t;
+        const float e0 = I.e0, e1 = I.e1, e2 = I.e2;
+        const long long sa = I.sa, sb = I.sb;
+        if (GEN && dif) {
+            nb4.e = ld2(ca, cb, q4 + 4u); nb4.w = ld2(ca, cb, q4 - 4u);
+            nb4.n = ld2(ca, cb, q4 + 4u * (unsigned)Gx); nb4.s = ld2(ca, cb, q4 - 4u * (unsigned)Gx);
+            nb4.dn = next.c;
+        }
+        fetch(I, l + 2);
+        const fx2 Fb = zflux(e + 32, w0, w1, w2, w3);                  // zero at the bottom
+        const ZLev& L = S.lev[l];
+        const float tr = S.tr[e], ndtv = -L.dtv;
+        fx2 dF = fx2_sub(Ft, Fb);
+        if (LM) dF = cell_mask(dF, S.m[e]);
+        fx2 Gc = fx2_sub(upd_sweep2(w1, fx2_of(ndtv, ndtv), dF, c, fx2_of(tr, tr)), c);
+        Ft = Fb;
+        float cl, ch, gl, gh;
+        fx2_split(c, cl, ch);
+        if (GEN && dif) {
+            Gc = fx2_add(Gc, z_diffusion<LM>(nb4, c, LM ? S.d[e] : 0u, fx2_of(khx, khx), fx2_of(khy, khy), L.kzu, L.kzd));
+            nb4.up = c;
+        }
+        if (KIND == 0) {
+            // tracer_forcing! on max(0, tracer): G + (aS·T + aO·T_other)
+            Gc = fx2_add(Gc, fx2_fma(aS, fx2_max0(c), fx2_mul(aO, fx2_max0(fx2_of(has0 ? e0 : cl, has1 ? e1 : ch)))));
+        } else {
+            // tracer_sinking! (tracer_sinking.jl:1-42), then the iron forcing
+            float al, ah;
+            fx2_split(above, al, ah);
+            fx2_split(Gc, gl, gh);
+            auto sink = [&](float G0, float ws, float up, float own) {
+                const float fup = (k - 1 <= Hz) ? 0.0f : __fmul_rn(ws, up);
+                const float fdn = (k >= bot) ? 0.0f : __fmul_rn(ws, own);
+                return add_sinking(G0, fup, fdn, L.sk);
+            };
+            if (KIND == 2) gl = sink(gl, wsa, al, cl);
+            gh = sink(gh, wsb, ah, ch);
+            above = c;
+            const float poc = fmaxf(0.0f, e0);
+            if (KIND == 1) {
+                const float dfe = fmaxf(0.0f, cl), pfei = fmaxf(0.0f, ch), dust = fmaxf(0.0f, e1), pfeb = fmaxf(0.0f, e2);
+                gl = __fadd_rn(gl, fe_forcing(PI_DFe, fc, dfe, poc, dust, pfeb, pfei));
+                gh = __fadd_rn(gh, fe_forcing(PI_PFe_inorg, fc, dfe, poc, dust, pfeb, pfei));
+            } else {
+                const float dfe = fmaxf(0.0f, e1), pfeb = fmaxf(0.0f, cl);
+                gl = __fadd_rn(gl, fe_forcing(PI_PFe_bio, fc, dfe, poc, 0.0f, pfeb, 0.0f));
+            }
+            Gc = fx2_of(gl, gh);
         }
         // particle terms from the fixed-point sums (zeroed as they are consumed), apply_tendency!
         // (tracer_update.jl:6-13)
-        float plk = 0.0f;
-        if (NUT && (occm >> l & 1ull)) {
-            const long long vv = (long long)lds_u64(ra + 2u * so);   // zero where the cell holds no individual
-            if (vv) { acc[q] = 0ull; plk = (float)((double)vv * L.fxv); }
+        fx2 plk = 0ull;
+        if (KIND == 0 && (occm >> l & 1ull)) {
+            float pl = 0.0f, ph = 0.0f;
+            if (sa) { accA[q4 >> 2] = 0ull; pl = (float)((double)sa * L.fxv); }
+            if (sb) { accB[q4 >> 2] = 0ull; ph = (float)((double)sb * L.fxv); }
+            plk = fx2_of(pl, ph);
         }
-        out[q] = tendency(cc, Gc, plk);
+        float lo, hi;
+        fx2_split(fx2_add(c, fx2_add(Gc, plk)), lo, hi);
+        st_at(oa, q4, lo);
+        st_at(ob, q4, hi);
+        q4 += slab4;
+    };
+    int l = 0;
+#pragma unroll 2
+    for (; l + 1 < nl; l += 2) {
+        level(I0, I1, l);
+        level(I1, I0, l + 1);
     }
-    cpa_wait<0>();
-}
-
-template <int LZ, bool LM>
-__device__ __forceinline__ void z_walk_any(const TrArgs& a, const MemberDev& m, const int4 it, const float4* sFC,
-                                           const float* sFtr, const int* sPop, const ZLev* sLev, ZRing& R) {
-    const BgcDev32& b = a.bgc[it.x];
-    const bool gen = m.any_bc || b.kappa_h != 0.0f || b.kappa_v != 0.0f;
-    const bool nut = acc_slot(threadIdx.y) >= 0;
-    if (nut) {
-        if (gen) z_walk<LZ, LM, true, true>(a, m, it, sFC, sFtr, sPop, sLev, R);
-        else z_walk<LZ, LM, true, false>(a, m, it, sFC, sFtr, sPop, sLev, R);
-    } else {
-        if (gen) z_walk<LZ, LM, false, true>(a, m, it, sFC, sFtr, sPop, sLev, R);
-        else z_walk<LZ, LM, false, false>(a, m, it, sFC, sFtr, sPop, sLev, R);
+    if (l < nl) level(I0, I1, l);
+    if (GEN && bcs) {
+        // apply_bcs! touches boundary cells only: after the walk, so that its state takes no registers there
+        const bool edge = i == 1 + Hx || i == Nx + Hx || j == 1 + md.Hy || j == md.Ny + md.Hy;
+        for (int l = 0; l < nl; ++l) {
+            const int k = k0 + l, q = (int)(q40 >> 2) + l * slab;
+            if (!edge && k != top && k != bot) continue;
+            oa[q] += z_fluxes(a, md, na, i, j, k, S.lev[l].dz);
+            ob[q] += z_fluxes(a, md, nb, i, j, k, S.lev[l].dz);
+        }
     }
 }
 
-// dynamic shared memory of k32_ztail: one ring per tracer warp, then the per-item arrays (face
-// coefficients, transport terms, cell counts, per-level constants) of a walk of lz levels
-inline size_t ztail_smem(int lz) {
-    return sizeof(ZRing) * PI_NTRACERS + (size_t)(lz + 1) * 32 * sizeof(float4) + (size_t)lz * 32 * (sizeof(float) + sizeof(int))
-         + (size_t)lz * sizeof(ZLev);
+template <int LZ, bool LM, bool GEN>
+__device__ __forceinline__ void z_walk_any(const TrArgs& a, const MemberDev& m, const int4 it, const ZItem& S) {
+    const int p = warp_row();
+    if (p < 5) z_walk<LZ, LM, 0, GEN>(a, m, it, S);
+    else if (p == 5) z_walk<LZ, LM, 1, GEN>(a, m, it, S);
+    else z_walk<LZ, LM, 2, GEN>(a, m, it, S);
 }
 
-template <int LZ>
-__global__ void __launch_bounds__(32 * PI_NTRACERS, 2) k32_ztail(TrArgs a) {
+template <int LZ, bool GEN>
+__global__ void __launch_bounds__(32 * TR_PAIRS, GEN ? 3 : 4) k32_ztail(TrArgs a) {
     if (stopped(a.err)) return;
     extern __shared__ __align__(16) unsigned char zsm[];
-    ZRing* ring = reinterpret_cast<ZRing*>(zsm);
-    float4* sFC = reinterpret_cast<float4*>(zsm + sizeof(ZRing) * PI_NTRACERS);   // faces k0 .. k0+LZ of the 32 columns
-    float* sFtr = reinterpret_cast<float*>(sFC + (LZ + 1) * 32);       // vertical transport term of the cells k0 .. k0+LZ-1
-    int* sPop = reinterpret_cast<int*>(sFtr + LZ * 32);                 // individuals in those cells
-    ZLev* sLev = reinterpret_cast<ZLev*>(sPop + LZ * 32);               // per-level constants
+    ZItem S;
+    S.f = reinterpret_cast<float4*>(zsm);                               // faces k0 .. k0 + LZ of the 32 columns
+    S.lev = reinterpret_cast<ZLev*>(S.f + (LZ + 1) * 32);               // per-level constants
+    S.tr = reinterpret_cast<float*>(S.lev + LZ);                        // vertical transport term of the cells k0 .. k0 + LZ - 1
+    S.pop = reinterpret_cast<unsigned*>(S.tr + LZ * 32);                // a bit per cell of a level with individuals
+    S.m = reinterpret_cast<uint8_t*>(S.pop + LZ);
+    S.d = S.m + (LZ + 1) * 32;
     const int tid = threadIdx.y * 32 + threadIdx.x;
-    for (int w = blockIdx.x; w < a.nitems; w += gridDim.x) {
-        const int4 it = a.items[w];
-        const MemberDev& m = a.T.md[it.x];
-        const int k0 = it.w, bot = m.Nz + m.Hz;
-        const float* wv = a.F[it.x].vel1[2];
-        const float az = __fmul_rn(m.dx, m.dy);
-        for (int e = tid; e < (LZ + 1) * 32; e += 32 * PI_NTRACERS) {
-            const int f = k0 + e / 32, i = it.y + (e & 31);
-            const bool col = i <= m.Nx + m.Hx;
-            float4 fc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (col && f <= bot) {                            // fill_halo_bottom_Gc!: zero flux at the bottom
-                const int q = gid3(m, i, it.z, f);
-                const float wt = wv[q];
-                const FCu c = fcu(wt, az, a.rdzC[m.dz_off + f - 1], a.dT);
-                fc = make_float4(c.tr, c.d0c, c.d1c, c.R);
-                if (e < LZ * 32) {                            // cell f: w at its top and bottom faces
-                    const float ftr = tdiff(az, wt, wv[q + m.Gx * m.Gy]);
-                    sFtr[e] = m.all_water ? ftr : mulbf(mulbf(ftr, lm32(m, a.lm, i, it.z, f + 1)), lm32(m, a.lm, i, it.z, f));
-                    sPop[e] = a.pop[m.cell_off + q];
-                }
-            } else if (e < LZ * 32) {
-                sFtr[e] = 0.0f;
-                sPop[e] = 0;
+    const int4 it = a.items[blockIdx.x];
+    const MemberDev& m = a.T.md[it.x];
+    const int k0 = it.w, bot = m.Nz + m.Hz, nl = min(LZ, bot - k0 + 1);
+    const float* wv = a.F[it.x].vel1[2];
+    const float az = __fmul_rn(m.dx, m.dy);
+    const bool land = !m.all_water;
+#pragma unroll 4
+    for (int e = tid; e < (nl + 1) * 32; e += 32 * TR_PAIRS) {
+        const int f = k0 + e / 32, i = it.y + (e & 31), j = it.z;
+        FCu fc = {0.0f, 0.0f, 0.0f, 0.0f};
+        unsigned mb = 0u;
+        float ftr = 0.0f;
+        int pop = 0;
+        if (i <= m.Nx + m.Hx && f <= bot) {                   // fill_halo_bottom_Gc!: zero flux at the bottom
+            const int q = gid3(m, i, j, f);
+            const float wt = __ldg(wv + q);
+            fc = fcu(wt, az, __ldg(a.rdzC + m.dz_off + f - 1), a.dT);
+            ftr = tdiff(az, wt, __ldg(wv + q + m.Gx * m.Gy));  // cell f: w at its top and bottom faces
+            if (land) {
+                // the four points of the face from below, as those of an x or y face
+                const int c0 = lm32(m, a.lm, i, j, f), cp = lm32(m, a.lm, i, j, f + 1);
+                mb = mask_byte(fc.tr, cp, c0, lm32(m, a.lm, i, j, f - 1), lm32(m, a.lm, i, j, f - 2)) | (c0 & cp ? MB_CELL : 0u);
+                ftr = mulbf(mulbf(ftr, cp), c0);
             }
-            sFC[e] = fc;
+            pop = __ldg(a.pop + m.cell_off + q);
         }
-        if (tid < LZ) {
-            const int k = k0 + tid;
-            ZLev L = {0.0f, 0.0f, 1.0f, 1.0f, 0.0};
-            if (k <= bot) {
-                const float dz = a.dzF[m.dz_off + k - 1], volk = __fmul_rn(az, dz);
-                L.dtv = __fdiv_rn(a.dT, volk);
-                L.sk = __fdiv_rn(a.dT, a.dzC[m.dz_off + k - m.Hz - 1]);
-                L.dz = dz;
-                L.dzn = a.dzF[m.dz_off + k];
-                L.fxv = m.fx_unit / (double)volk;
-            }
-            sLev[tid] = L;
+        S.f[e] = make_float4(fc.tr, fc.d0c, fc.d1c, fc.R);
+        S.m[e] = (uint8_t)mb;
+        if (GEN && land && e < nl * 32) S.d[e] = (uint8_t)(i <= m.Nx + m.Hx ? dif_bits(m, a.lm, i, j, f) : 0u);
+        const unsigned occ = __ballot_sync(0xffffffffu, pop > 0);
+        if (e < nl * 32) {
+            S.tr[e] = -ftr;
+            if (threadIdx.x == 0) S.pop[e / 32] = occ;
         }
-        __syncthreads();
-        if (m.all_water) z_walk_any<LZ, false>(a, m, it, sFC, sFtr, sPop, sLev, ring[threadIdx.y]);
-        else z_walk_any<LZ, true>(a, m, it, sFC, sFtr, sPop, sLev, ring[threadIdx.y]);
-        __syncthreads();
     }
+    if (tid < nl) {
+        const int k = k0 + tid;
+        ZLev L;
+        const float dz = a.dzF[m.dz_off + k - 1], volk = __fmul_rn(az, dz);
+        L.dtv = __fdiv_rn(a.dT, volk);
+        L.sk = __fdiv_rn(a.dT, a.dzC[m.dz_off + k - m.Hz - 1]);
+        L.dz = dz;
+        const float kv = a.bgc[it.x].kappa_v * a.dT / dz;
+        L.kzu = kv / dz;
+        L.kzd = kv / a.dzF[m.dz_off + k];
+        L.fxv = m.fx_unit / (double)volk;
+        S.lev[tid] = L;
+    }
+    __syncthreads();
+    if (land) z_walk_any<LZ, true, GEN>(a, m, it, S);
+    else z_walk_any<LZ, false, GEN>(a, m, it, S);
 }
 
 // What the last kernel of a step does besides its own work: vel₀ .= vel₁ (time_step.jl:174-176),

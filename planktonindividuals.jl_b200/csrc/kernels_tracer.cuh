@@ -205,7 +205,6 @@ __device__ __forceinline__ void trk_body(const TrkArgs& A, const MemberDev& md, 
         Lv.dtv = __fdiv_rn(a.dT, volk);
         Lv.sk = __fdiv_rn(a.dT, a.dzC[md.dz_off + k - Hz - 1]);
         Lv.dz = dz;
-        Lv.dzn = a.dzF[md.dz_off + k];
         Lv.fxv = md.fx_unit / (double)volk;
         sLev[e] = Lv;
     }

@@ -1,4 +1,4 @@
-"""pi_batch_get_individuals writes its columns on the device: any subset of columns, separate or adjacent
+"""pi_batch_get_individuals and the FP64 form's pi_get_individuals write their columns on the device: any subset of columns, separate or adjacent
 arrays, one chunk or several, against the upload (logical order) and against each other."""
 import ctypes as ct
 
@@ -7,6 +7,7 @@ import pytest
 
 from PlanktonIndividuals import _abi, workloads as W
 from PlanktonIndividuals._abi import IND_DOUBLE, IND_INT, pi_individuals
+from PlanktonIndividuals._native import CModel
 from PlanktonIndividuals.batch import Member, PlanktonBatch
 from test_gpu_small_models import world, stepped
 
@@ -60,3 +61,17 @@ def test_column_subsets(gpu_lib, names):
         got = read(b, 0, names, adjacent)
         for k in names:
             assert np.array_equal(got[k], full[k].astype(got[k].dtype)), k
+
+
+@pytest.mark.parametrize("N,C", [(1, 1), (200, 257), (600000, 600001)])                    # the last in two chunks
+def test_fp64_upload_and_download_agree(gpu_lib, N, C):
+    w = world((6, 5, 4), N, C, 23)
+    m = CModel(gpu_lib, "pi_", w["grid"], w["bgc"], w["phyt"], 1, C, 1, precision=_abi.PI_FP64)
+    rng = np.random.default_rng(5)
+    inds = dict(w["inds"][0])
+    for k in ("graz", "mort", "dvid"):
+        inds[k] = (rng.random(C) < 0.5).astype(np.float64)
+    m.set_state([inds], w["trs"])
+    got = m.get_individuals(0)
+    for k in ("graz", "mort", "dvid", "xi", "yi", "zi", "ac"):
+        assert np.array_equal(got[k], inds[k]), k
