@@ -77,12 +77,13 @@ struct MemberHost {
 // Defaults: the autotuner's choices on a 256×256×64 model with 4 M individuals (pi_batch_autotune
 // retunes them for other sizes; no result depends on them)
 struct Tuning {
-    int bs_move = 256, bs_phys = 128, bs_assign = 128;
-    int persist_move = 2, persist_phys = 0;   // 0: one tile per block; k: k blocks per SM, looping
+    int bs_move = 128, bs_phys = 128, bs_assign = 128;
+    int persist_move = 0, persist_phys = 0;   // 0: one tile per block; k: k blocks per SM, looping
     int ty = 16;                              // rows of an x-y tracer tile (4, 8, 16 or 28)
     int lz = 32;                              // levels walked by a z thread (8, 16, 32 or 64)
     int wpb_par = 0;                          // warps per 32 columns of k32_par (0: by the levels)
-    int occ_move = 2, occ_phys = 4;           // register fit of k32_move / k32_physiology (blocks of 256 per SM)
+    int occ_move = 0, occ_phys = 3;           // register fit of k32_move / k32_physiology (blocks of 256 per SM;
+                                              // 0: k32_move<5> in blocks of 128, <2> in larger ones)
     int concurrent = -1;                      // k32_xy on a second branch beside the particle kernels (-1: by its size)
     int fused = 0;                            // k32_tracer when the batch allows it (the autotuner
                                               // picks it where it beats k32_xy + k32_ztail + halo fill)
@@ -526,7 +527,8 @@ pi_status enqueue_step(pi_batch* b, double dT, int cur) {
         a.sub = tile_sub(b, b->tune.bs_move);
         BScope sc(b, "k32_move");
         const unsigned g = unit_grid(b, b->tune.persist_move, a.sub);
-        if (b->tune.occ_move == 4) k32_move<4><<<g, b->tune.bs_move, 0, s>>>(a);
+        if (!b->tune.occ_move && b->tune.bs_move <= 128) k32_move<5><<<g, b->tune.bs_move, 0, s>>>(a);
+        else if (b->tune.occ_move == 4) k32_move<4><<<g, b->tune.bs_move, 0, s>>>(a);
         else if (b->tune.occ_move == 3) k32_move<3><<<g, b->tune.bs_move, 0, s>>>(a);
         else k32_move<2><<<g, b->tune.bs_move, 0, s>>>(a);
     }
@@ -583,7 +585,7 @@ pi_status enqueue_step(pi_batch* b, double dT, int cur) {
             BScope sc(b, "k32_ztail");
             const unsigned grid = (unsigned)std::max(1, b->nz_items);
             const dim3 blk(32, TR_PAIRS);
-                        bool gen = false;               // a member has tracer diffusion or flux boundary conditions
+            bool gen = false;               // a member has tracer diffusion or flux boundary conditions
             for (int m = 0; m < b->nm; ++m)
                 gen = gen || b->mdh[m].any_bc || (float)b->mh[m].bgc.kappa_h != 0.0f || (float)b->mh[m].bgc.kappa_v != 0.0f;
             const size_t zs = ztail_smem(b->tune.lz, gen);
@@ -1848,7 +1850,7 @@ pi_status pi_batch_autotune(pi_batch* b, double dT, int32_t k, char* report, siz
     struct Knob { const char* kernel; int* field; std::vector<int> values; const char* label; int threads_per_value; };
     Tuning& t = b->tune;
     std::vector<Knob> knobs = {
-        { "k32_move", &t.occ_move, {2, 3, 4}, "move register fit (blocks of 256 per SM)", 0 },
+        { "k32_move", &t.occ_move, {0, 2, 3, 4}, "move register fit (blocks of 256 per SM; 0 = by the block)", 0 },
         { "k32_move", &t.bs_move, {128, 256, 512, 1024}, "move block", 1 },
         { "k32_move", &t.persist_move, {0, 2, 4, 8}, "move blocks/SM (0 = one tile per block)", 0 },
         { "k32_physiology", &t.occ_phys, {2, 3, 4}, "physiology register fit (blocks of 256 per SM)", 0 },

@@ -119,14 +119,12 @@ __device__ __forceinline__ int clampb(int v, int lo, int hi, bool& bad) {
     return c;
 }
 
-// One velocity component around a position, as the coefficients of its trilinear interpolant in
-// grid cells per second: v(xd, yd, zd) = c0 + xd·cx + yd·cy + zd·cz + xd·yd·cxy + xd·zd·cxz +
-// yd·zd·cyz + xd·yd·zd·cxyz, formed from the 8 corner values (each divided by its ΔxC, ΔyC or ΔzC,
-// interpolation.jl:23-50) when they are loaded. The four RK stages of a step sample points a small
-// fraction of a cell apart, usually from the same field (vel₀ = vel½ = vel₁ between velocity
-// refreshes), so a stage reuses the coefficients of the previous one when the field and the base
-// corner are the same: only the loads and the setup are saved.
-struct Corners { int fid; int q; float c0, cx, cy, cz, cxy, cxz, cyz, cxyz; };   // fid: 0 vel₀, 1 vel½, 2 vel₁
+// The 8 corner values of each velocity component around a position, at (i + a, j + b, k + c) of the
+// component's base corner q (the vertical component in levels per second, its ΔzC differing between the
+// two). The four RK stages of a step sample points a small fraction of a cell apart, usually from the
+// same field (vel₀ = vel½ = vel₁ between velocity refreshes), so a stage reuses the corners of the
+// previous one when the field and the base corners are the same.
+struct Corners { int fid; int q[3]; float v[3][8]; };      // fid: 0 vel₀, 1 vel½, 2 vel₁
 
 // Member constants of the particle kernels, held in registers.
 struct PGeom {
@@ -147,46 +145,49 @@ __device__ __forceinline__ PGeom pgeom(const MemberDev& m, const MemberForcing& 
     return g;
 }
 
-// trilinear interpolation of one velocity component (member-local field pointer), in grid cells
-// per second
+// trilinear interpolation of the three velocity components (member-local fields), in grid cells per second
 // The 8 corner values come from the component's own halo-padded field: in the cell-sorted
 // storage order the lanes of a warp sit in neighbouring cells, so the corner loads of a warp
-// share sectors and the fields (12 bytes per cell) stay in L2.
+// share sectors and the fields (12 bytes per cell) stay in L2. In a warp some lane nearly always needs
+// other corners, of any component: one branch loads those of all three, so that a stage waits for memory
+// once, not three times.
 // Every position passed here lies in [0, N] on each axis (uploads are validated, stored positions
 // are clamped, stage positions pass through move_stage), so with H >= 2 the base corner (i, j, k)
 // satisfies 1 <= i <= Gx - 1 (likewise j, k) and needs no clamp.
-template <int COMP>
-__device__ __forceinline__ float itpl32(const PGeom& m, const float* __restrict__ fld, int fid,
-                                        const float* __restrict__ rdzC, const Ax1& X, const Ax1& Y,
-                                        const Ax1& Z, Corners& cc) {
-    int i, j, k;
-    float xd, yd, zd;
-    axis_iw(X, m.Hx, COMP == 0, i, xd);
-    axis_iw(Y, m.Hy, COMP == 1, j, yd);
-    axis_iw(Z, m.Hz, COMP == 2, k, zd);
-    const int q = (i - 1) + m.Gx * ((j - 1) + m.Gy * (k - 1));
-    if (cc.fid != fid || cc.q != q) {
-        const float* __restrict__ p = fld + q;                 // (i, j, k); level k+1 one slab on
-        const int sy = m.Gx, sz = m.Gx * m.Gy;
-        cc.fid = fid; cc.q = q;
-        // corners v_abc at (i + a, j + b, k + c), in cells per second
-        float s0 = m.rdx, s1 = m.rdx;
-        if (COMP == 1) { s0 = m.rdy; s1 = m.rdy; }
-        if (COMP == 2) { s0 = __ldg(rdzC + m.dz_off + k - 1); s1 = __ldg(rdzC + m.dz_off + k); }
-        const float v000 = __ldg(p) * s0, v010 = __ldg(p + sy) * s0, v100 = __ldg(p + 1) * s0, v110 = __ldg(p + 1 + sy) * s0;
-        const float v001 = __ldg(p + sz) * s1, v011 = __ldg(p + sz + sy) * s1, v101 = __ldg(p + sz + 1) * s1,
-                    v111 = __ldg(p + sz + 1 + sy) * s1;
-        cc.c0 = v000;
-        cc.cx = v100 - v000; cc.cy = v010 - v000; cc.cz = v001 - v000;
-        cc.cxy = (v110 - v100) - (v010 - v000);
-        cc.cxz = (v101 - v100) - (v001 - v000);
-        cc.cyz = (v011 - v010) - (v001 - v000);
-        cc.cxyz = ((v111 - v110) - (v101 - v100)) - ((v011 - v010) - (v001 - v000));
+__device__ __forceinline__ void itpl32(const PGeom& m, const float* const* fld, int fid, const float* __restrict__ rdzC,
+                                       const Ax1& X, const Ax1& Y, const Ax1& Z, Corners& cc, float& u, float& v, float& w) {
+    // own axis: on the faces; the other two: between the cell centres
+    int iF, jF, kF, iC, jC, kC;
+    float wx[2], wy[2], wz[2];
+    axis_iw(X, m.Hx, true, iF, wx[1]); axis_iw(Y, m.Hy, true, jF, wy[1]); axis_iw(Z, m.Hz, true, kF, wz[1]);
+    axis_iw(X, m.Hx, false, iC, wx[0]); axis_iw(Y, m.Hy, false, jC, wy[0]); axis_iw(Z, m.Hz, false, kC, wz[0]);
+    const int sy = m.Gx, sz = m.Gx * m.Gy;
+    const int q[3] = { (iF - 1) + sy * (jC - 1) + sz * (kC - 1), (iC - 1) + sy * (jF - 1) + sz * (kC - 1),
+                       (iC - 1) + sy * (jC - 1) + sz * (kF - 1) };
+    if (cc.fid != fid || cc.q[0] != q[0] || cc.q[1] != q[1] || cc.q[2] != q[2]) {
+        cc.fid = fid;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const float* __restrict__ p = fld[c] + q[c];
+            float* x = cc.v[c];
+            cc.q[c] = q[c];
+            x[0] = __ldg(p); x[1] = __ldg(p + 1); x[2] = __ldg(p + sy); x[3] = __ldg(p + sy + 1);
+            p += sz;
+            x[4] = __ldg(p); x[5] = __ldg(p + 1); x[6] = __ldg(p + sy); x[7] = __ldg(p + sy + 1);
+        }
+        const float s0 = __ldg(rdzC + m.dz_off + kF - 1), s1 = __ldg(rdzC + m.dz_off + kF);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) cc.v[2][e] *= e < 4 ? s0 : s1;
     }
-    const float ty = fmaf(zd, cc.cxyz, cc.cxy);
-    const float tx = fmaf(zd, cc.cxz, fmaf(yd, ty, cc.cx));
-    const float tz = fmaf(zd, cc.cyz, cc.cy);
-    return fmaf(zd, cc.cz, fmaf(yd, tz, fmaf(xd, tx, cc.c0)));
+    auto lerp = [](float t, float x, float y) { return fmaf(t, y - x, x); };
+    float r[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        const float tx = wx[c == 0], ty = wy[c == 1], tz = wz[c == 2];
+        const float* x = cc.v[c];
+        r[c] = lerp(tz, lerp(ty, lerp(tx, x[0], x[1]), lerp(tx, x[2], x[3])), lerp(ty, lerp(tx, x[4], x[5]), lerp(tx, x[6], x[7])));
+    }
+    u = r[0] * m.rdx; v = r[1] * m.rdy; w = r[2];
 }
 
 // the draws of the FP64 form (same keys, same numbers; lattice values are exact in float)
@@ -419,29 +420,23 @@ __device__ __forceinline__ MoveOut move_one(const MoveArgs& a, const MemberDev& 
     const Ax1 X0{ci, ox}, Y0{cj, oy}, Z0{ck, oz};
     const float dT = a.dT, hdT = 0.5f * dT;
     const float* __restrict__ rdzC = a.rdzC;
-    Corners cu{-1, -1}, cv{-1, -1}, cw{-1, -1};
-    const int fh = pg.fh, f1 = pg.f1;
-    float u1 = itpl32<0>(pg, f.vel0[0], 0, rdzC, X0, Y0, Z0, cu);
-    float v1 = itpl32<1>(pg, f.vel0[1], 0, rdzC, X0, Y0, Z0, cv);
-    float w1 = itpl32<2>(pg, f.vel0[2], 0, rdzC, X0, Y0, Z0, cw);
-    float u2 = u1, v2 = v1, w2 = w1;
+    // RK4: stages at X0, X0 + k1·ΔT/2, X0 + k2·ΔT/2, X0 + k3·ΔT, weights 1, 2, 2, 1
+    Corners cc;
+    cc.fid = -1;
     Ax1 X = X0, Y = Y0, Z = Z0;
-    move_stage(X, u1 * hdT, pg.Nx, pg.tx, bad); move_stage(Y, v1 * hdT, pg.Ny, pg.ty, bad); move_stage(Z, -(w1 * hdT), pg.Nz, pg.tz, bad);
-    u1 = itpl32<0>(pg, f.velh[0], fh, rdzC, X, Y, Z, cu); v1 = itpl32<1>(pg, f.velh[1], fh, rdzC, X, Y, Z, cv);
-    w1 = itpl32<2>(pg, f.velh[2], fh, rdzC, X, Y, Z, cw);
-    u2 += u1 * 2.0f; v2 += v1 * 2.0f; w2 += w1 * 2.0f;
-    X = X0; Y = Y0; Z = Z0;
-    move_stage(X, u1 * hdT, pg.Nx, pg.tx, bad); move_stage(Y, v1 * hdT, pg.Ny, pg.ty, bad); move_stage(Z, -(w1 * hdT), pg.Nz, pg.tz, bad);
-    u1 = itpl32<0>(pg, f.velh[0], fh, rdzC, X, Y, Z, cu); v1 = itpl32<1>(pg, f.velh[1], fh, rdzC, X, Y, Z, cv);
-    w1 = itpl32<2>(pg, f.velh[2], fh, rdzC, X, Y, Z, cw);
-    u2 += u1 * 2.0f; v2 += v1 * 2.0f; w2 += w1 * 2.0f;
-    X = X0; Y = Y0; Z = Z0;
-    move_stage(X, u1 * dT, pg.Nx, pg.tx, bad); move_stage(Y, v1 * dT, pg.Ny, pg.ty, bad); move_stage(Z, -(w1 * dT), pg.Nz, pg.tz, bad);
-    u1 = itpl32<0>(pg, f.vel1[0], f1, rdzC, X, Y, Z, cu); v1 = itpl32<1>(pg, f.vel1[1], f1, rdzC, X, Y, Z, cv);
-    w1 = itpl32<2>(pg, f.vel1[2], f1, rdzC, X, Y, Z, cw);
+    float u2 = 0.0f, v2 = 0.0f, w2 = 0.0f;
+#pragma unroll
+    for (int st = 0; st < 4; ++st) {
+        float u, v, w;
+        itpl32(pg, st == 0 ? f.vel0 : st == 3 ? f.vel1 : f.velh, st == 0 ? 0 : st == 3 ? pg.f1 : pg.fh, rdzC, X, Y, Z, cc, u, v, w);
+        const float wt = st == 0 || st == 3 ? 1.0f : 2.0f, h = st == 2 ? dT : hdT;
+        u2 += u * wt; v2 += v * wt; w2 += w * wt;
+        X = X0; Y = Y0; Z = Z0;
+        if (st == 3) break;
+        move_stage(X, u * h, pg.Nx, pg.tx, bad); move_stage(Y, v * h, pg.Ny, pg.ty, bad); move_stage(Z, -(w * h), pg.Nz, pg.tz, bad);
+    }
     const float sixth = 1.0f / 6.0f;
-    u2 = (u2 + u1) * sixth; v2 = (v2 + v1) * sixth; w2 = (w2 + w1) * sixth;
-    X = X0; Y = Y0; Z = Z0;
+    u2 *= sixth; v2 *= sixth; w2 *= sixth;
     move(X, u2 * dT, pg.Nx, pg.tx); move(Y, v2 * dT, pg.Ny, pg.ty); move(Z, -(w2 * dT), pg.Nz, pg.tz);
     // random-walk diffusion (particle_diffusion.jl:16-33); a zero κ moves nothing
     const BgcDev32& b = a.bgc[mi];
@@ -524,10 +519,12 @@ __device__ __forceinline__ void scatter_move(const MoveArgs& a, int s, int seg, 
     }
 }
 
-// MINB: blocks of 256 threads per SM the registers are fitted for (2: 128 registers, 3: 80, 4: 64);
-// the autotuner picks the variant.
+// MINB: blocks per SM the registers are fitted for, of 256 threads (2: 128 registers, 3: 80, 4: 64) or, as
+// 5, of 128 (96 registers). The stages' loads wait for L2, so what bounds the kernel is how many warps wait
+// beside them: on 256×256×64 with 4 M individuals 318 µs with 16 warps per SM, 262 with 20 at 96 registers,
+// 295 with 24 at 80 (which spill). The autotuner picks the variant.
 template <int MINB>
-__global__ void __launch_bounds__(256, MINB) k32_move(MoveArgs a) {
+__global__ void __launch_bounds__(MINB == 5 ? 128 : 256, MINB) k32_move(MoveArgs a) {
     if (stopped(a.err)) return;
     __shared__ PGeom sg;
     const int bs = blockDim.x, ppt = F32_TILE / (bs * a.sub);
@@ -1281,6 +1278,8 @@ __device__ __forceinline__ void scatter_phys(const PhysArgs& a, int s, const Phy
     }
 }
 
+// MINB: blocks of 256 threads per SM the registers are fitted for. On 256×256×64 with 4 M individuals in
+// blocks of 128: 264 µs with 4 (64 registers, which spill), 257 at 72 registers, 237 with 3 (80).
 template <int MINB>
 __global__ void __launch_bounds__(256, MINB) k32_physiology(PhysArgs a) {
     if (stopped(a.err)) return;
