@@ -1744,21 +1744,19 @@ __device__ __forceinline__ fx2 z_diffusion(const DifNb& v, fx2 c, unsigned bits,
     const fx2 z = fx2_fma(fx2_of(kzu, kzu), dif(v.up, DB_UP), fx2_mul(fx2_of(kzd, kzd), dif(v.dn, DB_DN)));
     return fx2_fma(kx, x, fx2_fma(ky, y, z));
 }
-// apply_bcs! (apply_bcs.jl:4-98) of tracer n in a cell on a boundary
-__device__ __forceinline__ float z_fluxes(const TrArgs& a, const MemberDev& md, int n, int i, int j, int k, float dz) {
-    const float dT = a.dT;
+// apply_bcs! (apply_bcs.jl:4-98) of a tracer (conditions B of its six faces) in a cell on the boundary faces
+// that are set in `on`
+__device__ __forceinline__ float z_fluxes(const MemberDev& md, const FluxBC32* B, unsigned on, int i, int j, int k, float dz, float dT, int64_t itn) {
     float Gc = 0.0f;
-    const int64_t itn = a.st->iteration + 1;
-    const FluxBC32* B = a.bcs + md.bc_off + n * 6;
     const int ii = i - md.Hx, jj = j - md.Hy, kk = k - md.Hz;
     const float az = md.dx * md.dy, volk = az * dz;
     const float axk = md.dy * dz, ayk = md.dx * dz;
-    if (B[PI_WEST].kind && i == 1 + md.Hx) Gc += getbc32(B[PI_WEST], jj, kk, itn) * dT * axk / volk;
-    if (B[PI_EAST].kind && i == md.Nx + md.Hx) Gc -= getbc32(B[PI_EAST], jj, kk, itn) * dT * axk / volk;
-    if (B[PI_SOUTH].kind && j == 1 + md.Hy) Gc += getbc32(B[PI_SOUTH], ii, kk, itn) * dT * ayk / volk;
-    if (B[PI_NORTH].kind && j == md.Ny + md.Hy) Gc -= getbc32(B[PI_NORTH], ii, kk, itn) * dT * ayk / volk;
-    if (B[PI_BOTTOM].kind && k == md.Nz + md.Hz) Gc += getbc32(B[PI_BOTTOM], ii, jj, itn) * dT * az / volk;
-    if (B[PI_TOP].kind && k == md.Hz + 1) Gc -= getbc32(B[PI_TOP], ii, jj, itn) * dT * az / volk;
+    if (on >> PI_WEST & 1u) Gc += getbc32(B[PI_WEST], jj, kk, itn) * dT * axk / volk;
+    if (on >> PI_EAST & 1u) Gc -= getbc32(B[PI_EAST], jj, kk, itn) * dT * axk / volk;
+    if (on >> PI_SOUTH & 1u) Gc += getbc32(B[PI_SOUTH], ii, kk, itn) * dT * ayk / volk;
+    if (on >> PI_NORTH & 1u) Gc -= getbc32(B[PI_NORTH], ii, kk, itn) * dT * ayk / volk;
+    if (on >> PI_BOTTOM & 1u) Gc += getbc32(B[PI_BOTTOM], ii, jj, itn) * dT * az / volk;
+    if (on >> PI_TOP & 1u) Gc -= getbc32(B[PI_TOP], ii, jj, itn) * dT * az / volk;
     return Gc;
 }
 
@@ -1969,13 +1967,22 @@ __device__ __forceinline__ void z_walk(const TrArgs& a, const MemberDev& md, con
     }
     if (l < nl) level(I0, I1, l);
     if (GEN && bcs) {
-        // apply_bcs! touches boundary cells only: after the walk, so that its state takes no registers there
-        const bool edge = i == 1 + Hx || i == Nx + Hx || j == 1 + md.Hy || j == md.Ny + md.Hy;
+        // apply_bcs! touches boundary cells only: after the walk, so that its state takes no registers there,
+        // and only where the tracer has a condition on a face of the cell
+        const FluxBC32 *Ba = a.bcs + md.bc_off + na * 6, *Bb = a.bcs + md.bc_off + nb * 6;
+        unsigned fa = 0u, fb = 0u;                        // faces with a condition
+#pragma unroll
+        for (int f = 0; f < 6; ++f) { fa |= (Ba[f].kind ? 1u : 0u) << f; fb |= (Bb[f].kind ? 1u : 0u) << f; }
+        const unsigned side = (i == 1 + Hx ? 1u << PI_WEST : 0u) | (i == Nx + Hx ? 1u << PI_EAST : 0u)
+                            | (j == 1 + md.Hy ? 1u << PI_SOUTH : 0u) | (j == md.Ny + md.Hy ? 1u << PI_NORTH : 0u);
+        const unsigned ends = 1u << PI_TOP | 1u << PI_BOTTOM;
+        if (!((fa | fb) & (side | ends))) return;
+        const int64_t itn = a.st->iteration + 1;
         for (int l = 0; l < nl; ++l) {
             const int k = k0 + l, q = (int)(q40 >> 2) + l * slab;
-            if (!edge && k != top && k != bot) continue;
-            oa[q] += z_fluxes(a, md, na, i, j, k, S.lev[l].dz);
-            ob[q] += z_fluxes(a, md, nb, i, j, k, S.lev[l].dz);
+            const unsigned on = side | (k == top ? 1u << PI_TOP : 0u) | (k == bot ? 1u << PI_BOTTOM : 0u);
+            if (fa & on) oa[q] += z_fluxes(md, Ba, fa & on, i, j, k, S.lev[l].dz, dT, itn);
+            if (fb & on) ob[q] += z_fluxes(md, Bb, fb & on, i, j, k, S.lev[l].dz, dT, itn);
         }
     }
 }
