@@ -170,8 +170,10 @@ def algorithmic_bytes(name, members, n_active_total, n_slots_total):
     # FP64 plain form (k_* kernels)
     if name == "k_particles_sorted":
         return n_active_total * (4 + 1 + 1 + 4 + 24 + 24 + 4 + 4 + 8)
-    if name in ("k_sweep_y", "k_sweep_z"):
-        return V * (14 * 8 * 3 + 8)
+    if name == "k64_xy":
+        return V * (14 * 8 * 2 + 16)                # tracers read, tracer_temp written; u, v
+    if name == "k64_ztail":
+        return V * (14 * 8 * 3 + 8)                 # tracers and tracer_temp read, tracers written; w
     return None
 
 

@@ -543,7 +543,8 @@ pi_status pi_batch_set_tracer_kernel(pi_batch* b, int32_t fused, int32_t levels)
 /* One launch-shape option (no counterpart in the reference; pi_batch_autotune sets them all):
  * "move_block" 128|256, "move_fit" 2|3|4 (register fit: blocks of 256 per SM),
  * "move_blocks_per_sm" 0|2|4|8 (0: one tile per block), the same three for "physiology_",
- * "xy_rows" 4|8|16|28, "z_levels" 8|16|32|64, "par_warps" 1|2|4|8, "tracer_fused" 0|1,
+ * "xy_rows" 4|8|16|28, "z_levels" 8|16|32|64, "par_warps" 1|2|4|8
+ * (warps per 32 surface columns), "tracer_fused" 0|1,
  * "tracer_fused_levels" 8|16|32|64, "xy_beside_particles" 0|1 (the x-y tracer kernel on a second
  * graph branch beside the particle kernels). Results are identical for every choice. */
 pi_status pi_batch_set_option(pi_batch* b, const char* name, int32_t value);
