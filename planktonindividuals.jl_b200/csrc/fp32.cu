@@ -21,8 +21,9 @@
 //                        down the levels
 //   (otherwise, and in the first step after a tracer upload, these three:)
 //   k32_xy               DST3FL x and y sweeps: a warp per tracer pair walks the rows of a level tile
-//   k32_ztail            z sweep walking columns, then diffusion, sinking, forcing, BCs, particle
-//                        terms and apply_tendency!
+//   k32_ztail            z sweep walking columns, then diffusion, sinking, forcing, particle terms and
+//                        apply_tendency!
+//   k32_close            the same with the flux BCs, in the cells that have one (members with flux BCs)
 //   k32_halo_direct (k32_halo_small, k32_halo<x,y,z>)  fill_halo_tracer!, then vel₀ ← vel₁,
 //                        iteration and t
 // Every sort_interval steps (and before the first step after an upload) the slots of every segment
@@ -585,14 +586,17 @@ pi_status enqueue_step(pi_batch* b, double dT, int cur) {
             BScope sc(b, "k32_ztail");
             const unsigned grid = (unsigned)std::max(1, b->nz_items);
             const dim3 blk(32, TR_PAIRS);
-            bool gen = false;               // a member has tracer diffusion or flux boundary conditions
-            for (int m = 0; m < b->nm; ++m)
+            bool bcs = false, gen = false;  // a member has flux boundary conditions; these or tracer diffusion
+            for (int m = 0; m < b->nm; ++m) {
+                bcs = bcs || b->mdh[m].any_bc;
                 gen = gen || b->mdh[m].any_bc || (float)b->mh[m].bgc.kappa_h != 0.0f || (float)b->mh[m].bgc.kappa_v != 0.0f;
+            }
             const size_t zs = ztail_smem(b->tune.lz, gen);
             if (b->tune.lz == 8) (gen ? k32_ztail<8, true> : k32_ztail<8, false>)<<<grid, blk, zs, s>>>(a);
             else if (b->tune.lz == 32) (gen ? k32_ztail<32, true> : k32_ztail<32, false>)<<<grid, blk, zs, s>>>(a);
             else if (b->tune.lz == 64) (gen ? k32_ztail<64, true> : k32_ztail<64, false>)<<<grid, blk, zs, s>>>(a);
             else (gen ? k32_ztail<16, true> : k32_ztail<16, false>)<<<grid, blk, zs, s>>>(a);
+            if (bcs) k32_close<<<grid, 256, 0, s>>>(a, b->tune.lz);
         }
         }
     }

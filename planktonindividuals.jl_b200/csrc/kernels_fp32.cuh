@@ -1760,13 +1760,25 @@ __device__ __forceinline__ float z_fluxes(const MemberDev& md, const FluxBC32* B
     return Gc;
 }
 
+// the faces of a tracer that have a condition
+__device__ __forceinline__ unsigned bc_faces(const FluxBC32* B) {
+    unsigned f = 0u;
+#pragma unroll
+    for (int e = 0; e < 6; ++e) f |= (B[e].kind ? 1u : 0u) << e;
+    return f;
+}
+// the x and y boundary faces of a cell in column (i, j)
+__device__ __forceinline__ unsigned side_faces(const MemberDev& md, int i, int j) {
+    return (i == 1 + md.Hx ? 1u << PI_WEST : 0u) | (i == md.Nx + md.Hx ? 1u << PI_EAST : 0u)
+         | (j == 1 + md.Hy ? 1u << PI_SOUTH : 0u) | (j == md.Ny + md.Hy ? 1u << PI_NORTH : 0u);
+}
 // Shared memory of an item: coefficients of the faces k0 .. k0 + LZ of the 32 columns, vertical transport
 // terms and populations of the cells, per-level constants, and with land the mask bits of face and cell
-// and of the cell's diffusion.
-struct ZItem { float4* f; float* tr; unsigned* pop; ZLev* lev; uint8_t *m, *d; };
+// and of the cell's diffusion; the faces of each tracer with a flux condition.
+struct ZItem { float4* f; float* tr; unsigned* pop; ZLev* lev; uint8_t *m, *d, *bc; };
 __host__ __device__ inline size_t ztail_smem(int lz, bool gen) {
     return (size_t)(lz + 1) * 32 * sizeof(float4) + (size_t)lz * (32 * sizeof(float) + sizeof(unsigned) + sizeof(ZLev))
-         + (size_t)((gen ? 2 : 1) * lz + 1) * 32;
+         + (size_t)((gen ? 2 : 1) * lz + 1) * 32 + (gen ? PI_NTRACERS : 0);
 }
 // add_forcing's coefficients of nutrient tracer n (tracer_forcings.jl:2-50): aS·T(n) + aO·T(other),
 // aO = 0 and other = n where there is no second tracer
@@ -1842,10 +1854,18 @@ __device__ __forceinline__ void z_walk(const TrArgs& a, const MemberDev& md, con
     }
     const FeCoef fc = fe_coef(b, dT);
     const float wsa = b.w_sink_org, wsb = b.w_sink_inorg;        // PFe_bio; Dust and PFe_inorg
-    const bool dif = GEN && (b.kappa_h != 0.0f || b.kappa_v != 0.0f), bcs = GEN && md.any_bc;
+    const bool dif = GEN && (b.kappa_h != 0.0f || b.kappa_v != 0.0f);
     const unsigned slab4 = 4u * (unsigned)slab, q40 = 4u * (unsigned)(qcol + (k0 - 1) * slab);
     auto tl = [&](int kk) { return 4u * (unsigned)(qcol + (min(max(kk, top), bot) - 1) * slab); };
     auto ld2 = [](const float* x, const float* y, unsigned q) { return fx2_of(ldg_at(x, q), ldg_at(y, q)); };
+    // apply_bcs! touches boundary cells only. Where a tracer of the pair has a condition on a face of the cell,
+    // the walk leaves the tendency in tr_next and the fluxes join it in k32_close; added to the new tracer, a flux below half an ulp of it would be lost.
+    // `open`: such cells are 1 all levels of the column, 2 the top one, 4 the bottom one.
+    unsigned open = 0u;
+    if (GEN) {
+        const unsigned any = S.bc[na] | S.bc[nb];
+        open = (any & side_faces(md, i, j) ? 1u : 0u) | (any >> PI_TOP & 1u ? 2u : 0u) | (any >> PI_BOTTOM & 1u ? 4u : 0u);
+    }
     // inputs of a level: own tracers, tracer_temp two levels below, the others, the particle sums
     struct In { fx2 c, t; float e0, e1, e2; long long sa, sb; };
     unsigned qf = q40, qt = tl(k0 + 2);                   // byte offsets of the next level to fetch
@@ -1954,7 +1974,8 @@ __device__ __forceinline__ void z_walk(const TrArgs& a, const MemberDev& md, con
             plk = fx2_of(pl, ph);
         }
         float lo, hi;
-        fx2_split(fx2_add(c, fx2_add(Gc, plk)), lo, hi);
+        Gc = fx2_add(Gc, plk);
+        fx2_split(GEN && (open & (1u | (k == top ? 2u : 0u) | (k == bot ? 4u : 0u))) ? Gc : fx2_add(c, Gc), lo, hi);
         st_at(oa, q4, lo);
         st_at(ob, q4, hi);
         q4 += slab4;
@@ -1966,25 +1987,6 @@ __device__ __forceinline__ void z_walk(const TrArgs& a, const MemberDev& md, con
         level(I1, I0, l + 1);
     }
     if (l < nl) level(I0, I1, l);
-    if (GEN && bcs) {
-        // apply_bcs! touches boundary cells only: after the walk, so that its state takes no registers there,
-        // and only where the tracer has a condition on a face of the cell
-        const FluxBC32 *Ba = a.bcs + md.bc_off + na * 6, *Bb = a.bcs + md.bc_off + nb * 6;
-        unsigned fa = 0u, fb = 0u;                        // faces with a condition
-#pragma unroll
-        for (int f = 0; f < 6; ++f) { fa |= (Ba[f].kind ? 1u : 0u) << f; fb |= (Bb[f].kind ? 1u : 0u) << f; }
-        const unsigned side = (i == 1 + Hx ? 1u << PI_WEST : 0u) | (i == Nx + Hx ? 1u << PI_EAST : 0u)
-                            | (j == 1 + md.Hy ? 1u << PI_SOUTH : 0u) | (j == md.Ny + md.Hy ? 1u << PI_NORTH : 0u);
-        const unsigned ends = 1u << PI_TOP | 1u << PI_BOTTOM;
-        if (!((fa | fb) & (side | ends))) return;
-        const int64_t itn = a.st->iteration + 1;
-        for (int l = 0; l < nl; ++l) {
-            const int k = k0 + l, q = (int)(q40 >> 2) + l * slab;
-            const unsigned on = side | (k == top ? 1u << PI_TOP : 0u) | (k == bot ? 1u << PI_BOTTOM : 0u);
-            if (fa & on) oa[q] += z_fluxes(md, Ba, fa & on, i, j, k, S.lev[l].dz, dT, itn);
-            if (fb & on) ob[q] += z_fluxes(md, Bb, fb & on, i, j, k, S.lev[l].dz, dT, itn);
-        }
-    }
 }
 
 template <int LZ, bool LM, bool GEN>
@@ -2006,6 +2008,7 @@ __global__ void __launch_bounds__(32 * TR_PAIRS, GEN ? 3 : 4) k32_ztail(TrArgs a
     S.pop = reinterpret_cast<unsigned*>(S.tr + LZ * 32);                // a bit per cell of a level with individuals
     S.m = reinterpret_cast<uint8_t*>(S.pop + LZ);
     S.d = S.m + (LZ + 1) * 32;
+    S.bc = S.d + LZ * 32;                                               // a bit per face with a condition, of each tracer
     const int tid = threadIdx.y * 32 + threadIdx.x;
     const int4 it = a.items[blockIdx.x];
     const MemberDev& m = a.T.md[it.x];
@@ -2042,6 +2045,9 @@ __global__ void __launch_bounds__(32 * TR_PAIRS, GEN ? 3 : 4) k32_ztail(TrArgs a
             if (threadIdx.x == 0) S.pop[e / 32] = occ;
         }
     }
+    if (GEN && tid < PI_NTRACERS) {
+        S.bc[tid] = (uint8_t)(m.any_bc ? bc_faces(a.bcs + m.bc_off + tid * 6) : 0u);
+    }
     if (tid < nl) {
         const int k = k0 + tid;
         ZLev L;
@@ -2058,6 +2064,41 @@ __global__ void __launch_bounds__(32 * TR_PAIRS, GEN ? 3 : 4) k32_ztail(TrArgs a
     __syncthreads();
     if (land) z_walk_any<LZ, true, GEN>(a, m, it, S);
     else z_walk_any<LZ, false, GEN>(a, m, it, S);
+}
+
+// Closes the cells that the walks of an item of k32_ztail left open (a tracer of the pair has a condition on
+// one of their faces): the fluxes join the tendency that waits in tr_next, and the tracer before the step is
+// added. A kernel of its own, launched when a member has a flux condition: at the end of k32_ztail a warp had
+// 31 levels of a boundary column one after the other, and the code cost the walk registers (117×93×31 with a
+// western, a bottom and a top condition: 75.5 µs there, 72 µs for the two kernels; 81 to 93 µs with the
+// tendency in k32_ztail in several forms).
+__global__ void __launch_bounds__(256) k32_close(TrArgs a, int lz) {
+    if (stopped(a.err)) return;
+    __shared__ uint8_t bc[PI_NTRACERS];                  // a bit per face with a condition
+    const int4 it = a.items[blockIdx.x];
+    const MemberDev& md = a.T.md[it.x];
+    if (!md.any_bc) return;
+    const FluxBC32* B = a.bcs + md.bc_off;
+    if (threadIdx.x < PI_NTRACERS) bc[threadIdx.x] = (uint8_t)bc_faces(B + threadIdx.x * 6);
+    __syncthreads();
+    const int j = it.z, k0 = it.w, bot = md.Nz + md.Hz, nl = min(lz, bot - k0 + 1);
+    const int64_t itn = a.st->iteration + 1;
+    for (int p = 0; p < TR_PAIRS; ++p) {
+        const int na = pair_tracer(p, 0), nb = pair_tracer(p, 1);
+        const unsigned fa = bc[na], fb = bc[nb];
+        if (!(fa | fb)) continue;
+        const float *ca = a.tr + na * a.Gtot + md.cell_off, *cb = a.tr + nb * a.Gtot + md.cell_off;
+        float *oa = a.tr_next + na * a.Gtot + md.cell_off, *ob = a.tr_next + nb * a.Gtot + md.cell_off;
+        for (int e = threadIdx.x; e < nl * 32; e += 256) {
+            const int i = it.y + (e & 31), k = k0 + (e >> 5);
+            const unsigned on = side_faces(md, i, j) | (k == 1 + md.Hz ? 1u << PI_TOP : 0u) | (k == bot ? 1u << PI_BOTTOM : 0u);
+            if (i > md.Nx + md.Hx || !((fa | fb) & on)) continue;
+            const int q = gid3(md, i, j, k);
+            const float ga = oa[q], gb = ob[q], va = __ldg(ca + q), vb = __ldg(cb + q), dz = a.dzF[md.dz_off + k - 1];
+            oa[q] = __fadd_rn(va, __fadd_rn(ga, z_fluxes(md, B + na * 6, fa & on, i, j, k, dz, a.dT, itn)));
+            ob[q] = __fadd_rn(vb, __fadd_rn(gb, z_fluxes(md, B + nb * 6, fb & on, i, j, k, dz, a.dT, itn)));
+        }
+    }
 }
 
 // What the last kernel of a step does besides its own work: vel₀ .= vel₁ (time_step.jl:174-176),
