@@ -253,10 +253,11 @@ __global__ void __launch_bounds__(128, 6) k_particles_sorted(DGrid g, const SpcD
 // The cell-sorted entry list (cells in order, gid = species·C + slot ascending within a cell, the
 // order of a sequential reference run) from the counting sort that k_particles began: k64_place puts
 // the individuals of a cell together in the order of the atomics, k64_order gives each its rank by
-// gid among them. A cell holds a few individuals, so a rank is a few comparisons; cells with more
-// than ORDER_BIG are left to k64_order_big. The radix sort of all keys took six launches: 35 µs for
-// 32,768 slots, 80 µs for 2,097,152.
-#define ORDER_BIG 2048
+// gid among them, by comparing it with all of them (98 per cell: 84 µs, 125 by a block each); cells of more
+// than ORDER_CELL are left to k64_order_big. Cells of more than CROWD_CELL are listed for the particle terms
+// (k64_plk). The radix sort of all keys took six launches: 35 µs for 32,768 slots, 80 µs for 2,097,152.
+#define ORDER_CELL 128
+#define CROWD_CELL 64
 __global__ void k64_place(const uint32_t* __restrict__ off, uint32_t Gcells, const uint32_t* __restrict__ key,
                           const int32_t* __restrict__ pos, uint32_t* __restrict__ list, long long n, const uint32_t* err) {
     const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -266,53 +267,96 @@ __global__ void k64_place(const uint32_t* __restrict__ off, uint32_t Gcells, con
 }
 __global__ void k64_order(const uint32_t* __restrict__ off, long long G, const uint32_t* __restrict__ key,
                           const uint32_t* __restrict__ list, uint32_t* __restrict__ gid_sorted, int32_t* __restrict__ pos,
-                          long long n, uint32_t* __restrict__ nbig, uint32_t* __restrict__ big, const uint32_t* err) {
+                          long long n, uint32_t* __restrict__ ncell, uint32_t* __restrict__ big, uint32_t* __restrict__ crowd,
+                          const uint32_t* err) {
     const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n || (*err & PI_DEVERR_CAPACITY) || p >= (long long)off[G]) return;
     const uint32_t gid = list[p], c = key[gid], p0 = off[c], m = off[c + 1] - p0;
-    if (m > ORDER_BIG) {
-        if (p == (long long)p0) big[atomicAdd(nbig, 1u)] = c;
-        return;
+    if (m > CROWD_CELL && p == (long long)p0) {
+        crowd[atomicAdd(&ncell[1], 1u)] = c;
+        if (m > ORDER_CELL) big[atomicAdd(&ncell[0], 1u)] = c;
     }
+    if (m > ORDER_CELL) return;
     uint32_t r = 0;
 #pragma unroll 4
     for (uint32_t x = 0; x < m; ++x) r += list[p0 + x] < gid;
     gid_sorted[p0 + r] = gid;
     pos[gid] = (int32_t)(p0 + r);
 }
-// A block per crowded cell (0D models: one cell holds every individual): the keys of all slots are in
-// gid order, so the cell's run is the slots with its key one after another. Each warp counts its share
-// of the keys, then writes behind the counts of the warps before it.
-__global__ void __launch_bounds__(1024) k64_order_big(const uint32_t* __restrict__ off, const uint32_t* __restrict__ key, long long n,
-                                                      const uint32_t* __restrict__ nbig, const uint32_t* __restrict__ big,
-                                                      uint32_t* __restrict__ gid_sorted, int32_t* __restrict__ pos,
-                                                      const uint32_t* err) {
-    __shared__ uint32_t sh[32];
+// A block per crowded cell, from the cell's own entries: up to ORDER_SORT of them are sorted in shared
+// memory (bitonic), more are set as bits of a window of the gids at a time and read back in order
+// (0D models: one cell holds every individual). The work grows with the entries, not with the slots. A step
+// with 1.6 million individuals in 2,097,152 slots, k64_place to here (radix sort of all keys; looking for each
+// crowded cell's key among all slots): 16 cells 422 µs (75; 614), 256 161 (82; 1,129), 1,024 102 (87; 813),
+// 4,096 90 (88; 230). Blocks of 256: with 1,024 threads 236, 123, 114 and 179.
+#define ORDER_SORT 8192
+#define ORDER_THREADS 256
+__global__ void __launch_bounds__(ORDER_THREADS) k64_order_big(const uint32_t* __restrict__ off, const uint32_t* __restrict__ list,
+                                                               long long n, const uint32_t* __restrict__ ncell,
+                                                               const uint32_t* __restrict__ big, uint32_t* __restrict__ gid_sorted,
+                                                               int32_t* __restrict__ pos, const uint32_t* err) {
+    // the entries, or a bit per gid of the window (32 words per thread, padded by one against bank conflicts)
+    __shared__ uint32_t s[ORDER_SORT + ORDER_SORT / 32], sums[ORDER_THREADS / 32];
     if (*err & PI_DEVERR_CAPACITY) return;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const long long run = (n + 1023) / 1024 * 32, a = min(n, wid * run), b = min(n, a + run);
-    for (uint32_t t = blockIdx.x; t < *nbig; t += gridDim.x) {
-        const uint32_t c = big[t];
-        uint32_t m = 0;
-#pragma unroll 8
-        for (long long q = a; q < b; q += 32) m += __popc(__ballot_sync(0xffffffffu, q + lane < b && key[q + lane] == c));
-        if (lane == 0) sh[wid] = m;
-        __syncthreads();
-        uint32_t at = off[c];
-        for (int w = 0; w < wid; ++w) at += sh[w];
-        if (m) {
-            for (long long q = a; q < b; q += 32) {
-                const bool in = q + lane < b && key[q + lane] == c;
-                const unsigned mk = __ballot_sync(0xffffffffu, in);
-                if (in) {
-                    const uint32_t e = at + __popc(mk & ((1u << lane) - 1u));
-                    gid_sorted[e] = (uint32_t)(q + lane);
-                    pos[q + lane] = (int32_t)e;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    auto pad = [](uint32_t w) { return w + (w >> 5); };
+    for (uint32_t t = blockIdx.x; t < ncell[0]; t += gridDim.x) {
+        const uint32_t c = big[t], p0 = off[c], m = off[c + 1] - p0;
+        if (m <= ORDER_SORT) {
+            uint32_t P = 2 * ORDER_CELL;
+            while (P < m) P *= 2;
+            for (uint32_t q = tid; q < P; q += ORDER_THREADS) s[q] = q < m ? list[p0 + q] : 0xffffffffu;
+            __syncthreads();
+            for (uint32_t k = 2; k <= P; k *= 2)
+                for (uint32_t j = k / 2; j; j /= 2) {
+                    for (uint32_t q = tid; q < P / 2; q += ORDER_THREADS) {
+                        const uint32_t i0 = 2 * q - (q & (j - 1)), i1 = i0 + j, x = s[i0], y = s[i1];
+                        if ((x > y) == ((i0 & k) == 0)) { s[i0] = y; s[i1] = x; }
+                    }
+                    __syncthreads();
                 }
-                at += __popc(mk);
+            for (uint32_t q = tid; q < m; q += ORDER_THREADS) {
+                gid_sorted[p0 + q] = s[q];
+                pos[s[q]] = (int32_t)(p0 + q);
             }
+            __syncthreads();
+            continue;
         }
-        __syncthreads();
+        uint32_t at = p0;
+        for (long long base = 0; base < n; base += 32LL * ORDER_SORT) {
+            for (int q = tid; q < ORDER_SORT + ORDER_SORT / 32; q += ORDER_THREADS) s[q] = 0u;
+            __syncthreads();
+#pragma unroll 4
+            for (uint32_t q = tid; q < m; q += ORDER_THREADS) {
+                const long long g = (long long)list[p0 + q] - base;
+                if (g >= 0 && g < 32LL * ORDER_SORT) atomicOr(&s[pad((uint32_t)g >> 5)], 1u << ((uint32_t)g & 31u));
+            }
+            __syncthreads();
+            // each thread its run of words, behind the counts of the threads before it
+            const uint32_t w0 = tid * (ORDER_SORT / ORDER_THREADS);
+            uint32_t cnt = 0;
+            for (uint32_t w = w0; w < w0 + ORDER_SORT / ORDER_THREADS; ++w) cnt += __popc(s[pad(w)]);
+            uint32_t inc = cnt;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= o) inc += y;
+            }
+            if (lane == 31) sums[wid] = inc;
+            __syncthreads();
+            uint32_t e = at + inc - cnt;
+            for (int w = 0; w < ORDER_THREADS / 32; ++w) {
+                if (w < wid) e += sums[w];
+                at += sums[w];
+            }
+            for (uint32_t w = w0; cnt && w < w0 + ORDER_SORT / ORDER_THREADS; ++w)
+                for (uint32_t b = s[pad(w)]; b; b &= b - 1u, ++e) {
+                    const uint32_t gid = (uint32_t)base + w * 32u + __ffs(b) - 1u;
+                    gid_sorted[e] = gid;
+                    pos[gid] = (int32_t)e;
+                }
+            __syncthreads();
+        }
     }
 }
 

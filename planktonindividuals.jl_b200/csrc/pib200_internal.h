@@ -117,12 +117,12 @@ struct FluxBCDev {
 
 // Per-step work arrays shared by the kernels.
 struct StepBufs {
-    uint32_t* cnt;          // G+1 counts of active individuals per cell (then nbig)
+    uint32_t* cnt;          // G+1 counts of active individuals per cell (then ncell)
     uint32_t* off;          // G+1 exclusive prefix of cnt
     uint32_t* key;          // nsp*C cell key (G-linear) per individual, sentinel when inactive
     uint32_t* list;         // nsp*C: the cells' individuals in the order of the atomics
-    uint32_t* nbig;         // cells of more than ORDER_BIG individuals, listed in big
-    uint32_t* big;
+    uint32_t* ncell;        // [0] cells of more than ORDER_CELL individuals, [1] of more than CROWD_CELL
+    uint32_t *big, *crowd;  // those cells
     uint32_t* gid_sorted;   // nsp*C: gid = sp*C + slot sorted by (cell, gid)
     int32_t* pos;           // nsp*C: position of gid in gid_sorted (valid when ST_AC0); while binning,
                             // its number among its cell's individuals
