@@ -620,35 +620,74 @@ __global__ void k_daughters(SpcDev P, const int32_t* __restrict__ divlist,
 }
 
 // The k-th divider (slot order) and the k-th free slot (findall(!ac), ascending) — get_tind!,
-// Individuals/utils.jl:76-86 — by one block from k_decide's bits, with the capacity check
-// (plankton_update.jl:18-22): each warp counts a run of words, then lists behind the warps before it,
-// and with `daughters` the block copies and halves them too. A scan of one 64-bit flag per slot and
-// two kernels took 20 µs at any size (the words are a 32nd of the slots: 64 KB for 262,144).
-__global__ void __launch_bounds__(1024) k64_divide(SpcDev P, long long C, const uint32_t* __restrict__ dvw,
-                                                   const uint32_t* __restrict__ frw, int32_t* divlist, int32_t* freelist,
-                                                   uint32_t* ndiv, uint32_t* err, int64_t* err_iter, int64_t iter,
-                                                   int daughters, int mode) {
-    __shared__ uint32_t shd[32], shf[32];
-    if (*err & PI_DEVERR_CAPACITY) return;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const long long words = (C + 31) / 32, run = (words + 1023) / 1024 * 32, w0 = min(words, wid * run), w1 = min(words, w0 + run);
+// Individuals/utils.jl:76-86 — from k_decide's bits, with the capacity check (plankton_update.jl:18-22). A block
+// takes DIVIDE_WORDS words: each warp counts a run of them, then lists behind the warps and blocks before
+// it. One block serves a species of up to DIVIDE_INBLOCK slots, and with `daughters` copies and halves them
+// too; above, k64_divide_count leaves every block's counts first, and k_daughters follows. With 1, 2, 4 and 8
+// times 1,048,576 slots: a scan of one 64-bit flag per slot and a list kernel 23, 31, 43 and 83 µs, one block for
+// all of them 24, 43, 75 and 139, these two 15, 15, 16 and 16.
+#define DIVIDE_WORDS 2048
+__device__ __forceinline__ uint2 divide_count(const uint32_t* __restrict__ dvw, const uint32_t* __restrict__ frw, long long w0, long long w1) {
     uint32_t nd = 0, nf = 0;
 #pragma unroll 4
-    for (long long w = w0 + lane; w < w1; w += 32) { nd += __popc(dvw[w]); nf += __popc(frw[w]); }
-    nd = __reduce_add_sync(0xffffffffu, nd);
-    nf = __reduce_add_sync(0xffffffffu, nf);
+    for (long long w = w0 + (threadIdx.x & 31); w < w1; w += 32) { nd += __popc(dvw[w]); nf += __popc(frw[w]); }
+    return make_uint2(__reduce_add_sync(0xffffffffu, nd), __reduce_add_sync(0xffffffffu, nf));
+}
+__global__ void __launch_bounds__(1024) k64_divide_count(long long words, const uint32_t* __restrict__ dvw, const uint32_t* __restrict__ frw,
+                                                         uint2* __restrict__ counts, const uint32_t* err) {
+    __shared__ uint32_t shd[32], shf[32];
+    if (*err & PI_DEVERR_CAPACITY) return;
+    const int wid = threadIdx.x >> 5;
+    const long long b0 = (long long)blockIdx.x * DIVIDE_WORDS, w0 = min(words, b0 + wid * (DIVIDE_WORDS / 32)), w1 = min(words, w0 + DIVIDE_WORDS / 32);
+    const uint2 n = divide_count(dvw, frw, w0, w1);
+    if ((threadIdx.x & 31) == 0) { shd[wid] = n.x; shf[wid] = n.y; }
+    __syncthreads();
+    if (wid) return;
+    const uint32_t nd = __reduce_add_sync(0xffffffffu, shd[threadIdx.x]), nf = __reduce_add_sync(0xffffffffu, shf[threadIdx.x]);
+    if (threadIdx.x == 0) counts[blockIdx.x] = make_uint2(nd, nf);
+}
+// words of a block: DIVIDE_WORDS, or all of them when it is the only one
+__global__ void __launch_bounds__(1024) k64_divide(SpcDev P, long long C, const uint32_t* __restrict__ dvw,
+                                                   const uint32_t* __restrict__ frw, const uint2* __restrict__ counts,
+                                                   int32_t* divlist, int32_t* freelist,
+                                                   uint32_t* ndiv, uint32_t* err, int64_t* err_iter, int64_t iter,
+                                                   int daughters, int mode) {
+    __shared__ uint32_t shd[32], shf[32], blk[4];
+    if (*err & PI_DEVERR_CAPACITY) return;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const long long words = (C + 31) / 32, b0 = (long long)blockIdx.x * DIVIDE_WORDS, b1 = gridDim.x == 1 ? words : min(words, b0 + DIVIDE_WORDS);
+    const long long run = (b1 - b0 + 1023) / 1024 * 32, w0 = min(b1, b0 + wid * run), w1 = min(b1, w0 + run);
+    const uint2 own = divide_count(dvw, frw, w0, w1);
+    const uint32_t nd = own.x, nf = own.y;
     if (lane == 0) { shd[wid] = nd; shf[wid] = nf; }
+    if (threadIdx.x < 4) blk[threadIdx.x] = 0u;
     __syncthreads();
     uint32_t tdiv = 0, tfree = 0, db = 0, fb = 0;
     for (int w = 0; w < 32; ++w) {
         if (w < wid) { db += shd[w]; fb += shf[w]; }
         tdiv += shd[w]; tfree += shf[w];
     }
+    if (gridDim.x > 1) {
+        // all blocks' counts: the blocks before this one, and the totals
+        uint32_t v[4] = { 0u, 0u, 0u, 0u };
+        for (unsigned q = threadIdx.x; q < gridDim.x; q += blockDim.x) {
+            const uint2 n = counts[q];
+            if (q < blockIdx.x) { v[0] += n.x; v[1] += n.y; }
+            v[2] += n.x; v[3] += n.y;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            v[q] = __reduce_add_sync(0xffffffffu, v[q]);
+            if (lane == 0 && v[q]) atomicAdd(&blk[q], v[q]);
+        }
+        __syncthreads();
+        db += blk[0]; fb += blk[1]; tdiv = blk[2]; tfree = blk[3];
+    }
     if (tdiv > tfree) {
-        if (threadIdx.x == 0) { *ndiv = 0; *err_iter = iter; __threadfence(); set_err(err, PI_DEVERR_CAPACITY); }
+        if (threadIdx.x == 0 && blockIdx.x == 0) { *ndiv = 0; *err_iter = iter; __threadfence(); set_err(err, PI_DEVERR_CAPACITY); }
         return;
     }
-    if (threadIdx.x == 0) *ndiv = tdiv;
+    if (threadIdx.x == 0 && blockIdx.x == 0) *ndiv = tdiv;
     if (tdiv == 0) return;
     for (long long w = w0; w < w1 && (nd || fb < tdiv); w += 32) {          // uniform over the warp
         uint32_t dw = nd && w + lane < w1 ? dvw[w + lane] : 0u, fw = fb < tdiv && w + lane < w1 ? frw[w + lane] : 0u;

@@ -375,10 +375,8 @@ pi_status enqueue_abiotic_exchange(pi_model* m, double dT) {
     return PI_OK;
 }
 
-// Enqueues one TimeStep! on the model's stream (no synchronisation).
-// Most slots of a species whose daughters k64_divide's one block copies: above, dividers come by the
-// thousand and k_daughters' 592 blocks are faster than one block's waits (the lists alone take one
-// block about 17 µs for 1,048,576 slots, where the scan and list kernels took 19).
+// Most slots of a species whose dividers one block of k64_divide lists and copies: above, dividers come by
+// the thousand, and the blocks of k_daughters are faster than one block's waits.
 #define DIVIDE_INBLOCK 262144
 
 // Rows or levels walked by a block of a tracer kernel (a power of two up to `most`): two blocks fit an
@@ -396,6 +394,7 @@ int walk_length(int most, int over, B blocks) {
     return best;
 }
 
+// Enqueues one TimeStep! on the model's stream (no synchronisation).
 pi_status enqueue_step(pi_model* m, double dT) {
     // getbc(bc, i, j, t) of a time-dependent flux reads bc[i, j, iteration] (boundary_conditions.jl:44-52)
     for (int n = 0; n < PI_NTRACERS; ++n)
@@ -469,11 +468,12 @@ pi_status enqueue_step(pi_model* m, double dT) {
         k_decide<<<nblk(C, BS), BS, 0, st>>>(g, m->h_spc[s], m->sp[s], mpz, ipz, C, s, sb.pos, sb.loss, sb.evk,
                                              sb.dvw, sb.frw, dsp + 1 * G, dsp + 2 * G, dsp + 3 * G, sb.err, m->mode());
         CK(cudaGetLastError(), "k_decide"); }
-        // one block copies the daughters too where they are few
         const int inblock = C <= DIVIDE_INBLOCK;
+        const long long dwords = (C + 31) / 32;
         { ProfScope ps_(m, "k64_divide");
-        k64_divide<<<1, 1024, 0, st>>>(m->h_spc[s], C, sb.dvw, sb.frw, sb.divlist, sb.freelist, sb.ndiv, sb.err, sb.err_iter,
-                                       m->iteration, inblock, m->mode());
+        if (!inblock) k64_divide_count<<<nblk(dwords, DIVIDE_WORDS), 1024, 0, st>>>(dwords, sb.dvw, sb.frw, sb.divcnt, sb.err);
+        k64_divide<<<inblock ? 1u : nblk(dwords, DIVIDE_WORDS), 1024, 0, st>>>(m->h_spc[s], C, sb.dvw, sb.frw, sb.divcnt, sb.divlist, sb.freelist,
+                                                                               sb.ndiv, sb.err, sb.err_iter, m->iteration, inblock, m->mode());
         CK(cudaGetLastError(), "k64_divide"); }
         if (!inblock) { ProfScope ps_(m, "k_daughters");
         k_daughters<<<148 * 4, 256, 0, st>>>(m->h_spc[s], sb.divlist, sb.freelist, sb.ndiv, sb.err, m->mode());
@@ -727,7 +727,7 @@ pi_status pi_create(const pi_grid* grid, const pi_bgc_params* bgc, const pi_quot
     StepBufs& sb = m->sb;
     ALB(sb.cnt, G + 3); ALB(sb.off, G + 1); ALB(sb.key, NC); ALB(sb.list, NC); ALB(sb.big, NC / ORDER_CELL + 1); ALB(sb.crowd, NC / CROWD_CELL + 1);
     sb.ncell = sb.cnt + G + 1;
-    ALB(sb.dvw, (C + 31) / 32); ALB(sb.frw, (C + 31) / 32);
+    ALB(sb.dvw, (C + 31) / 32); ALB(sb.frw, (C + 31) / 32); ALB(sb.divcnt, C / 32 / DIVIDE_WORDS + 1);
     ALB(sb.gid_sorted, NC); ALB(sb.pos, NC); ALB(sb.contrib, 5 * NC); ALB(sb.loss, 6 * NC);
     ALB(sb.evk, NC); ALB(sb.flag64, C); ALB(sb.rank64, C); ALB(sb.divlist, C); ALB(sb.freelist, C);
     ALB(sb.ndiv, 1); ALB(sb.err, 1); ALB(sb.err_iter, 1);

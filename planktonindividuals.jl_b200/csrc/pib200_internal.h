@@ -131,6 +131,7 @@ struct StepBufs {
     uint8_t* evk;           // per entry: 0 none, 1 grazing loss, 2 mortality loss
     uint32_t* dvw;          // C/32: one bit per slot, a divider
     uint32_t* frw;          // C/32: a free slot
+    uint2* divcnt;          // dividers and free slots of every DIVIDE_WORDS of these words
     unsigned long long* flag64;   // C: (releases << 32) | is_free (abiotic release)
     unsigned long long* rank64;   // C: exclusive prefix of flag64
     int32_t* divlist;       // C
