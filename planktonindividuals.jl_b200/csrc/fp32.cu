@@ -75,8 +75,9 @@ struct MemberHost {
     HostBC bcs[PI_NTRACERS][6];
 };
 
-// Defaults: the autotuner's choices on a 256×256×64 model with 4 M individuals (pi_batch_autotune
-// retunes them for other sizes; no result depends on them)
+// Defaults: a rule on the sizes where there is one (0 or -1), otherwise the autotuner's choices on a
+// 256×256×64 model with 4 M individuals. pi_batch_autotune and pi_batch_set_option set them; no result depends
+// on them.
 struct Tuning {
     int bs_move = 128, bs_phys = 128, bs_assign = 128;
     int persist_move = 0, persist_phys = 0;   // 0: one tile per block; k: k blocks per SM, looping
@@ -1739,17 +1740,17 @@ pi_status pi_batch_set_option(pi_batch* b, const char* name, int32_t value) {
     struct Opt { const char* name; int Tuning::*field; std::vector<int> values; };
     static const Opt opts[] = {
         { "move_block", &Tuning::bs_move, {128, 256} },
-        { "move_fit", &Tuning::occ_move, {2, 3, 4} },
+        { "move_fit", &Tuning::occ_move, {0, 2, 3, 4} },
         { "move_blocks_per_sm", &Tuning::persist_move, {0, 2, 4, 8} },
         { "physiology_block", &Tuning::bs_phys, {128, 256} },
         { "physiology_fit", &Tuning::occ_phys, {2, 3, 4} },
         { "physiology_blocks_per_sm", &Tuning::persist_phys, {0, 2, 4, 8} },
         { "xy_rows", &Tuning::ty, {4, 8, 16, 28} },
         { "z_levels", &Tuning::lz, {8, 16, 32, 64} },
-        { "par_warps", &Tuning::wpb_par, {1, 2, 4, 8} },
+        { "par_warps", &Tuning::wpb_par, {0, 1, 2, 4, 8} },
         { "tracer_fused", &Tuning::fused, {0, 1} },
         { "tracer_fused_levels", &Tuning::lz_fused, {8, 16, 32, 64} },
-        { "xy_beside_particles", &Tuning::concurrent, {0, 1} },
+        { "xy_beside_particles", &Tuning::concurrent, {-1, 0, 1} },
     };
     for (const Opt& o : opts) {
         if (strcmp(o.name, name)) continue;
