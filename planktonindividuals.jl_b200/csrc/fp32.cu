@@ -480,6 +480,9 @@ unsigned unit_grid(pi_batch* b, int persist, int sub) {
     return sub > 1 ? (unsigned)std::max(1, b->ntiles * sub) : tile_grid(b, persist);
 }
 
+// k32_par_divide: a block per segment, which reads every segment's counts (at most 1,024 of them)
+bool small_segments(const pi_batch* b) { return b->maxwps <= DIV_WORDS && b->nseg <= 1024; }
+
 // Enqueues one step on the batch stream (eager launches, or the body of a graph capture).
 pi_status enqueue_step(pi_batch* b, double dT, int cur) {
     cudaStream_t s = b->stream;
@@ -538,8 +541,7 @@ pi_status enqueue_step(pi_batch* b, double dT, int cur) {
     const int lw = b->tune.wpb_par ? b->tune.wpb_par : b->maxNz <= PAR_CH ? 1 : b->maxNz <= 2 * PAR_CH ? 2 : b->maxNz <= 4 * PAR_CH ? 4 : 8;
     const ParArgs pa{ b->T, b->dzF, b->bgc, b->chl_acc, b->PARF, b->par, b->diag_par, tr, G, b->F, b->pop, b->env, b->st, lw, b->maxNz };
     const unsigned parblocks = nblk((long long)b->T.nicol * lw, PAR_WARPS);
-    // a block per segment reads every segment's counts: at most 1,024 of them
-    if (b->maxwps <= DIV_WORDS && b->nseg <= 1024) {
+    if (small_segments(b)) {
       BScope sc(b, "k32_par_divide");
       k32_par_divide<<<b->nseg + parblocks, 32 * DIV_WARPS, 0, s>>>(
           pa, DivArgs{ b->T, b->P, b->divlist, b->freelist, b->nseg, b->st, b->errw });
@@ -1878,10 +1880,23 @@ pi_status pi_batch_autotune(pi_batch* b, double dT, int32_t k, char* report, siz
         return fa.maxThreadsPerBlock;
     };
     free_graphs(b);
-    // the knobs of the two-kernel tracer path are tuned on that path
-    const int fused0 = t.fused;
+    // the knobs of the two-kernel tracer path are tuned on that path, each kernel timed on its own (beside
+    // one another they share the SMs)
+    const int fused0 = t.fused, concurrent0 = t.concurrent;
     t.fused = 0;
+    t.concurrent = 0;
+    auto failed = [&](pi_status e) { t.fused = fused0; t.concurrent = concurrent0; b->profiling = was; return e; };
+    auto used = [&](const Knob& kb) {       // the kernel runs in this batch, and its shape is the knob's
+        if (kb.field == &t.bs_assign) return !small_segments(b);
+        if (kb.field == &t.persist_move) return tile_sub(b, t.bs_move) == 1;
+        if (kb.field == &t.persist_phys) return tile_sub(b, t.bs_phys) == 1;
+        return true;
+    };
     for (auto& kb : knobs) {
+        if (!used(kb)) {
+            rep += std::string(kb.label) + ": not used\n";
+            continue;
+        }
         int best = *kb.field;
         double best_ms = 1e300;
         const int lim = max_threads(kb.kernel);
@@ -1890,37 +1905,38 @@ pi_status pi_batch_autotune(pi_batch* b, double dT, int32_t k, char* report, siz
             *kb.field = v;
             double ms = 0.0;
             pi_status e = kernel_ms(kb.kernel, ms);
-            if (e) { b->profiling = was; return e; }
+            if (e) return failed(e);
             if (ms > 0.0 && ms < best_ms) { best_ms = ms; best = v; }
         }
         *kb.field = best;
         char line[160];
-        snprintf(line, sizeof line, "%s = %d (%.4f ms)\n", kb.label, best, best_ms);
+        snprintf(line, sizeof line, "%s = %d (%.4f ms)\n", kb.label, best, best_ms < 1e300 ? best_ms : 0.0);
         rep += line;
     }
     // tracer path: k32_tracer (levels per block tuned) against k32_xy + k32_ztail + halo fill
     double two = 0.0;
     pi_status e0 = kernel_ms("k32_xy|k32_ztail|k32_halo", two);
-    if (e0) { b->profiling = was; return e0; }
+    if (e0) return failed(e0);
     t.fused = 1;
     int best_lz = t.lz_fused;
     double fused_ms = 1e300;
     for (int v : {8, 16, 32, 64}) {
         t.lz_fused = v;
         double ms = 0.0;
-        if ((e0 = kernel_ms("k32_tracer", ms))) { b->profiling = was; return e0; }
+        if ((e0 = kernel_ms("k32_tracer", ms))) return failed(e0);
         if (ms > 0.0 && ms < fused_ms) { fused_ms = ms; best_lz = v; }
     }
     t.lz_fused = best_lz;
     t.fused = (fused_ms < two) ? 1 : (fused_ms < 1e300 ? 0 : fused0);
     // with the x-y/z kernels: k32_xy beside the particle kernels or after them (whole step timed)
+    t.concurrent = concurrent0;
     if (!t.fused) {
         double best_ms = 1e300;
         int best = t.concurrent;
         for (int v : {0, 1}) {
             t.concurrent = v;
             double ms = 0.0;
-            if ((e0 = kernel_ms("step", ms))) { b->profiling = was; return e0; }
+            if ((e0 = kernel_ms("step", ms))) return failed(e0);
             if (ms > 0.0 && ms < best_ms) { best_ms = ms; best = v; }
         }
         t.concurrent = best;

@@ -1,4 +1,6 @@
 """The launch-shape options of a batch: every default can be set again, and changes no result."""
+import re
+
 import pytest
 
 from PlanktonIndividuals import workloads as W
@@ -15,8 +17,8 @@ OTHERS = {"move_block": 256, "move_fit": 3, "move_blocks_per_sm": 2, "physiology
           "tracer_fused_levels": 8, "xy_beside_particles": 1}
 
 
-def make():
-    wl = W.config2(nx=24, nz=8, N_per_species=600, steps=60, nmodes=8, capacity=1500)
+def make(capacity=1500):
+    wl = W.config2(nx=24, nz=8, N_per_species=600, steps=60, nmodes=8, capacity=capacity)
     b = PlanktonBatch([Member(wl.grid, wl.bgc, wl.phyt, wl.capacity, wl.seed)], nspecies=2)
     b.set_state(0, wl.individuals, wl.tracers)
     b.set_series(0, vels={c: x[..., None] for c, x in zip("uvw", wl.velocity(0))}, ΔT_vel=wl.dT * 1000, PARF=wl.parf,
@@ -33,3 +35,14 @@ def test_every_default_can_be_set_again(gpu_lib):
             b.set_option(k, v)
         b.step(wl.dT, steps)
     assert compare_states(a.member(0), b.member(0), 2) == []
+
+
+@pytest.mark.parametrize("capacity", [1500, 270000])       # division in one block, and by tiles
+def test_autotune_report_is_well_formed(gpu_lib, capacity):
+    b, wl = make(capacity)
+    lines = b.autotune(wl.dT, steps_per_candidate=1).splitlines()
+    assert len(lines) == 12 and lines[-1].startswith("tracer path = ")
+    for line in lines[:-1]:
+        assert re.fullmatch(r"[^=:]+( \([^)]*\))?(: not used| = \d+ \(\d+\.\d{4} ms( per step)?\))", line), line
+    unused = [line for line in lines if line.endswith(": not used")]
+    assert any(line.startswith("assign block") for line in unused) == (capacity == 1500)
