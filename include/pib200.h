@@ -544,7 +544,7 @@ pi_status pi_batch_set_tracer_kernel(pi_batch* b, int32_t fused, int32_t levels)
  * "move_block" 128|256, "move_fit" 0|2|3|4 (register fit: blocks of 256 per SM; 0: 96 registers in blocks of
  * 128, 2 in larger ones), "move_blocks_per_sm" 0|2|4|8 (0: one tile per block), the same three for
  * "physiology_" (its fit 2|3|4), "xy_rows" 4|8|16|28, "z_levels" 8|16|32|64, "par_warps" 0|1|2|4|8 (warps per
- * 32 surface columns; 0: by the levels), "tracer_fused" 0|1, "tracer_fused_levels" 8|16|32|64,
+ * 32 surface columns; 0: by levels and columns), "tracer_fused" 0|1, "tracer_fused_levels" 8|16|32|64,
  * "xy_beside_particles" -1|0|1 (the x-y tracer kernel on a second graph branch beside the particle kernels;
  * -1: by its size). Results are identical for every choice. */
 pi_status pi_batch_set_option(pi_batch* b, const char* name, int32_t value);

@@ -83,7 +83,7 @@ struct Tuning {
     int persist_move = 0, persist_phys = 0;   // 0: one tile per block; k: k blocks per SM, looping
     int ty = 16;                              // rows of an x-y tracer tile (4, 8, 16 or 28)
     int lz = 32;                              // levels walked by a z thread (8, 16, 32 or 64)
-    int wpb_par = 0;                          // warps per 32 columns of k32_par (0: by the levels)
+    int wpb_par = 0;                          // warps per 32 columns of k32_par (0: by levels and columns)
     int occ_move = 0, occ_phys = 3;           // register fit of k32_move / k32_physiology (blocks of 256 per SM;
                                               // 0: k32_move<5> in blocks of 128, <2> in larger ones)
     int concurrent = -1;                      // k32_xy on a second branch beside the particle kernels (-1: by its size)
@@ -537,8 +537,11 @@ pi_status enqueue_step(pi_batch* b, double dT, int cur) {
         else if (b->tune.occ_move == 3) k32_move<3><<<g, b->tune.bs_move, 0, s>>>(a);
         else k32_move<2><<<g, b->tune.bs_move, 0, s>>>(a);
     }
-    // light: as many warps per 32 columns as the levels give work to
-    const int lw = b->tune.wpb_par ? b->tune.wpb_par : b->maxNz <= PAR_CH ? 1 : b->maxNz <= 2 * PAR_CH ? 2 : b->maxNz <= 4 * PAR_CH ? 4 : 8;
+    // light: as many warps per 32 columns as the levels give work to, as long as all of them run at once (1, 2, 4
+    // and 8: 256×256×64 53, 55, 59 and 64 µs, 181×181×40 31, 25, 30 and 34, 128×128×64 40, 27, 21 and 23)
+    int lw = b->maxNz <= PAR_CH ? 1 : b->maxNz <= 2 * PAR_CH ? 2 : b->maxNz <= 4 * PAR_CH ? 4 : 8;
+    while (lw > 1 && (long long)b->T.nicol * lw > (long long)b->nsm * PAR_BLOCKS * PAR_WARPS) lw /= 2;
+    if (b->tune.wpb_par) lw = b->tune.wpb_par;
     const ParArgs pa{ b->T, b->dzF, b->bgc, b->chl_acc, b->PARF, b->par, b->diag_par, tr, G, b->F, b->pop, b->env, b->st, lw, b->maxNz };
     const unsigned parblocks = nblk((long long)b->T.nicol * lw, PAR_WARPS);
     if (small_segments(b)) {

@@ -562,9 +562,13 @@ __global__ void __launch_bounds__(MINB == 5 ? 128 : 256, MINB) k32_move(MoveArgs
 // One thread walking a column waits for memory level by level, and 32 columns are one warp (ncu on
 // 128×128×64: 5 % of the warps resident, 34 µs at 9 % of DRAM). So 1, 2, 4 or 8 warps take the same 32
 // columns: each forms the attenuation of PAR_CH levels, the first carries the light down through
-// shared memory (one product per level), and all write their levels.
+// shared memory (one product per level), and all write their levels. Two blocks per SM, so that no register of
+// the loads in flight spills: three, which spilled, took 58 µs on 256×256×64 and 23 on 128×128×64, two 53
+// and 21 (one thread per column there 48 and 37, and 75 and 62 once the individuals had spread over more levels,
+// where two blocks take 60 and 23).
 #define PAR_CH 8
 #define PAR_WARPS 8
+#define PAR_BLOCKS 2
 struct ParArgs {
     Tab32 T;
     const float* dzF;
@@ -611,7 +615,7 @@ __device__ __forceinline__ void par_columns(const ParArgs& a, int block) {
     float parf = col && part == 0 ? a.PARF[fcol] : 0.0f;
     for (int kc0 = 0; kc0 < a.maxNz; kc0 += PAR_CH * lw) {          // same trip count for every warp
         const int k0 = kc0 + part * PAR_CH;                         // 0-based levels k0 .. k0 + PAR_CH - 1
-        float ex[PAR_CH], at[PAR_CH];
+        float ex[PAR_CH], at[PAR_CH], dg[PAR_CH];
         int pp[PAR_CH];
         if (col) {
             long long v[PAR_CH];
@@ -621,6 +625,7 @@ __device__ __forceinline__ void par_columns(const ParArgs& a, int block) {
                 const int q = q1 + (k0 + e) * slab;
                 v[e] = in ? (long long)chl_acc[q] : 0;
                 pp[e] = in ? __ldg(pop + q) : 0;
+                dg[e] = in ? diag[q] : 0.0f;
             }
 #pragma unroll
             for (int e = 0; e < PAR_CH; ++e) {
@@ -643,16 +648,14 @@ __device__ __forceinline__ void par_columns(const ParArgs& a, int block) {
         }
         __syncthreads();
         if (col) {
-            // four levels' loads (diagnostics, and the environment of occupied cells) at a time
+            // four levels' loads of the environment of occupied cells at a time
 #pragma unroll
             for (int g = 0; g < PAR_CH; g += 4) {
-                float dp[4];
                 float4 nv[4];
                 float tv[4];
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     const int q = q1 + (k0 + g + e) * slab;
-                    dp[e] = k0 + g + e < Nz ? diag[q] : 0.0f;
                     if (pp[g + e] > 0) {
                         nv[e] = make_float4(__ldg(tr + PI_NH4 * a.Gtot + q), __ldg(tr + PI_NO3 * a.Gtot + q),
                                             __ldg(tr + PI_PO4 * a.Gtot + q), __ldg(tr + PI_DOC * a.Gtot + q));
@@ -665,7 +668,7 @@ __device__ __forceinline__ void par_columns(const ParArgs& a, int block) {
                     const int q = q1 + (k0 + g + e) * slab;
                     const float pv = sIn[row0 + g + e][lane] * (1.0f - ex[g + e]) / at[g + e];
                     par[q] = pv;
-                    diag[q] = dp[e] + pv;
+                    diag[q] = dg[g + e] + pv;
                     if (pp[g + e] > 0) {
                         env[2 * q] = nv[e];
                         env[2 * q + 1] = make_float4(pv, tv[e], (float)pp[g + e], 0.0f);
@@ -678,7 +681,7 @@ __device__ __forceinline__ void par_columns(const ParArgs& a, int block) {
     if (col && part == 0) a.PARF[fcol] = parf;
 }
 
-__global__ void __launch_bounds__(32 * PAR_WARPS, 3) k32_par(ParArgs a) { par_columns(a, blockIdx.x); }
+__global__ void __launch_bounds__(32 * PAR_WARPS, PAR_BLOCKS) k32_par(ParArgs a) { par_columns(a, blockIdx.x); }
 
 // ------------------------------------------------------------------------------------------
 // (e) division: k-th divider (logical slot order) → k-th free logical slot (findall(!ac),
@@ -1006,7 +1009,7 @@ __device__ __forceinline__ void divide_segment(const DivArgs& a, int seg) {
 // Division and light depend on k32_move only and touch different arrays, so small models run both
 // in one launch: blocks 0 .. nseg - 1 divide a segment each, the others take the columns. Both go by
 // the step's `live` mark: a step that a dividing block stops still has its light.
-__global__ void __launch_bounds__(32 * DIV_WARPS, 3) k32_par_divide(ParArgs pa, DivArgs da) {
+__global__ void __launch_bounds__(32 * DIV_WARPS, PAR_BLOCKS) k32_par_divide(ParArgs pa, DivArgs da) {
     if ((int)blockIdx.x < da.nseg) {
         if (da.st->live) divide_segment(da, blockIdx.x);
     } else {
