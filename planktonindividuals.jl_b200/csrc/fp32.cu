@@ -1090,6 +1090,8 @@ pi_status pi_batch_set_individuals(pi_batch* b, int32_t member, int32_t sp, cons
     return PI_OK;
 }
 
+// Most slots of a segment that pi_batch_get_individuals brings to pageable memory in one copy
+#define EXPORT_ONE_COPY 8192
 pi_status pi_batch_get_individuals(pi_batch* b, int32_t member, int32_t sp, pi_individuals* out) {
     pi_status e = check_mem(b, member, "pi_get_individuals");
     if (e) return e;
@@ -1126,11 +1128,22 @@ pi_status pi_batch_get_individuals(pi_batch* b, int32_t member, int32_t sp, pi_i
     cudaStream_t s = b->stream;
     uint32_t* bad = (uint32_t*)b->scratch;
     BK(cudaMemsetAsync(bad, 0, sizeof(uint32_t), s), "download individuals");
+    // A copy into pageable memory costs about 10 µs of its own: up to EXPORT_ONE_COPY slots the columns come in one
+    // copy and are dealt out on the host (300 slots 45 µs against 217, 4,000 152 against 256, 8,000 296 against 313)
+    std::vector<const void*> to(dst.begin(), dst.end());
+    to.push_back(out->ac);
+    std::vector<char> host;
+    if (C <= EXPORT_ONE_COPY && C <= b->exp_slots && !all_direct(to.data(), (int)to.size()))
+        host.resize(dst.size() * (size_t)C * 8 + (out->ac ? (size_t)C : 0));
     for (long long L0 = 0; L0 < C; L0 += b->exp_slots) {
         const long long n = std::min(C - L0, b->exp_slots);
         k32_export<<<nblk(n, 256), 256, 0, s>>>(b->P, md, g0, L0, n, mask, cq_ns, b->exp_buf, bad);
         BK(cudaGetLastError(), "k32_export");
         const char* src = (const char*)b->exp_buf;
+        if (!host.empty()) {
+            BK(cudaMemcpyAsync(host.data(), src, host.size(), cudaMemcpyDeviceToHost, s), "download individuals");
+            break;
+        }
         for (size_t q = 0; q < dst.size();) {
             // columns that follow one another in the caller's memory too are one copy (two page-locked
             // allocations side by side are not: that copy is refused, and they are copied in turn)
@@ -1150,6 +1163,10 @@ pi_status pi_batch_get_individuals(pi_batch* b, int32_t member, int32_t sp, pi_i
     BK(cudaMemcpyAsync(&hb, bad, sizeof hb, cudaMemcpyDeviceToHost, s), "download individuals");
     BK(cudaStreamSynchronize(s), "synchronize");
     if (hb) return bfail(b, PI_ERR_STATE, "pi_get_individuals: storage order corrupted");
+    if (!host.empty()) {
+        for (size_t q = 0; q < dst.size(); ++q) memcpy(dst[q], host.data() + q * C * 8, C * 8);
+        if (out->ac) memcpy(out->ac, host.data() + dst.size() * C * 8, C);
+    }
     return PI_OK;
 }
 

@@ -9,9 +9,23 @@
 #include <string>
 #include <vector>
 
+#include <cuda_runtime.h>
+
 #include "../../include/pib200.h"
 
 namespace pih {
+
+// Whether every pointer that is not NULL is memory that the device copies to directly (page-locked or
+// managed), not pageable memory of the host.
+inline bool all_direct(const void* const* p, int n) {
+    for (int q = 0; q < n; ++q) {
+        cudaPointerAttributes a{};
+        if (!p[q]) continue;
+        if (cudaPointerGetAttributes(&a, p[q]) != cudaSuccess) { cudaGetLastError(); return false; }
+        if (a.type == cudaMemoryTypeUnregistered) return false;
+    }
+    return true;
+}
 
 struct HostGrid {
     int Nx, Ny, Nz, Hx, Hy, Hz, Gx, Gy, Gz;
