@@ -514,10 +514,12 @@ pi_status enqueue_step(pi_batch* b, double dT, int cur) {
         else if (ty == 8) k32_xy<8><<<grid, blk, xy_smem(8), st>>>(a);
         else k32_xy<4><<<grid, blk, xy_smem(4), st>>>(a);
     };
-    // beside the particle kernels when it leaves at least half of the SMs to them (measured per
-    // step: 0D parcel 38.6 -> 34.3 µs, 128×128×1 gyre 49.9 -> 45.1, 64 parcels 93.6 -> 89.0; no gain
-    // at 96×80×24 (114.5 -> 116.9) and above, where the two compete)
-    const bool branch = !fused && (b->tune.concurrent < 0 ? 2 * b->nxy_items <= b->nsm : b->tune.concurrent);
+    // beside the particle kernels up to 8 items per SM: both wait for loads more than they compute, and the
+    // shorter a model's launches are the more of them hides behind the other branch. In line and beside, µs per
+    // step: 0D parcel 33.8 and 32.0, 64 parcels 96.0 and 94.2, 128×128×1 44.8 and 37.6, 48×48×16 55.0 and 47.3,
+    // 64×64×24 73.2 and 68.2, 96×96×32 (768 items) 155.8 and 152.9; above, the two fill the SMs: 128×128×64 (2,560)
+    // 325.3 and 323.6, 256×256×64 (9,216) 1,014.8 and 1,018.1
+    const bool branch = !fused && (b->tune.concurrent < 0 ? b->nxy_items <= 8 * b->nsm : b->tune.concurrent);
     if (branch) {
         BK(cudaEventRecord(b->ev_fork, s), "fork");
         BK(cudaStreamWaitEvent(b->s2, b->ev_fork, 0), "fork");
