@@ -150,13 +150,15 @@ template <bool IRON>
 __global__ void __launch_bounds__(128) k64_plk(PlkArgs a) {
     __shared__ double sh[4][160];
     const DGrid& g = a.g;
-    if (*a.err & PI_DEVERR_CAPACITY) return;
     if (blockIdx.x >= a.cell_blocks) {
         const int wid = threadIdx.x >> 5;
-        for (uint32_t t = (blockIdx.x - a.cell_blocks) * 4 + wid; t < *a.ncrowd; t += (gridDim.x - a.cell_blocks) * 4)
+        const uint32_t n = *a.ncrowd;                     // (beside the error word: both loads are on the way)
+        if (*a.err & PI_DEVERR_CAPACITY) return;
+        for (uint32_t t = (blockIdx.x - a.cell_blocks) * 4 + wid; t < n; t += (gridDim.x - a.cell_blocks) * 4)
             plk_crowded<IRON>(a, a.crowd[t], sh[wid]);
         return;
     }
+    if (*a.err & PI_DEVERR_CAPACITY) return;
     const long long V = (long long)g.Nx * g.Ny * g.Nz, t = (long long)blockIdx.x * 128 + threadIdx.x;
     if (t >= V) return;
     const int i = (int)(t % g.Nx), r = (int)(t / g.Nx);

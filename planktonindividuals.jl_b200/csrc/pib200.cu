@@ -418,7 +418,7 @@ pi_status enqueue_step(pi_model* m, double dT) {
     StepBufs& sb = m->sb;
     const int BS = 256;
 
-    CK(cudaMemsetAsync(sb.cnt, 0, (G + 3) * sizeof(uint32_t), st), "zero counts");
+    CK(cudaMemsetAsync(sb.cnt, 0, (G + 6) / 4 * 4 * sizeof(uint32_t), st), "zero counts");       // cnt and ncell, in 16 bytes
     // vel½ = (vel₀ + vel₁)·0.5 is vel₁ itself, bit for bit, while vel₀ and vel₁ are the same field
     const bool steady = m->vel0[0] == m->vel1[0] && m->vel0[1] == m->vel1[1] && m->vel0[2] == m->vel1[2];
     const double* const* vh = steady ? m->vel1 : (const double* const*)m->velh;
@@ -447,7 +447,7 @@ pi_status enqueue_step(pi_model* m, double dT) {
     k64_order<<<nblk(NC, BS), BS, 0, st>>>(sb.off, G, sb.key, sb.list, sb.gid_sorted, sb.pos, NC, sb.ncell, sb.big, sb.crowd, sb.err);
     // no cell can be crowded in a model of few slots
     if (NC > ORDER_CELL)
-        k64_order_big<<<(unsigned)std::min<long long>(148 * 6, NC / ORDER_CELL), ORDER_THREADS, 0, st>>>(
+        k64_order_big<<<(unsigned)std::min<long long>(148 * 6, nblk(NC / ORDER_CELL, 4)), ORDER_THREADS, 0, st>>>(
             sb.off, sb.list, NC, sb.ncell, sb.big, sb.gid_sorted, sb.pos, sb.err);
     CK(cudaGetLastError(), "k64_order"); }
     {
@@ -521,7 +521,7 @@ pi_status enqueue_step(pi_model* m, double dT) {
         const bool lm = !g.all_water;
         { ProfScope ps_(m, "k64_plk");
         const unsigned cb = nblk((long long)g.Nx * g.Ny * g.Nz, 128);
-        const unsigned crowd = (unsigned)std::min<long long>(148 * 8, NC > CROWD_CELL ? nblk(NC / CROWD_CELL, 4) : 0);
+        const unsigned crowd = (unsigned)std::min<long long>(148 * 8, NC > CROWD_CELL ? nblk(NC / CROWD_CELL, 16) : 0);
         PlkArgs pa{ g, C, sb.off, sb.gid_sorted, sb.evk, sb.loss, sb.contrib, m->plk, sb.ncell + 1, sb.crowd, cb, sb.err };
         (m->iron ? k64_plk<true> : k64_plk<false>)<<<cb + crowd, 128, 0, st>>>(pa);
         CK(cudaGetLastError(), "k64_plk"); }
@@ -725,7 +725,7 @@ pi_status pi_create(const pi_grid* grid, const pi_bgc_params* bgc, const pi_quot
     ALB(m->zeros, G); ALB(m->par, G); ALB(m->PARF, (long long)hg.Nx * hg.Ny); ALB(m->temp_own, G);
     ALB(m->diag_par, G); ALB(m->diag_sp, 4LL * nspecies * G);
     StepBufs& sb = m->sb;
-    ALB(sb.cnt, G + 3); ALB(sb.off, G + 1); ALB(sb.key, NC); ALB(sb.list, NC); ALB(sb.big, NC / ORDER_CELL + 1); ALB(sb.crowd, NC / CROWD_CELL + 1);
+    ALB(sb.cnt, G + 6); ALB(sb.off, G + 1); ALB(sb.key, NC); ALB(sb.list, NC); ALB(sb.big, NC / ORDER_CELL + 1); ALB(sb.crowd, NC / CROWD_CELL + 1);
     sb.ncell = sb.cnt + G + 1;
     ALB(sb.dvw, (C + 31) / 32); ALB(sb.frw, (C + 31) / 32); ALB(sb.divcnt, C / 32 / DIVIDE_WORDS + 1);
     ALB(sb.gid_sorted, NC); ALB(sb.pos, NC); ALB(sb.contrib, 5 * NC); ALB(sb.loss, 6 * NC);
