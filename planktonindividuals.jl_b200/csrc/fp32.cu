@@ -1132,10 +1132,8 @@ pi_status pi_batch_get_individuals(pi_batch* b, int32_t member, int32_t sp, pi_i
     BK(cudaMemsetAsync(bad, 0, sizeof(uint32_t), s), "download individuals");
     // A copy into pageable memory costs about 10 µs of its own: up to EXPORT_ONE_COPY slots the columns come in one
     // copy and are dealt out on the host (300 slots 45 µs against 217, 4,000 152 against 256, 8,000 296 against 313)
-    std::vector<const void*> to(dst.begin(), dst.end());
-    to.push_back(out->ac);
     std::vector<char> host;
-    if (C <= EXPORT_ONE_COPY && C <= b->exp_slots && !all_direct(to.data(), (int)to.size()))
+    if (mask && C <= EXPORT_ONE_COPY && C <= b->exp_slots && !is_direct(dst.empty() ? (void*)out->ac : dst[0]))
         host.resize(dst.size() * (size_t)C * 8 + (out->ac ? (size_t)C : 0));
     for (long long L0 = 0; L0 < C; L0 += b->exp_slots) {
         const long long n = std::min(C - L0, b->exp_slots);

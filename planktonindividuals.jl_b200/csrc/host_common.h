@@ -15,16 +15,12 @@
 
 namespace pih {
 
-// Whether every pointer that is not NULL is memory that the device copies to directly (page-locked or
-// managed), not pageable memory of the host.
-inline bool all_direct(const void* const* p, int n) {
-    for (int q = 0; q < n; ++q) {
-        cudaPointerAttributes a{};
-        if (!p[q]) continue;
-        if (cudaPointerGetAttributes(&a, p[q]) != cudaSuccess) { cudaGetLastError(); return false; }
-        if (a.type == cudaMemoryTypeUnregistered) return false;
-    }
-    return true;
+// Whether p is memory that the device copies to directly (page-locked or managed), not pageable memory of
+// the host. The way taken for a set of columns goes by one of them: any way is right for any memory.
+inline bool is_direct(const void* p) {
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) { cudaGetLastError(); return false; }
+    return a.type != cudaMemoryTypeUnregistered;
 }
 
 struct HostGrid {

@@ -1041,10 +1041,10 @@ pi_status pi_get_individuals(pi_model* m, int32_t sp, pi_individuals* out) {
     // 20,000 378 and 392, 100,000 1.35 and 1.17 ms (never touched before: 4.8 and 5.4), 1 million 10.3 and 7.6
     // (41.6 and 43.2).
     void* const cols[6] = { out->graz, out->mort, out->dvid, out->xi, out->yi, out->zi };
-    const void* const wanted[7] = { cols[0], cols[1], cols[2], cols[3], cols[4], cols[5], out->ac };
+    const void* one = out->ac;
     uint32_t mask = out->ac ? 64u : 0u;
-    for (int q = 0; q < 6; ++q) if (cols[q]) mask |= 1u << q;
-    if (mask && C <= EXPORT_ON_HOST && !all_direct(wanted, 7)) {
+    for (int q = 0; q < 6; ++q) if (cols[q]) { mask |= 1u << q; one = cols[q]; }
+    if (mask && C <= EXPORT_ON_HOST && !is_direct(one)) {
         std::vector<uint8_t> flags(C);
         std::vector<int32_t> cell(C);
         CK(cudaMemcpyAsync(flags.data(), P.flags, C, cudaMemcpyDeviceToHost, m->stream), "download flags");
