@@ -203,8 +203,8 @@ def gpu_launches(prof, P, K, workload):
 # DRAM traffic per launch measured with ncu (dram__bytes_read.sum + dram__bytes_write.sum, one pass,
 # --clock-control none) on config 2 (256x256x64, 2 x 2,097,152 individuals), per interior cell or per
 # active individual; a launch's traffic is this figure times its units
-MEASURED_TRAFFIC = {"k32_xy": ("cell", 113.0), "k32_ztail": ("cell", 214.4),
-                    "k32_move": ("active", 78.0), "k32_physiology": ("active", 123.8)}
+MEASURED_TRAFFIC = {"k32_xy": ("cell", 114.6), "k32_ztail": ("cell", 214.2),
+                    "k32_move": ("active", 77.9), "k32_physiology": ("active", 123.8)}
 
 
 def profile_roofline(prof, members, nact, nslots):

@@ -76,8 +76,8 @@ struct MemberHost {
 };
 
 // Defaults: a rule on the sizes where there is one (0 or -1), otherwise the autotuner's choices on a
-// 256×256×64 model with 4 M individuals. pi_batch_autotune and pi_batch_set_option set them; no result depends
-// on them.
+// 256×256×64 model with 4 M individuals, but for ty (28 there, which small models are slower with: see k32_xy).
+// pi_batch_autotune and pi_batch_set_option set them; no result depends on them.
 struct Tuning {
     int bs_move = 128, bs_phys = 128, bs_assign = 128;
     int persist_move = 0, persist_phys = 0;   // 0: one tile per block; k: k blocks per SM, looping

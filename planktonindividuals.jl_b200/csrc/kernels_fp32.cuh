@@ -1314,10 +1314,11 @@ __global__ void __launch_bounds__(256, MINB) k32_physiology(PhysArgs a) {
 
 // ------------------------------------------------------------------------------------------
 // (d) tracer update in Float32: the three DST3FL sweeps (DST3FL.jl:1-73, multi_dim_adv.jl:1-135)
-//     and the rest of tracer_update! (tracer_update.jl:22-43) in two kernels: k32_xy (x and y
-//     sweeps of a level tile staged in shared memory) and k32_ztail (z sweep walking columns, then
-//     diffusion, sinking, forcing, boundary fluxes, particle terms and apply_tendency!). Both
-//     handle all 14 tracers per thread, so face coefficients and indices are formed once per face.
+//     and the rest of tracer_update! (tracer_update.jl:22-43) in two kernels: k32_xy (x and y sweeps
+//     of a level tile, walked row by row) and k32_ztail (z sweep walking columns, then diffusion, sinking,
+//     forcing, particle terms and apply_tendency!), and k32_close for the cells with a flux condition.
+//     A warp walks one pair of tracers with its stencil window in registers; the coefficients of a face
+//     are formed once, in shared memory, for the seven pairs of a block.
 //
 // The flux limiter is evaluated without forming θ: for the upwind side,
 //   ψ(δ/δ⁰)·δ⁰ = max(0, min(δ⁰, d₀δ⁰ + d₁δ, Rδ)) for δ⁰ ≥ 0 and min(0, max(δ⁰, d₀δ⁰ + d₁δ, Rδ))
@@ -1531,8 +1532,8 @@ __device__ __forceinline__ void st_at(float* base, unsigned byte, float v) {
 // those loads and of the limiter's chain, so warps count more than registers: on 256×256×64 309 µs with
 // two pairs per warp (16 warps per SM), 256 µs with one (28 warps), 231 µs at five blocks (35 warps, 56
 // registers); 326 µs when every tile staged its rows, fluxes and intermediate rows in shared memory.
-// Rows per tile (the walk costs TY + 4): at four blocks 363 µs with 8, 256 with 16, 245 with 28, which in
-// turn leaves small models short of blocks (96×80×24: 15.8 µs with 16, 19.5 with 28).
+// Rows per tile (the walk costs TY + 4): 16 and 28 take 231 and 221 µs on 256×256×64, 74 and 75 on 128×128×64,
+// 20 and 23 on 88×88×24, which 28 leaves short of blocks.
 struct XYRows { float4 *fx, *fy; float *tx, *ty; int* row; uint8_t *mx, *my; };
 __host__ __device__ inline size_t xy_smem(int ty) {
     return (size_t)(2 * ty + 5) * 32 * (sizeof(float4) + sizeof(float) + 1) + (size_t)(ty + 4) * sizeof(int);
