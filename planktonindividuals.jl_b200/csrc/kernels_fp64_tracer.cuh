@@ -58,7 +58,8 @@ __device__ __forceinline__ double flux_s(const double* s, int stride, double cm2
     const double dn = pos ? mk(cm1 - cm2, lm1, lm2) : mk(cp1 - c0, lp1, l0);
     const double ps = psi_s(s, stride, dn, d0);
     const double F = h * (pos ? cm1 + ps * d0 : c0 - ps * d0);
-    if (!finite64(pos ? cp1 : cm2)) {
+    // (a water cell beyond makes d0, and with it F, not finite; one on land is masked out of d0)
+    if (!finite64(pos ? cp1 : cm2) || (LM && !finite64(pos ? c0 : cm1))) {
         const double dx = pos ? mk(cp1 - c0, lp1, l0) : mk(cm1 - cm2, lm1, lm2);
         const double px = psi_s(s, stride, dx, d0);
         return F + 0.0 * (pos ? c0 - px * d0 : cm1 + px * d0);

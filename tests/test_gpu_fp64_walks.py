@@ -9,7 +9,7 @@ import oracle
 from PlanktonIndividuals import _abi, workloads as W
 from PlanktonIndividuals._native import CModel
 from PlanktonIndividuals.architectures import IronEnergyMode
-from PlanktonIndividuals.grids import Bounded, LatLonGrid, Periodic, RectilinearGrid
+from PlanktonIndividuals.grids import Bounded, LatLonGrid, Periodic, RectilinearGrid, fill_halo_tracer
 from PlanktonIndividuals.init import initialize_plankton_iron
 from PlanktonIndividuals.parameters import update_bgc_params, update_phyt_params
 from helpers import compare_states
@@ -58,4 +58,43 @@ def test_ragged_walks_identical_to_oracle(gpu_lib, size, kind):
             m.set_temp(np.full(size, 25.0))
             m.time_step(60.0)
     assert compare_states(models[1], models[0], 1) == []
+    models[0].close()
+
+
+@pytest.mark.parametrize("land", [False, True])
+@pytest.mark.parametrize("odd", ["courant", "zeros", "nonfinite"])
+def test_flux_shortcuts_identical_to_oracle(gpu_lib, odd, land):
+    """The flux of a face leaves out the side without transport and, where a product decides it, the limiter's
+    last quotient: Courant numbers above 1, faces at rest, flat and zero tracers, NaN and infinities."""
+    size = (33, 37, 9)
+    rng = np.random.default_rng(len(odd))
+    lm = rng.random(size) < 0.8 if land else np.ones(size, dtype=bool)
+    grid = RectilinearGrid(size=size, x=(0.0, size[0] * 50.0), y=(0.0, size[1] * 50.0), z=(0.0, -2.0 * size[2]),
+                           FT=np.float64, topology=(Periodic, Bounded, Bounded), landmask=lm)
+    phyt, bgc = update_phyt_params({}, np.float64, N=1), update_bgc_params({}, np.float64)
+    inds = [W.make_individuals(grid, phyt, 0, 8, 8, rng)]
+    trs = W.make_tracers(grid, rng)
+    cfl = 1.5 if odd == "courant" else 0.2
+    vel = [cfl * w / 60.0 * rng.standard_normal(n) for w, n in zip((50.0, 50.0, 2.0), (size, (size[0], size[1] + 1, size[2]),
+                                                                                       (size[0], size[1], size[2] + 1)))]
+    if odd == "zeros":
+        vel = [np.where(rng.random(v.shape) < 0.4, rng.choice([0.0, -0.0], v.shape), v) for v in vel]
+    for n, t in enumerate(trs):
+        hit = rng.random(t.shape) < (0.3 if odd == "zeros" else 0.01)
+        if odd == "zeros":
+            t[hit] = rng.choice([0.0, 1.0, 1e-310, -1e-3], t.shape)[hit]
+        if odd == "nonfinite" and n % 2:
+            t[hit] = rng.choice([np.nan, np.inf, -np.inf], t.shape)[hit]
+        fill_halo_tracer(t, grid)
+    models = [CModel(gpu_lib, "pi_", grid, bgc, phyt, 1, 8, 3, precision=_abi.PI_FP64), oracle.OracleModel(grid, bgc, phyt, 1, 8, 3)]
+    for m in models:
+        m.set_state(inds, trs)
+        for _ in range(2):
+            m.set_velocity(*vel)
+            m.set_PARF(np.full(size[:2], 300.0))
+            m.set_temp(np.full(size, 25.0))
+            m.time_step(60.0)
+    for n, name in enumerate(_abi.tracer_names):
+        a, b = models[1].get_tracer(n), models[0].get_tracer(n)
+        assert np.array_equal(a, b, equal_nan=True), (name, int(np.sum(~((a == b) | (np.isnan(a) & np.isnan(b))))))
     models[0].close()
