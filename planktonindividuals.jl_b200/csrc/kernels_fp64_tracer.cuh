@@ -88,7 +88,7 @@ struct PlkArgs {
 // A crowded cell by a warp: the entries' contributions are loaded 32 entries at a time, and lane q adds its
 // tracer's in the order of the entries (the sums of a sequential run), the five of calc_consume! from
 // shared memory. A thread alone waited for the loads of each entry: 1.6 million individuals in 16,384 cells
-// 186 µs, in 4,096 717, in 256 10,669; so 41, 36 and 346. A cell of up to CROWD_CELL keeps its thread: many
+// 186 µs, in 4,096 717, in 256 10,669; so 37, 35 and 327. A cell of up to CROWD_CELL keeps its thread: many
 // cells hide the waits of one another.
 template <bool IRON>
 __device__ __forceinline__ void plk_crowded(const PlkArgs& a, uint32_t c, double* sh) {
