@@ -23,7 +23,8 @@
 //   k32_xy               DST3FL x and y sweeps: a warp per tracer pair walks the rows of a level tile
 //   k32_ztail            z sweep walking columns, then diffusion, sinking, forcing, particle terms and
 //                        apply_tendency!
-//   k32_close            the same with the flux BCs, in the cells that have one (members with flux BCs)
+//   k32_close            the same with the flux BCs, in the cells that have one (members with flux BCs, of more
+//                        than a few levels)
 //   k32_halo_direct (k32_halo_small, k32_halo<x,y,z>)  fill_halo_tracer!, then vel₀ ← vel₁,
 //                        iteration and t
 // Every sort_interval steps (and before the first step after an upload) the slots of every segment
@@ -599,12 +600,15 @@ pi_status enqueue_step(pi_batch* b, double dT, int cur) {
                 bcs = bcs || b->mdh[m].any_bc;
                 gen = gen || b->mdh[m].any_bc || (float)b->mh[m].bgc.kappa_h != 0.0f || (float)b->mh[m].bgc.kappa_v != 0.0f;
             }
+            // (a member of so few levels is one item deep, whatever lz is)
+            const bool in_walk = bcs && b->maxNz <= CLOSE_LEVELS && b->maxNz <= b->tune.lz;
             const size_t zs = ztail_smem(b->tune.lz, gen);
-            if (b->tune.lz == 8) (gen ? k32_ztail<8, true> : k32_ztail<8, false>)<<<grid, blk, zs, s>>>(a);
+            if (in_walk) k32_ztail<16, true, true><<<grid, blk, ztail_smem(16, true), s>>>(a);
+            else if (b->tune.lz == 8) (gen ? k32_ztail<8, true> : k32_ztail<8, false>)<<<grid, blk, zs, s>>>(a);
             else if (b->tune.lz == 32) (gen ? k32_ztail<32, true> : k32_ztail<32, false>)<<<grid, blk, zs, s>>>(a);
             else if (b->tune.lz == 64) (gen ? k32_ztail<64, true> : k32_ztail<64, false>)<<<grid, blk, zs, s>>>(a);
             else (gen ? k32_ztail<16, true> : k32_ztail<16, false>)<<<grid, blk, zs, s>>>(a);
-            if (bcs) k32_close<<<grid, 256, 0, s>>>(a, b->tune.lz);
+            if (bcs && !in_walk) k32_close<<<grid, 256, 0, s>>>(a, b->tune.lz);
         }
         }
     }
@@ -798,7 +802,7 @@ pi_status pi_batch_create(const pi_member* members, int32_t nmembers, int32_t ns
         MemberDev& d = b->mdh[m];
         d.Nx = g.Nx; d.Ny = g.Ny; d.Nz = g.Nz; d.Hx = g.Hx; d.Hy = g.Hy; d.Hz = g.Hz;
         d.Gx = g.Gx; d.Gy = g.Gy; d.Gz = g.Gz; d.tx = g.topo[0]; d.ty = g.topo[1]; d.tz = g.topo[2];
-        d.all_water = h.all_water; d.any_bc = 0;
+        d.all_water = h.all_water; d.any_bc = 0; memset(d.bcf, 0, sizeof d.bcf);
         d.dx = (float)g.dx; d.dy = (float)g.dy;
         d.rdx = 1.0f / d.dx; d.rdy = 1.0f / d.dy;
         d.cbx = f32_bits(g.Nx); d.cby = f32_bits(g.Ny);
@@ -1397,7 +1401,12 @@ pi_status pi_batch_set_flux_bc(pi_batch* b, int32_t member, int32_t tracer, int3
     FluxBC32& d = b->bch[(size_t)b->mdh[member].bc_off + tracer * 6 + face];
     d.kind = kind; d.nt = nt; d.v = hb.v; d.n1 = (int)n1; d.n2 = (int)n2;
     int any = 0;
-    for (int q = 0; q < PI_NTRACERS * 6; ++q) if (b->bch[(size_t)b->mdh[member].bc_off + q].kind) any = 1;
+    for (int n = 0; n < PI_NTRACERS; ++n) {
+        uint8_t f = 0;
+        for (int q = 0; q < 6; ++q) f |= (b->bch[(size_t)b->mdh[member].bc_off + n * 6 + q].kind ? 1 : 0) << q;
+        b->mdh[member].bcf[n] = f;
+        any |= f != 0;
+    }
     b->mdh[member].any_bc = any;
     BK(cudaMemcpyAsync(b->bcs, b->bch.data(), b->bch.size() * sizeof(FluxBC32), cudaMemcpyHostToDevice, b->stream), "upload bcs");
     BK(cudaMemcpyAsync(b->md + member, &b->mdh[member], sizeof(MemberDev), cudaMemcpyHostToDevice, b->stream), "upload member");

@@ -56,6 +56,7 @@ struct MemberDev {
     double chl_unit;        // mg Chl per fixed-point unit of the Chl sums
     double fx_inv;          // 1 / fx_unit
     double chl_inv;         // 1 / chl_unit
+    uint8_t bcf[PI_NTRACERS];   // of each tracer, a bit per face (PI_WEST ..) with a flux boundary condition
 };
 
 // Cell codes: three indices in bit fields of one int32 (a, b, c from the low bits up, widths of a

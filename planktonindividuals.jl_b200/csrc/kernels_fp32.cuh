@@ -1764,13 +1764,6 @@ __device__ __forceinline__ float z_fluxes(const MemberDev& md, const FluxBC32* B
     return Gc;
 }
 
-// the faces of a tracer that have a condition
-__device__ __forceinline__ unsigned bc_faces(const FluxBC32* B) {
-    unsigned f = 0u;
-#pragma unroll
-    for (int e = 0; e < 6; ++e) f |= (B[e].kind ? 1u : 0u) << e;
-    return f;
-}
 // the x and y boundary faces of a cell in column (i, j)
 __device__ __forceinline__ unsigned side_faces(const MemberDev& md, int i, int j) {
     return (i == 1 + md.Hx ? 1u << PI_WEST : 0u) | (i == md.Nx + md.Hx ? 1u << PI_EAST : 0u)
@@ -1778,11 +1771,11 @@ __device__ __forceinline__ unsigned side_faces(const MemberDev& md, int i, int j
 }
 // Shared memory of an item: coefficients of the faces k0 .. k0 + LZ of the 32 columns, vertical transport
 // terms and populations of the cells, per-level constants, and with land the mask bits of face and cell
-// and of the cell's diffusion; the faces of each tracer with a flux condition.
-struct ZItem { float4* f; float* tr; unsigned* pop; ZLev* lev; uint8_t *m, *d, *bc; };
+// and of the cell's diffusion.
+struct ZItem { float4* f; float* tr; unsigned* pop; ZLev* lev; uint8_t *m, *d; };
 __host__ __device__ inline size_t ztail_smem(int lz, bool gen) {
     return (size_t)(lz + 1) * 32 * sizeof(float4) + (size_t)lz * (32 * sizeof(float) + sizeof(unsigned) + sizeof(ZLev))
-         + (size_t)((gen ? 2 : 1) * lz + 1) * 32 + (gen ? PI_NTRACERS : 0);
+         + (size_t)((gen ? 2 : 1) * lz + 1) * 32;
 }
 // add_forcing's coefficients of nutrient tracer n (tracer_forcings.jl:2-50): aS·T(n) + aO·T(other),
 // aO = 0 and other = n where there is no second tracer
@@ -1808,8 +1801,9 @@ __device__ __forceinline__ fx2 fx2_max0(fx2 v) {
 }
 
 // KIND 0: a nutrient pair (linear forcing, particle sums); 1: DFe and PFe_inorg; 2: PFe_bio and Dust (iron
-// forcing, sinking). GEN: diffusion or flux boundary conditions are switched on.
-template <int LZ, bool LM, int KIND, bool GEN>
+// forcing, sinking). GEN: diffusion or flux boundary conditions are switched on. CLOSE: the cells with a flux
+// condition are finished here, not in k32_close.
+template <int LZ, bool LM, int KIND, bool GEN, bool CLOSE>
 __device__ __forceinline__ void z_walk(const TrArgs& a, const MemberDev& md, const int4 it, const ZItem& S) {
     const int lane = threadIdx.x, p = warp_row();
     const int na = pair_tracer(p, 0), nb = pair_tracer(p, 1);
@@ -1863,11 +1857,12 @@ __device__ __forceinline__ void z_walk(const TrArgs& a, const MemberDev& md, con
     auto tl = [&](int kk) { return 4u * (unsigned)(qcol + (min(max(kk, top), bot) - 1) * slab); };
     auto ld2 = [](const float* x, const float* y, unsigned q) { return fx2_of(ldg_at(x, q), ldg_at(y, q)); };
     // apply_bcs! touches boundary cells only. Where a tracer of the pair has a condition on a face of the cell,
-    // the walk leaves the tendency in tr_next and the fluxes join it in k32_close; added to the new tracer, a flux below half an ulp of it would be lost.
+    // the walk leaves the tendency in tr_next and the fluxes join it after the walk (CLOSE) or in k32_close; added
+    // to the new tracer, a flux below half an ulp of it would be lost.
     // `open`: such cells are 1 all levels of the column, 2 the top one, 4 the bottom one.
     unsigned open = 0u;
     if (GEN) {
-        const unsigned any = S.bc[na] | S.bc[nb];
+        const unsigned any = md.bcf[na] | md.bcf[nb];
         open = (any & side_faces(md, i, j) ? 1u : 0u) | (any >> PI_TOP & 1u ? 2u : 0u) | (any >> PI_BOTTOM & 1u ? 4u : 0u);
     }
     // inputs of a level: own tracers, tracer_temp two levels below, the others, the particle sums
@@ -1991,17 +1986,30 @@ __device__ __forceinline__ void z_walk(const TrArgs& a, const MemberDev& md, con
         level(I1, I0, l + 1);
     }
     if (l < nl) level(I0, I1, l);
+    if (CLOSE && open) {
+        const FluxBC32 *Ba = a.bcs + md.bc_off + na * 6, *Bb = a.bcs + md.bc_off + nb * 6;
+        const unsigned fa = md.bcf[na], fb = md.bcf[nb], side = side_faces(md, i, j);
+        const int64_t itn = a.st->iteration + 1;
+        for (l = 0; l < nl; ++l) {
+            const int k = k0 + l, q = (int)(q40 >> 2) + l * slab;
+            const unsigned on = side | (k == top ? 1u << PI_TOP : 0u) | (k == bot ? 1u << PI_BOTTOM : 0u);
+            if (!((fa | fb) & on)) continue;
+            const float ga = oa[q], gb = ob[q], va = __ldg(ca + q), vb = __ldg(cb + q), dz = S.lev[l].dz;
+            oa[q] = __fadd_rn(va, __fadd_rn(ga, z_fluxes(md, Ba, fa & on, i, j, k, dz, dT, itn)));
+            ob[q] = __fadd_rn(vb, __fadd_rn(gb, z_fluxes(md, Bb, fb & on, i, j, k, dz, dT, itn)));
+        }
+    }
 }
 
-template <int LZ, bool LM, bool GEN>
+template <int LZ, bool LM, bool GEN, bool CLOSE>
 __device__ __forceinline__ void z_walk_any(const TrArgs& a, const MemberDev& m, const int4 it, const ZItem& S) {
     const int p = warp_row();
-    if (p < 5) z_walk<LZ, LM, 0, GEN>(a, m, it, S);
-    else if (p == 5) z_walk<LZ, LM, 1, GEN>(a, m, it, S);
-    else z_walk<LZ, LM, 2, GEN>(a, m, it, S);
+    if (p < 5) z_walk<LZ, LM, 0, GEN, CLOSE>(a, m, it, S);
+    else if (p == 5) z_walk<LZ, LM, 1, GEN, CLOSE>(a, m, it, S);
+    else z_walk<LZ, LM, 2, GEN, CLOSE>(a, m, it, S);
 }
 
-template <int LZ, bool GEN>
+template <int LZ, bool GEN, bool CLOSE = false>
 __global__ void __launch_bounds__(32 * TR_PAIRS, GEN ? 3 : 4) k32_ztail(TrArgs a) {
     if (stopped(a.err)) return;
     extern __shared__ __align__(16) unsigned char zsm[];
@@ -2012,7 +2020,6 @@ __global__ void __launch_bounds__(32 * TR_PAIRS, GEN ? 3 : 4) k32_ztail(TrArgs a
     S.pop = reinterpret_cast<unsigned*>(S.tr + LZ * 32);                // a bit per cell of a level with individuals
     S.m = reinterpret_cast<uint8_t*>(S.pop + LZ);
     S.d = S.m + (LZ + 1) * 32;
-    S.bc = S.d + LZ * 32;                                               // a bit per face with a condition, of each tracer
     const int tid = threadIdx.y * 32 + threadIdx.x;
     const int4 it = a.items[blockIdx.x];
     const MemberDev& m = a.T.md[it.x];
@@ -2049,9 +2056,6 @@ __global__ void __launch_bounds__(32 * TR_PAIRS, GEN ? 3 : 4) k32_ztail(TrArgs a
             if (threadIdx.x == 0) S.pop[e / 32] = occ;
         }
     }
-    if (GEN && tid < PI_NTRACERS) {
-        S.bc[tid] = (uint8_t)(m.any_bc ? bc_faces(a.bcs + m.bc_off + tid * 6) : 0u);
-    }
     if (tid < nl) {
         const int k = k0 + tid;
         ZLev L;
@@ -2066,8 +2070,8 @@ __global__ void __launch_bounds__(32 * TR_PAIRS, GEN ? 3 : 4) k32_ztail(TrArgs a
         S.lev[tid] = L;
     }
     __syncthreads();
-    if (land) z_walk_any<LZ, true, GEN>(a, m, it, S);
-    else z_walk_any<LZ, false, GEN>(a, m, it, S);
+    if (land) z_walk_any<LZ, true, GEN, CLOSE>(a, m, it, S);
+    else z_walk_any<LZ, false, GEN, CLOSE>(a, m, it, S);
 }
 
 // Closes the cells that the walks of an item of k32_ztail left open (a tracer of the pair has a condition on
@@ -2075,21 +2079,21 @@ __global__ void __launch_bounds__(32 * TR_PAIRS, GEN ? 3 : 4) k32_ztail(TrArgs a
 // added. A kernel of its own, launched when a member has a flux condition: at the end of k32_ztail a warp had
 // 31 levels of a boundary column one after the other, and the code cost the walk registers (117×93×31 with a
 // western, a bottom and a top condition: 75.5 µs there, 72 µs for the two kernels; 81 to 93 µs with the
-// tendency in k32_ztail in several forms).
+// tendency in k32_ztail in several forms). A launch more costs 4 µs of a small step, so batches of at most
+// CLOSE_LEVELS levels have their walks finish the cells themselves (CLOSE): 22×33×5 44.2 µs per step against 47.4,
+// 22×33×9 50.5 and 53.5, 60×50×12 59.0 and 57.8, 117×93×16 80.4 and 75.8.
+#define CLOSE_LEVELS 10
 __global__ void __launch_bounds__(256) k32_close(TrArgs a, int lz) {
     if (stopped(a.err)) return;
-    __shared__ uint8_t bc[PI_NTRACERS];                  // a bit per face with a condition
     const int4 it = a.items[blockIdx.x];
     const MemberDev& md = a.T.md[it.x];
     if (!md.any_bc) return;
     const FluxBC32* B = a.bcs + md.bc_off;
-    if (threadIdx.x < PI_NTRACERS) bc[threadIdx.x] = (uint8_t)bc_faces(B + threadIdx.x * 6);
-    __syncthreads();
     const int j = it.z, k0 = it.w, bot = md.Nz + md.Hz, nl = min(lz, bot - k0 + 1);
     const int64_t itn = a.st->iteration + 1;
     for (int p = 0; p < TR_PAIRS; ++p) {
         const int na = pair_tracer(p, 0), nb = pair_tracer(p, 1);
-        const unsigned fa = bc[na], fb = bc[nb];
+        const unsigned fa = md.bcf[na], fb = md.bcf[nb];
         if (!(fa | fb)) continue;
         const float *ca = a.tr + na * a.Gtot + md.cell_off, *cb = a.tr + nb * a.Gtot + md.cell_off;
         float *oa = a.tr_next + na * a.Gtot + md.cell_off, *ob = a.tr_next + nb * a.Gtot + md.cell_off;
